@@ -513,11 +513,12 @@ def fp64_roofline(kernel_ms, n_mems, peak, kernel, workload):
     path = os.path.join(ROOT, 'profiles', 'fp64_counts.json')
     counts = json.load(open(path)).get('kernels', {}).get(workload, {}) if os.path.exists(path) else {}
     entry, counted = counts.get(kernel), kernel
-    if entry is None and kernel.startswith('k_cell_step<double>'):
-        # another tile size of the same kernel: every thread runs the same
-        # code per membrane slot, so its count per membrane stands in
+    family = kernel.split(' (')[0]
+    if entry is None and family in ('k_cell_step<double>', 'k_plain_step'):
+        # another tile size of the same kernel: the same code per membrane
+        # slot (or junction and cell), so its count per membrane stands in
         for name, e in counts.items():
-            if name.startswith('k_cell_step<double>'):
+            if name.startswith(family):
                 entry, counted = e, name
                 break
     if entry is None:
@@ -568,17 +569,15 @@ def config_plain250(wl, stream, flush, cpu=True):
         kb = e.cell_kernel_bytes()
     out = {'workload': w['desc'], 'cells': g.n_cells, 'membranes': g.n_mems, 'time_steps_per_run': T,
            'form': 'plain FP64', 'value': g.n_mems * T / (ms / 1e3), 'unit': UNIT, 'ms_per_run': ms,
-           'roofline': roofline_entry(kb, kms / 1e3, 'k_cell_step<double>',
-                                      note='a 1.4k-membrane cluster fills a few dozen CTAs: bound by '
-                                           'the dependent FP64 instruction chain of a lane, not by HBM',
+           'roofline': roofline_entry(kb, kms / 1e3, 'k_plain_step',
+                                      note='a 1.4k-membrane cluster is bound by the dependent FP64 instruction '
+                                           'chain of a step and the grid barrier between steps, not by HBM',
                                       step=step_bytes('fp64', g.n_cells, g.n_mems)),
-           'kernel_launches_per_step': 1 if launch[1] == 5 else 2,   # the ion kernel mixes the environment
-           'autotuned_launch': {'cta_slots': launch[0], 'kernel': 'k_cell_step_ion' if launch[1] == 5
-                                else 'k_cell_step<double>'},
+           'kernel_launches_per_run': 1,                 # the resident form: every step in one launch
+           'autotuned_launch': {'cta_slots': launch[0], 'kernel': 'k_plain_step'},
            'autotune_table': table}
-    out['roofline']['kernel'] = out['autotuned_launch']['kernel']
-    kname = f"k_cell_step_ion<{launch[0]}>" if launch[1] == 5 else f"k_cell_step<double> ({launch[0]} slots)"
-    out['roofline_fp64'] = fp64_roofline(kms, g.n_mems, fp64_peak(stream), kname, 'plain250')
+    out['roofline_fp64'] = fp64_roofline(kms, g.n_mems, fp64_peak(stream), f'k_plain_step ({launch[0] // 4} cells)',
+                                         'plain250')
     if cpu:
         out['cpu_baseline'] = cpu_baseline(g, p, Dm, st, budget_s=6.0)
     return out
@@ -872,14 +871,14 @@ def profile_kernel(which):
 
 # kernels, by the number bx_set_launch_config takes (5: the plain form's)
 KERNEL_NAMES = {0: 'k_split_step', 1: 'k_split_persist', 2: 'k_split_fact', 3: 'k_split_resident',
-                4: 'k_split_fact_pipe', 5: 'k_cell_step_ion'}
+                4: 'k_split_fact_pipe', 5: 'k_plain_step'}
 LAUNCH_SUFFIX = {'': 0, 'p': 1, 'f': 2, 'r': 3, 'q': 4, 'i': 5}
 
 
 def parse_launch(text):
     """'192' tile kernel, '192p' persistent, '192f' factored, '256r' resident,
-    '256q' pipelined factored, '32i' the plain form's one-lane-per-ion
-    kernel; a number after 'f' picks the factored kernel's
+    '256q' pipelined factored, '32i' the plain form's step (as '32');
+    a number after 'f' picks the factored kernel's
     variant ('256f12': two junctions per round, entries prefetched)."""
     head = text.lstrip('0123456789')
     tpb = int(text[:len(text) - len(head)])
@@ -1137,7 +1136,7 @@ def main():
                            'vm_err_curve_V': curve,
                            'roofline_fp64': None if kms_plain is None else fp64_roofline(
                                kms_plain, n_mems, fp64_peak(stream),
-                               f'k_cell_step<double> ({tune_plain[0]} slots)', args.workload)},
+                               f'k_plain_step ({tune_plain[0] // 4} cells)', args.workload)},
             'roofline': roof,
             'cpu_baseline': cpu,
             'e2e': {'value': e2e_val, 'unit': UNIT, 'h2d_bytes_per_step': int(h2d),

@@ -29,6 +29,7 @@
 #include "bx_launch.cuh"
 #include "bx_lapinv.cuh"
 #include "bx_network.cuh"
+#include "bx_plain.cuh"
 #include "bx_split.cuh"
 #include "bx_state.cuh"
 
@@ -143,7 +144,20 @@ struct bx_cluster {
   double *d_Denv = nullptr, *d_Ex = nullptr, *d_Ey = nullptr, *d_fx = nullptr, *d_fy = nullptr,
          *d_tmp = nullptr, *d_tmp2 = nullptr, *d_venv = nullptr, *d_rho_env = nullptr, *d_vsrc = nullptr;
   unsigned long long* d_status = nullptr;
-  unsigned* d_env_ticket = nullptr;   // [ncl] k_cell_step_ion's last-CTA counters (zero between steps)
+  // ---- factored plain step (bx_plain.cuh)
+  bool vm_uniform = false;         // Vmem is one value per cell (the factored step needs it)
+  int pl_pin = 0;                  // cells per tile pinned by a launch configuration (0: by size)
+  int pl_nc = 0, pl_ntile = 0, pl_ngroup = 0, pl_ne = 0, pl_nm = 0;   // cells per tile, tiles, groups, largest tile
+  bool pl_res = false;             // the resident form fits: one tile per co-resident CTA
+  unsigned char* pl_base = nullptr;   // the one allocation that the pl_ pointers point into
+  int2* pl_tile = nullptr;
+  int4* pl_ent = nullptr;
+  int *pl_tile_cl = nullptr, *pl_cl_tile = nullptr, *pl_cl_group = nullptr, *pl_ent_ptr = nullptr,
+      *pl_n_local = nullptr, *pl_mem_ent = nullptr, *pl_mem_gate = nullptr;
+  double *pl_mem_w = nullptr, *pl_dsa = nullptr, *pl_sa = nullptr, *pl_ivol = nullptr, *pl_part = nullptr,
+         *pl_gpart = nullptr;
+  unsigned *pl_ticket = nullptr, *pl_ctl = nullptr;   // [groups + ncl]; barrier counter and timeout flag
+  int64_t pl_nent = 0;
   // ---- outputs
   double *o_fmem = nullptr, *o_fgj = nullptr, *o_rate = nullptr, *o_rho = nullptr, *o_Jn = nullptr,
          *o_Imem = nullptr, *o_Jcx = nullptr, *o_Jcy = nullptr, *o_Jc = nullptr, *o_vmave = nullptr,
@@ -156,6 +170,7 @@ struct bx_cluster {
   int64_t steps_done = 0, launches = 0;
   cudaGraphExec_t graph = nullptr;
   bool graph_valid = false;
+  int64_t layout_gen = 0;          // bumped with every change that a captured graph would not see
   std::vector<int> h_cell_ptr, h_m2c, h_map_env;
   std::vector<double> h_phib;
   // ---- environment fields on demand (bx_env_fields)
@@ -216,13 +231,14 @@ void free_all(bx_cluster* h) {
       h->t_gw, h->t_dtv, h->t_dvc, h->t_rng,
       h->s_cenv_f, h->s_pump, h->s_part, h->s_phib, h->d_cenv, h->d_phib, h->d_env_part,
       h->d_mem_flux_sa, h->d_pump, h->d_env_scale, h->d_Denv, h->d_Ex, h->d_Ey, h->d_fx, h->d_fy,
-      h->d_tmp, h->d_tmp2, h->d_venv, h->d_rho_env, h->d_vsrc, h->d_status, h->d_env_ticket, h->o_fmem, h->o_fgj, h->o_rate,
+      h->d_tmp, h->d_tmp2, h->d_venv, h->d_rho_env, h->d_vsrc, h->d_status, h->o_fmem, h->o_fgj, h->o_rate,
       h->o_rho, h->o_Jn, h->o_Imem, h->o_Jcx, h->o_Jcy, h->o_Jc, h->o_vmave, h->o_dvm, h->o_Ecx,
       h->o_Ecy, h->o_Emc, h->o_Egjx, h->o_Egjy, h->o_gjopen, h->o_sigma, h->o_vmc, h->o_vm_mem,
       h->o_drho, h->f_lap, h->f_X, h->f_buf, h->f_last, h->d_cl_mem, h->d_resid,
       h->bf_ci, h->bf_last, h->bf_cd, h->bf_buf, h->bf_X, h->bf_Y, h->bf_scale, h->d_gjo, h->t_gjo, h->d_cnew, h->d_Rrads,
       h->st_vm, h->st_cc, h->st_cam, h->st_go, h->d_flag, h->t_slot_of_mem, h->t_blob,
-      h->f_dsa, h->f_cst, h->f_gbeg, h->f_gj, h->f_tile_e0, h->r_cta, h->r_gj, h->r_gbeg, h->r_halo, h->r_cpart, h->r_ctl};
+      h->f_dsa, h->f_cst, h->f_gbeg, h->f_gj, h->f_tile_e0, h->r_cta, h->r_gj, h->r_gbeg, h->r_halo, h->r_cpart, h->r_ctl,
+      h->pl_base};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (auto& fs : h->fshapes)
@@ -436,11 +452,11 @@ bool fact_eligible(const bx_cluster* h, bool out) {
   return h->mode == MODE_SPLIT && !out && !h->phib_nonzero && !h->ecm && !h->vgj && !h->ca;
 }
 
-// The plain form's one-lane-per-ion kernel covers the same configuration
-// without polarizability, on CTAs of 8 to 64 membrane slots.
-bool ion_eligible(const bx_cluster* h, bool out) {
-  return h->mode != MODE_SPLIT && !out && !h->phib_nonzero && !h->ecm && !h->vgj && !h->ca && !h->polar &&
-         (h->tpb == 8 || h->tpb == 16 || h->tpb == 32 || h->tpb == 64);
+// The plain form's factored step (bx_plain.cuh) needs one Vmem and one
+// environment per cell: no Phi_b, no extracellular spaces, no polarizability,
+// no outputs.
+bool plain_factored(const bx_cluster* h, bool out) {
+  return h->mode == MODE_PLAIN && !out && !h->phib_nonzero && !h->ecm && !h->polar;
 }
 
 bool is_betse_six_ions(const bx_cluster* h) {
@@ -757,15 +773,6 @@ cudaError_t launch_cell(bx_cluster* h, int parity, bool out, cudaStream_t s) {
   bx::DevGeom g = dev_geom(h);
   bx::StepConst k = make_step_const(h);
   bx::StepPtrs p = step_ptrs(h, parity);
-  if (h->kind == KIND_ION && ion_eligible(h, out)) {
-    const bx::EnvMix em{h->d_cenv, h->d_cl_blk, h->d_env_scale, h->d_env_ticket};
-    switch (h->tpb) {
-      case 8: return bx::launch_cell_step_ion<8>(h->nblk, s, g, p, k, em);
-      case 16: return bx::launch_cell_step_ion<16>(h->nblk, s, g, p, k, em);
-      case 32: return bx::launch_cell_step_ion<32>(h->nblk, s, g, p, k, em);
-      default: return bx::launch_cell_step_ion<64>(h->nblk, s, g, p, k, em);
-    }
-  }
   // partitions of 8 or 16 membrane slots run on 32-thread CTAs
   switch (h->tpb) {
     case 8:
@@ -775,6 +782,31 @@ cudaError_t launch_cell(bx_cluster* h, int parity, bool out, cudaStream_t s) {
     case 128: return bx::launch_cell_step<double, 128>(h->ecm, out, h->phib_nonzero, h->nblk, s, g, p, k);
     default: return bx::launch_cell_step<double, 256>(h->ecm, out, h->phib_nonzero, h->nblk, s, g, p, k);
   }
+}
+
+// n steps of the factored plain step: one per launch, or (resident) all in
+// one cooperative launch
+cudaError_t launch_plain(bx_cluster* h, int parity, int n, bool resident, cudaStream_t s,
+                         long long timeout_ns = kResTimeoutNs) {
+  bx::PlainGeom g{};
+  g.C = h->C; g.M = h->M; g.ntile = h->pl_ntile;
+  g.tile = h->pl_tile; g.tile_cl = h->pl_tile_cl; g.cl_tile = h->pl_cl_tile; g.cl_group = h->pl_cl_group;
+  g.ent_ptr = h->pl_ent_ptr; g.n_local = h->pl_n_local; g.ent = h->pl_ent;
+  g.mem_ent = h->pl_mem_ent; g.mem_gate = h->pl_mem_gate; g.cell_ptr = h->d_cell_ptr; g.m2c = h->d_m2c;
+  g.mem_w = h->pl_mem_w; g.mem_sa = h->d_mem_sa; g.dsa = h->pl_dsa; g.sa = h->pl_sa; g.ivol = h->pl_ivol;
+  g.diviterm = h->d_diviterm;
+  bx::PlainRun r{};
+  r.vm[0] = h->d_vm[parity]; r.vm[1] = h->d_vm[parity ^ 1];
+  r.ccm[0] = h->d_ccm[parity]; r.ccm[1] = h->d_ccm[parity ^ 1];
+  r.n_steps = n;
+  r.nc_max = h->pl_nc; r.ne_max = h->pl_ne; r.nm_max = h->pl_nm;
+  r.part = h->pl_part; r.gpart = h->pl_gpart; r.ticket = h->pl_ticket;
+  r.cenv = h->d_cenv; r.env_scale = h->d_env_scale; r.ctl = h->pl_ctl; r.timeout_ns = timeout_ns;
+  const bx::StepConst k = make_step_const(h);
+  const bx::StepPtrs p = step_ptrs(h, parity);
+  const bool six = is_betse_six_ions(h);
+  return resident ? bx::launch_plain_resident(six, h->vgj, s, g, p, k, r)
+                  : bx::launch_plain_step(six, h->vgj, s, g, p, k, r);
 }
 
 // The extracellular grid of one step (update_ecm, update_Co's ECM term, get_current's E_env).
@@ -888,10 +920,14 @@ cudaError_t enqueue_step(bx_cluster* h, int parity, bool out, cudaStream_t s) {
     }
     return cudaGetLastError();
   }
+  if (h->vm_uniform && plain_factored(h, out)) {
+    h->launches++;
+    return launch_plain(h, parity, 1, false, s);
+  }
   e = launch_cell(h, parity, out, s);
   if (e != cudaSuccess) return e;
   h->launches++;
-  if (h->kind == KIND_ION && ion_eligible(h, out)) return cudaSuccess;   // it mixed the environment
+  h->vm_uniform = !h->polar && !h->phib_nonzero;
   if (!h->ecm) {
     bx::k_env_mix<<<h->ncl, 256, 0, s>>>(h->d_env_part, h->d_cl_blk, h->I, h->d_cenv, h->d_env_scale);
     h->launches++;
@@ -901,7 +937,7 @@ cudaError_t enqueue_step(bx_cluster* h, int parity, bool out, cudaStream_t s) {
 }
 
 int launches_per_step(const bx_cluster* h) {
-  if (h->kind == KIND_ION && ion_eligible(h, false)) return 1;
+  if (plain_factored(h, false)) return 1;
   if (!h->ecm) return 2;
   if (h->ca) return h->par.sharpness < 1.0 ? 9 : 8;
   return h->par.sharpness < 1.0 ? 8 : 4;
@@ -1159,6 +1195,168 @@ int build_split_layout(bx_cluster* h, const std::vector<int>& blk) {
   return upload_param_arrays(h);
 }
 
+// sum of Dm_i * mem_sa of every cell, on the handle's stream
+cudaError_t plain_dsa(bx_cluster* h) {
+  bx::k_plain_dsa<<<dim3((unsigned)((h->C + 255) / 256), (unsigned)h->I), 256, 0, h->stream>>>(
+      h->C, h->M, h->I, h->d_cell_ptr, h->d_Dm, h->d_mem_sa, h->pl_dsa);
+  return cudaGetLastError();
+}
+
+// Tiles, junction entries and buffers of the factored plain step.  Cells per
+// tile (a power of two):
+//   pinned    by the launch configuration (a quarter of its membrane slots);
+//   resident  the smallest of 2 to 64 whose tiles fit one a SM (one cluster):
+//             small clusters spread over every SM and keep their state there;
+//   else      64, halved while fewer than two tiles an SM would be left.
+// Measured us per step, cells per tile 8 / 16 / 32 / 64 (r: resident):
+// 2,878 cells 15.1 / 16.6 / 10.9r / 13.7r, 6,069 cells 25.6 / 17.2 / 20.9 /
+// 13.6r, 9,918 cells 37.5 / 28.3 / 21.2 / 30.7 (so at 64 the resident rule
+// stops where the tiles exceed the SMs), 20,432 cells 67.6 / 42.6 / 37.3 /
+// 33.0, 100,043 cells 293 / 176 / 121 / 108.
+// Halved further while a tile's shared memory would exceed kPlainSmemMax (cells with
+// very many membranes).
+constexpr size_t kPlainSmemMax = 100 * 1024;
+int build_plain_layout(bx_cluster* h) {
+  const int C = h->C, M = h->M, I = h->I, ncl = h->ncl;
+  const std::vector<int>& ptr = h->h_cell_ptr;
+  const std::vector<int>& m2c = h->h_m2c;
+  const std::vector<int>& nn = h->h_nn;
+  auto tiles_of = [&](int nc) {
+    int n = 0;
+    for (int cl = 0; cl < ncl; ++cl) n += (h->cl_cell[cl + 1] - h->cl_cell[cl] + nc - 1) / nc;
+    return n;
+  };
+  int nc = 64;
+  bool want_res = ncl == 1;
+  if (h->pl_pin) {
+    nc = h->pl_pin;
+  } else if (want_res && tiles_of(64) <= h->sm_count) {
+    for (nc = 2; tiles_of(nc) > h->sm_count;) nc <<= 1;
+  } else {
+    want_res = false;
+    while (nc > 4 && tiles_of(nc) < 2 * h->sm_count) nc >>= 1;
+  }
+  std::vector<int2> tile;
+  std::vector<int4> ent;
+  std::vector<int> tile_cl, cl_tile(ncl + 1, 0), cl_group(ncl + 1, 0), ent_ptr, n_local, mem_ent(M),
+      mem_gate(h->vgj ? M : 0);
+  ent.reserve((size_t)M * 2 / 3 + 16);
+  std::vector<int4> halo;
+  std::vector<int> halo_mem;
+  int ne_max = 0, nm_max = 0;
+  for (;; nc >>= 1) {
+    tile.clear(); ent.clear(); tile_cl.clear(); ent_ptr.assign(1, 0); n_local.clear();
+    ne_max = nm_max = 0;
+    for (int cl = 0; cl < ncl; ++cl) {
+      for (int c0 = h->cl_cell[cl]; c0 < h->cl_cell[cl + 1]; c0 += nc) {
+        const int c1 = std::min(c0 + nc, h->cl_cell[cl + 1]), m0 = ptr[c0], m1 = ptr[c1];
+        tile.push_back(make_int2(c0, c1 - c0));
+        tile_cl.push_back(cl);
+        const int e0 = (int)ent.size();
+        halo.clear();
+        halo_mem.clear();
+        for (int m = m0; m < m1; ++m) {
+          const int a = m2c[m], q = nn[m], c = m2c[q];
+          const bool bnd = h->h_bflag[m] != 0;
+          if (bnd) mem_ent[m] = bx::kPlainNone;
+          if (bnd && !h->vgj) continue;               // no flux; a gated one still updates its open fraction
+          const bool local = q >= m0 && q < m1;
+          int e;
+          if (local && q < m && nn[q] == m && !h->h_bflag[q]) {
+            e = ~mem_ent[q];                          // the junction's entry, from the partner's side
+            if (h->vgj) mem_gate[m] = ~e;
+          } else if (local) {
+            e = (int)ent.size() - e0;
+            ent.push_back(make_int4(a - c0, c - c0, ptr[c], 0));
+            if (h->vgj) mem_gate[m] = e;
+          } else {
+            halo.push_back(make_int4(a - c0, c, ptr[c], 0));
+            halo_mem.push_back(m);
+            continue;
+          }
+          if (!bnd) mem_ent[m] = e;
+        }
+        const int nl = (int)ent.size() - e0;
+        n_local.push_back(nl);
+        for (size_t j = 0; j < halo.size(); ++j) {
+          const int m = halo_mem[j], e = (int)ent.size() - e0;
+          if (h->vgj) mem_gate[m] = e;
+          if (!h->h_bflag[m]) mem_ent[m] = e;
+          ent.push_back(halo[j]);
+        }
+        ent_ptr.push_back((int)ent.size());
+        ne_max = std::max(ne_max, (int)ent.size() - e0);
+        nm_max = std::max(nm_max, m1 - m0);
+      }
+      cl_tile[cl + 1] = (int)tile.size();
+      cl_group[cl + 1] = cl_group[cl] + (cl_tile[cl + 1] - cl_tile[cl] + 31) / 32;
+    }
+    const size_t smem = sizeof(double) * (size_t)bx::PlainSmem(nc, ne_max, nm_max, I, h->vgj).total;
+    if (smem <= kPlainSmemMax || nc == 1) break;
+  }
+  const int nt = (int)tile.size(), ng = cl_group[ncl];
+  const bool six = is_betse_six_ions(h);
+  const size_t smem = sizeof(double) * (size_t)bx::PlainSmem(nc, ne_max, nm_max, I, h->vgj).total;
+  int per_sm = 0, coop = 0;
+  BX_CU(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->dev));
+  if (smem > kPlainSmemMax) return fail(BX_EINVAL, "a cell's junctions do not fit the shared memory of one SM");
+  // one limit for every handle, so that handles of different sizes never undercut each other
+  BX_CU(bx::plain_smem_attr(six, h->vgj, kPlainSmemMax));
+  h->pl_res = false;
+  if (want_res && coop && nt <= 256) {                // 256: the environment tree of the resident form
+    BX_CU(bx::plain_resident_per_sm(six, h->vgj, smem, &per_sm));
+    h->pl_res = nt <= per_sm * h->sm_count;
+  }
+  h->pl_nc = nc; h->pl_ntile = nt; h->pl_ngroup = ng; h->pl_ne = ne_max; h->pl_nm = nm_max;
+  h->pl_nent = (int64_t)ent.size();
+  // one allocation and one copy: the tables (and the zeroed counters), then
+  // what the device fills
+  size_t off = 0;
+  auto take = [&](size_t bytes) { const size_t at = off; off += (bytes + 255) & ~(size_t)255; return at; };
+  const size_t o_tile = take(nt * sizeof(int2)), o_ent = take(ent.size() * sizeof(int4)),
+               o_tcl = take(nt * sizeof(int)), o_clt = take((ncl + 1) * sizeof(int)),
+               o_clg = take((ncl + 1) * sizeof(int)), o_ep = take((nt + 1) * sizeof(int)),
+               o_nl = take(nt * sizeof(int)), o_me = take((size_t)M * sizeof(int)),
+               o_mg = take(mem_gate.size() * sizeof(int)), o_tk = take((ng + ncl) * sizeof(unsigned)),
+               o_ctl = take(2 * sizeof(unsigned)), host_bytes = off, o_part = take((size_t)2 * nt * I * sizeof(double)),
+               o_gp = take((size_t)(2 * ng + 8 * ncl) * I * sizeof(double)), o_mw = take((size_t)M * sizeof(double)),
+               o_sa = take((size_t)C * sizeof(double)), o_iv = take((size_t)C * sizeof(double)),
+               o_dsa = take((size_t)I * C * sizeof(double));
+  std::vector<unsigned char> blob(host_bytes, 0);
+  auto put = [&](size_t at, const void* src, size_t bytes) { if (bytes) std::memcpy(blob.data() + at, src, bytes); };
+  put(o_tile, tile.data(), nt * sizeof(int2));
+  put(o_ent, ent.data(), ent.size() * sizeof(int4));
+  put(o_tcl, tile_cl.data(), nt * sizeof(int));
+  put(o_clt, cl_tile.data(), (ncl + 1) * sizeof(int));
+  put(o_clg, cl_group.data(), (ncl + 1) * sizeof(int));
+  put(o_ep, ent_ptr.data(), (nt + 1) * sizeof(int));
+  put(o_nl, n_local.data(), nt * sizeof(int));
+  put(o_me, mem_ent.data(), (size_t)M * sizeof(int));
+  put(o_mg, mem_gate.data(), mem_gate.size() * sizeof(int));
+  if (h->pl_base) cudaFree(h->pl_base);
+  h->pl_base = nullptr;
+  h->pl_dsa = nullptr;
+  BX_CU(dalloc(&h->pl_base, off));
+  BX_CU(h2d(h->pl_base, blob.data(), host_bytes));
+  unsigned char* d = h->pl_base;
+  auto dbl = [&](size_t at) { return reinterpret_cast<double*>(d + at); };
+  auto i32 = [&](size_t at) { return reinterpret_cast<int*>(d + at); };
+  h->pl_tile = reinterpret_cast<int2*>(d + o_tile);
+  h->pl_ent = reinterpret_cast<int4*>(d + o_ent);
+  h->pl_tile_cl = i32(o_tcl); h->pl_cl_tile = i32(o_clt); h->pl_cl_group = i32(o_clg); h->pl_ent_ptr = i32(o_ep);
+  h->pl_n_local = i32(o_nl); h->pl_mem_ent = i32(o_me); h->pl_mem_gate = i32(o_mg);
+  h->pl_ticket = reinterpret_cast<unsigned*>(d + o_tk);
+  h->pl_ctl = reinterpret_cast<unsigned*>(d + o_ctl);
+  h->pl_part = dbl(o_part); h->pl_gpart = dbl(o_gp); h->pl_mem_w = dbl(o_mw); h->pl_sa = dbl(o_sa);
+  h->pl_ivol = dbl(o_iv); h->pl_dsa = dbl(o_dsa);
+  bx::k_plain_static<<<(C + 255) / 256, 256, 0, h->stream>>>(C, h->d_cell_ptr, h->d_gj_w, h->d_mem_sa, h->d_cell_vol,
+                                                             h->pl_mem_w, h->pl_sa, h->pl_ivol);
+  BX_CU(cudaGetLastError());
+  if (h->have_dm) BX_CU(plain_dsa(h));
+  BX_CU(cudaStreamSynchronize(h->stream));
+  return BX_OK;
+}
+
 // CTA partition for `tpb` membrane slots: runs of whole cells of one cluster
 // with at most tpb membranes; the split form also caps a tile at 32 cells
 // (its (ion, cell) phase maps ion -> warp, cell -> lane).  Rebuilt by the
@@ -1211,8 +1409,9 @@ int build_partition(bx_cluster* h, int tpb) {
   h->nblk = nblk;
   h->tpb = tpb;
   h->graph_valid = false;
+  ++h->layout_gen;
   if (h->mode == MODE_SPLIT) return build_split_layout(h, blk);
-  return BX_OK;
+  return h->ecm || h->polar ? BX_OK : build_plain_layout(h);
 }
 
 int create_impl(const bx_geom* gs, const bx_params* ps, int ncl, int precision, bx_handle* out) {
@@ -1308,6 +1507,7 @@ int create_impl(const bx_geom* gs, const bx_params* ps, int ncl, int precision, 
   h->h_cell_ptr = ptr; h->h_m2c = m2c; h->h_map_env = map_env;
   h->h_phib.assign(G, 0.0);
   h->h_gjw = gjw;
+  h->h_bflag = bflag; h->h_nn = nn;
 
   // environment CSR (grid cell -> its membranes, ascending) for the ECM scatter
   std::vector<int> env_ptr(G + 1, 0), env_mem(M);
@@ -1352,14 +1552,12 @@ int create_impl(const bx_geom* gs, const bx_params* ps, int ncl, int precision, 
   ALLOC(h->d_pump, ncl); ALLOC(h->d_env_scale, ncl);
   ALLOC(h->d_phib, G);
   ALLOC(h->d_status, 4);
-  ALLOC(h->d_env_ticket, ncl);
   if (cudaMemset(h->d_status, 0, 4 * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMemset(h->d_env_ticket, 0, (size_t)ncl * sizeof(unsigned)) != cudaSuccess ||
       cudaMemset(h->d_phib, 0, (size_t)G * sizeof(double)) != cudaSuccess)
     return bail(BX_ECUDA, "cudaMemset");
   if (h->mode == MODE_SPLIT) {
     // host copies for the tile-major relayout (build_split_layout)
-    h->h_msa = msa; h->h_bflag = bflag; h->h_nn = nn; h->h_vol = vol; h->h_div = div;
+    h->h_msa = msa; h->h_vol = vol; h->h_div = div;
     ALLOC(h->s_cenv_f, (size_t)ncl * I); ALLOC(h->d_cenv, h->ecm ? (size_t)I * G : (size_t)ncl * I);
     ALLOC(h->s_pump, ncl);
     ALLOC(h->s_phib, G);
@@ -1447,6 +1645,7 @@ int bx_set_params(bx_handle h, const bx_params* p) {
   h->par = *p;
   h->cl_par[0] = *p;
   h->graph_valid = false;
+  ++h->layout_gen;
   return upload_param_arrays(h);
 }
 
@@ -1461,6 +1660,7 @@ int bx_batch_set_params(bx_handle h, const bx_params* p) {
   h->par = p[0];
   h->cl_par.assign(p, p + h->ncl);
   h->graph_valid = false;
+  ++h->layout_gen;
   return upload_param_arrays(h);
 }
 
@@ -1486,6 +1686,10 @@ int bx_set_membrane_diffusivity(bx_handle h, const double* Dm) {
     BX_CU(cudaMemcpy(h->d_Dm_f, f.data(), n * sizeof(float), cudaMemcpyHostToDevice));
   } else {
     BX_CU(cudaMemcpy(h->d_Dm, Dm, n * sizeof(double), cudaMemcpyHostToDevice));
+    if (h->pl_dsa) {
+      BX_CU(plain_dsa(h));
+      BX_CU(cudaStreamSynchronize(h->stream));
+    }
   }
   h->have_dm = true;
   return BX_OK;
@@ -1551,7 +1755,10 @@ int bx_set_boundary_potential(bx_handle h, const double* Phi_b) {
     for (int k = 0; k < h->G; ++k) f[k] = (float)h->h_phib[k];
     BX_CU(cudaMemcpy(h->s_phib, f.data(), (size_t)h->G * sizeof(float), cudaMemcpyHostToDevice));
   }
-  if (nz != h->phib_nonzero) h->graph_valid = false;
+  if (nz != h->phib_nonzero) {
+    h->graph_valid = false;
+    ++h->layout_gen;
+  }
   h->phib_nonzero = nz;
   return BX_OK;
 }
@@ -1578,7 +1785,7 @@ int bx_state_upload(bx_handle h, const bx_state* s) {
   BX_CU(cudaMemcpyAsync(h->st_cam, s->cc_at_mem, (size_t)I * M * sizeof(double), cudaMemcpyDefault, st));
   BX_CU(cudaMemsetAsync(h->d_flag, 0, 2 * sizeof(int), st));
   const int tb = 256;
-  bx::k_state_check<<<(M + tb - 1) / tb, tb, 0, st>>>(io, vm_dst, h->st_cam, split ? 1 : 0, h->d_flag);
+  bx::k_state_check<<<(M + tb - 1) / tb, tb, 0, st>>>(io, vm_dst, h->st_cam, split ? 1 : 2, h->d_flag);
   BX_CU(cudaGetLastError());
   int flag[2] = {0, 0};
   BX_CU(cudaMemcpyAsync(flag, h->d_flag, sizeof(flag), cudaMemcpyDeviceToHost, st));
@@ -1586,8 +1793,9 @@ int bx_state_upload(bx_handle h, const bx_state* s) {
   if (flag[0]) return fail(BX_EINVAL, "cc_at_mem must be constant over each cell's membranes");
   // Vmem is constant per cell (minus Phi_b per membrane) in BETSE's full
   // solver with cell_polarizability == 0 (sim.py:2027-2029)
-  if (flag[1]) return fail(BX_EINVAL, "split form: vm must be uniform over each cell's membranes");
+  if (split && flag[1]) return fail(BX_EINVAL, "split form: vm must be uniform over each cell's membranes");
   h->parity = 0;
+  h->vm_uniform = !flag[1];
   if (split) {
     BX_CU(cudaMemsetAsync(h->s_rec[0], 0, (size_t)kRec * h->S * sizeof(float), st));
     BX_CU(cudaMemsetAsync(h->s_cc2, 0, (size_t)I * h->S * sizeof(float2), st));
@@ -1626,7 +1834,8 @@ int bx_state_upload(bx_handle h, const bx_state* s) {
       BX_CU(cudaMemcpyAsync(h->d_Ey, s->E_env_y, (size_t)h->G * sizeof(double), cudaMemcpyDefault, st));
     }
   }
-  if (h->r_ctl) BX_CU(cudaMemsetAsync(h->r_ctl, 0, 2 * sizeof(unsigned), st));   // a fresh state: no timeout
+  for (unsigned* c : {h->r_ctl, h->pl_ctl})
+    if (c) BX_CU(cudaMemsetAsync(c, 0, 2 * sizeof(unsigned), st));   // a fresh state: no timeout
   BX_CU(cudaStreamSynchronize(st));
   h->have_state = true;
   h->have_outputs = false;
@@ -1713,6 +1922,25 @@ int bx_step(bx_handle h, int n_steps, int want_outputs, void* stream) {
       }
     }
   }
+  if (plain_factored(h, false)) {
+    if (!h->vm_uniform && left - tail_out > 0) {
+      // a Vmem that differs within a cell: one step of the per-membrane kernel makes it uniform
+      cudaError_t e = enqueue_step(h, h->parity, false, s);
+      if (e != cudaSuccess) return fail(BX_ECUDA, std::string("step launch: ") + cudaGetErrorString(e));
+      h->parity ^= 1;
+      --left;
+    }
+    if (h->pl_res && left - tail_out >= 2) {
+      while (left - tail_out > 0) {
+        const int n = std::min(left - tail_out, 1 << 20);   // the barrier counter is 32-bit
+        cudaError_t e = launch_plain(h, h->parity, n, true, s);
+        if (e != cudaSuccess) return fail(BX_ECUDA, std::string("resident step launch: ") + cudaGetErrorString(e));
+        h->launches += 1;
+        h->parity ^= (n & 1);
+        left -= n;
+      }
+    }
+  }
   if (left - tail_out >= kGraphChunk) {
     if (h->parity != 0) {
       cudaError_t e = enqueue_step(h, h->parity, false, s);
@@ -1778,14 +2006,15 @@ int bx_status(bx_handle h, bx_step_status* st) {
   st->neg_clamped = (int64_t)v[2];
   st->unstable = (v[0] || v[1]) ? 1 : 0;
   st->precision = h->precision;
-  if (h->r_ctl) {
+  unsigned* rc = h->mode == MODE_SPLIT ? h->r_ctl : h->pl_res ? h->pl_ctl : nullptr;
+  if (rc) {
     // the resident kernel's grid barrier gave up (its wait is bounded): the
     // state of that run is incomplete
     unsigned ctl[2] = {0u, 0u};
-    BX_CU(cudaMemcpy(ctl, h->r_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
+    BX_CU(cudaMemcpy(ctl, rc, sizeof(ctl), cudaMemcpyDeviceToHost));
     if (ctl[1]) {
       h->have_state = false;
-      BX_CU(cudaMemset(h->r_ctl, 0, sizeof(ctl)));
+      BX_CU(cudaMemset(rc, 0, sizeof(ctl)));
       return fail(BX_ECUDA, "the resident kernel's grid barrier timed out; upload the state again");
     }
   }
@@ -1847,10 +2076,27 @@ int bx_time_cell_kernel(bx_handle h, int n, double* ms_per_launch) {
       return BX_OK;
     }
   }
+  const bool plain = h->vm_uniform && plain_factored(h, false);
+  if (plain && h->pl_res && n >= 2) {
+    BX_CU(cudaEventRecord(e0, h->stream));
+    cudaError_t e = launch_plain(h, h->parity, n, true, h->stream);
+    if (e != cudaSuccess) return fail(BX_ECUDA, cudaGetErrorString(e));
+    BX_CU(cudaEventRecord(e1, h->stream));
+    BX_CU(cudaEventSynchronize(e1));
+    float ms = 0.f;
+    BX_CU(cudaEventElapsedTime(&ms, e0, e1));
+    h->parity ^= (n & 1);
+    h->launches++;
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    *ms_per_launch = ms / n;
+    return BX_OK;
+  }
   double tot = 0.0;
   for (int q = 0; q < n; ++q) {
     BX_CU(cudaEventRecord(e0, h->stream));
     cudaError_t e = (h->mode == MODE_SPLIT) ? launch_split(h, h->parity, false, h->stream)
+                    : plain                 ? launch_plain(h, h->parity, 1, false, h->stream)
                                             : launch_cell(h, h->parity, false, h->stream);
     if (e != cudaSuccess) return fail(BX_ECUDA, cudaGetErrorString(e));
     BX_CU(cudaEventRecord(e1, h->stream));
@@ -1889,6 +2135,12 @@ int64_t bx_cell_kernel_bytes(bx_handle h) {
     if (h->ecm) return M * (4 * I + 13 + 4 + 16 * I + gv) + C * (16 * I + 8 * kRec + 12) + B * 4;
     return M * (4 * I + 13 + gv) + C * (16 * I + 8 * kRec + 12) + B * (4 * I + 4);
   }
+  if (plain_factored(h, false)) {
+    // factored plain step: per cell cc in+out, membrane-side concentrations in+out, dsa (8I each),
+    // area, 1/vol, diviterm, row pointer, Vmem in; per membrane the entry, the weight and Vmem out
+    // (gating: area, open fraction in+out, gate entry); per entry 16; per tile the environment part
+    return C * (40 * I + 36) + M * (20 + (h->vgj ? 28 : 0)) + h->pl_nent * 16 + (int64_t)h->pl_ntile * (8 * I + 24);
+  }
   const int64_t w = 8;  // Dm, mem_sa, gj_w width
   // membrane: Dm, vm in+out, m2c, nn, nn_cell, bflag, mem_sa, gj_w (+ map_env and the f*sa
   // export with ECM); cell: cc in+out, cc_mem in+out, cell_vol, diviterm, ptr
@@ -1926,10 +2178,8 @@ int bx_set_launch_config(bx_handle h, int tpb, int kernel) {
   if (kernel < KIND_TILE || kernel > KIND_ION) return fail(BX_EINVAL, "kernel must be 0 to 5");
   if (variant && !(variant == 2 || variant == 4 || variant == 12 || variant == 13 || variant == 14 || variant == 16))
     return fail(BX_EINVAL, "factored-kernel variant must be 2, 4, 12, 13, 14 or 16");
-  if (kernel == KIND_ION && h->mode == MODE_SPLIT)
-    return fail(BX_EINVAL, "the one-lane-per-ion kernel is the plain form's");
-  if (kernel == KIND_ION && (h->polar))
-    return fail(BX_EINVAL, "the one-lane-per-ion kernel has no polarizability variant");
+  if (kernel == KIND_ION && h->mode == MODE_SPLIT) return fail(BX_EINVAL, "kernel 5 is the plain form's");
+  if (kernel == KIND_ION && (h->polar)) return fail(BX_EINVAL, "kernel 5 has no polarizability variant");
   if (kernel != KIND_TILE && kernel != KIND_ION && h->mode != MODE_SPLIT)
     return fail(BX_EINVAL, "the persistent, factored and resident kernels are the split form's");
   if (kernel != KIND_TILE && h->ecm) return fail(BX_EINVAL, "only the tile kernel has an extracellular-space variant");
@@ -1945,10 +2195,12 @@ int bx_set_launch_config(bx_handle h, int tpb, int kernel) {
   const bool had_state = h->have_state;
   int rc;
   if (had_state && (rc = bx_state_download(h, &sv)) != BX_OK) return rc;
+  h->pl_pin = tpb / 4;
   if ((rc = build_partition(h, tpb)) != BX_OK) return rc;
   h->kind = kernel;
   if (variant) h->fact_unroll = variant;
   h->graph_valid = false;
+  ++h->layout_gen;
   if (had_state && (rc = bx_state_upload(h, &sv)) != BX_OK) return rc;
   return BX_OK;
 }
@@ -2032,8 +2284,6 @@ int bx_autotune_table(bx_handle h, int n_steps, int max_rows, int* n_rows, int* 
   else {
     cands = {{256, KIND_TILE, 4}, {128, KIND_TILE, 4}, {64, KIND_TILE, 4}, {32, KIND_TILE, 4},
              {16, KIND_TILE, 4},  {8, KIND_TILE, 4}};
-    if (!h->phib_nonzero && !h->ecm && !h->vgj && !h->ca && !h->polar)
-      for (int mb : {64, 32, 16, 8}) cands.push_back({mb, KIND_ION, 4});
   }
   double best = 1e300;
   int best_tpb = h->tpb, best_kind = h->kind, best_unroll = h->fact_unroll;
@@ -2041,10 +2291,12 @@ int bx_autotune_table(bx_handle h, int n_steps, int max_rows, int* n_rows, int* 
   BX_CU(cudaEventCreate(&e0));
   BX_CU(cudaEventCreate(&e1));
   for (const Cand& cd : cands) {
+    h->pl_pin = cd.tpb / 4;
     if (build_partition(h, cd.tpb) != BX_OK) continue;
     h->kind = cd.kind;
     h->fact_unroll = cd.unroll;
     h->graph_valid = false;
+    ++h->layout_gen;
     if (cd.kind == KIND_RESIDENT) {
       if ((rc = build_resident(h)) != BX_OK) return rc;
       if (h->r_state != 1) continue;            // does not fit: not a candidate
@@ -2069,11 +2321,13 @@ int bx_autotune_table(bx_handle h, int n_steps, int max_rows, int* n_rows, int* 
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  h->pl_pin = best_tpb / 4;
   if ((rc = build_partition(h, best_tpb)) != BX_OK) return rc;
   h->kind = best_kind;
   h->fact_unroll = best_unroll;
   h->tune_ms = best;
   h->graph_valid = false;
+  ++h->layout_gen;
   if ((rc = bx_state_upload(h, &sv)) != BX_OK) return rc;
   BX_CU(cudaMemcpy(h->d_status, status, sizeof(status), cudaMemcpyHostToDevice));
   h->launches = launches0;
@@ -2536,6 +2790,7 @@ struct bx_network {
   cudaGraphExec_t graph = nullptr;   // kGraphChunk coupled steps from ion parity 0
   cudaGraphExec_t graph_net = nullptr;   // kGraphChunk network-only steps
   int graph_net_parity = -1;
+  int64_t graph_gen = -1, graph_net_gen = -1;   // the cluster's layout_gen that they were captured at
 };
 
 namespace {
@@ -2816,15 +3071,18 @@ int bx_network_step(bx_network_handle n, int n_steps, int with_ions, int want_ou
   const int tail = want_outputs ? 1 : 0;
   if (with_ions) {
     if (left - tail >= kGraphChunk) {
-      if (h->parity != 0) {
+      if (h->parity != 0 || !h->vm_uniform) {
         cudaError_t e = net_enqueue_coupled(n, h->parity, false, s);
         if (e != cudaSuccess) return fail(BX_ECUDA, std::string("network step launch: ") + cudaGetErrorString(e));
         h->parity ^= 1;
         --left;
       }
-      if (!n->graph) {
+      if (!n->graph || n->graph_gen != h->layout_gen) {
+        if (n->graph) cudaGraphExecDestroy(n->graph);
+        n->graph = nullptr;
         const int rc = net_capture(n, true, 0, &n->graph);
         if (rc != BX_OK) return rc;
+        n->graph_gen = h->layout_gen;
       }
       while (left - tail >= kGraphChunk) {
         BX_CU(cudaGraphLaunch(n->graph, s));
@@ -2844,12 +3102,13 @@ int bx_network_step(bx_network_handle n, int n_steps, int with_ions, int want_ou
     h->last_step_outputs = want_outputs != 0;
   } else {
     if (left - tail >= kGraphChunk) {
-      if (!n->graph_net || n->graph_net_parity != h->parity) {
+      if (!n->graph_net || n->graph_net_parity != h->parity || n->graph_net_gen != h->layout_gen) {
         if (n->graph_net) cudaGraphExecDestroy(n->graph_net);
         n->graph_net = nullptr;
         const int rc = net_capture(n, false, h->parity, &n->graph_net);
         if (rc != BX_OK) return rc;
         n->graph_net_parity = h->parity;
+        n->graph_net_gen = h->layout_gen;
       }
       while (left - tail >= kGraphChunk) {
         BX_CU(cudaGraphLaunch(n->graph_net, s));

@@ -1,0 +1,516 @@
+// bx_plain.cuh -- the plain FP64 step, factored per cell and per junction.
+//
+// GB300's FP64 pipe (one warp instruction in ~18 cycles per SM) bounds the
+// plain form, so the kernel is built around how few FP64 instructions a step
+// needs.  Without extracellular spaces, Phi_b and polarizability every
+// membrane of a cell sees the same Vmem, the same membrane-side
+// concentrations and the same environment.  So, exactly as real numbers:
+//   * the transmembrane GHK flux of membrane m is Dm_i(m) times one factor
+//     H_i per cell, and the Na/K and Ca pumps are one rate per cell:
+//       sum_m f_i(m) sa(m) = H_i sum_m Dm_i(m) sa(m) + f_pump,i sum_m sa(m);
+//   * the gap-junction flux through membrane m is w(m) D_i Q_i with Q_i
+//     antisymmetric under swapping the two cells (expm1(a) = -expm1(-a) /
+//     exp(-a)), so the two membranes of a junction share one evaluation.
+// A cell with six membranes needs one set of exponentials and the pump once,
+// and three junctions, where k_cell_step (bx_kernels.cuh) needs six of each:
+// about 400 FP64 thread instructions a cell against 1900.  Everything stays
+// FP64; only the order of the sums differs (one rounding per term).
+// Measured per step (k_cell_step with k_env_mix before): 100k cells 403 ->
+// 108 us, 20k cells 85 -> 33 us, 2900 cells 41 -> 10.9 us, 185 cells
+// 40 -> 10.3 us (12.5 with the one-lane-per-ion kernel that this one replaced).
+//
+// One CTA advances one tile: NC consecutive cells of one cluster (NC a power
+// of two), in phases separated by bar.sync:
+//   A  lane per junction ("entry"): the shared exponentials and Q of every ion;
+//      lane per cell: the shared exponentials and the pumps
+//   G  (voltage-gated junctions) lane per membrane: the open fraction, once
+//      per ion as BETSE updates it
+//   C  lane per (cell, ion): the segment sum over the cell's junctions, the
+//      transmembrane sum and the concentration update
+//   D  lane per cell: charge and Vmem; warp per ion: the tile's part of the
+//      environment exchange
+// Entries whose partner cell lies in the tile serve both sides; a halo entry
+// (partner in another tile) is evaluated by both tiles.
+//
+// The environment sum runs over a binary tree of the cluster's cell indices
+// (aligned powers of two, missing leaves zero), so its rounding depends
+// neither on the tile size nor on what else is in a batch.
+//
+// Two launches of the same body (build_plain_layout chooses):
+//   streaming   one step per launch (programmatic dependent launch); the last
+//               tile of every 32 adds their parts, the last such group of the
+//               cluster the groups' (ticket counters), and mixes the environment
+//   resident    many steps per cooperative launch, one tile per CTA, all of
+//               them co-resident: the state stays in shared memory, tiles
+//               exchange Vmem and concentrations through L2 and meet once a
+//               step at a bounded grid barrier; the cells' own exponentials
+//               and the junctions inside the tile are evaluated while the
+//               barrier completes.
+#pragma once
+#include "bx_kernels.cuh"
+#include "bx_sync.cuh"
+
+namespace bx {
+
+constexpr int kPlainT = 256;            // threads per CTA
+constexpr int kPlainNone = INT32_MIN;   // mem_ent: no junction
+
+struct PlainGeom {
+  int C, M, ntile;
+  const int2* tile;        // [ntile] {first cell, cells}
+  const int* tile_cl;      // [ntile] cluster
+  const int* cl_tile;      // [ncl + 1] first tile of each cluster
+  const int* cl_group;     // [ncl + 1] first group (of 32 tiles) of each cluster
+  const int* ent_ptr;      // [ntile + 1] entries of each tile
+  const int* n_local;      // [ntile] of them, those whose partner is in the tile (they come first)
+  const int4* ent;         // {own cell (in the tile), partner cell (in the tile; halo: global), partner's first membrane, 0}
+  const int* mem_ent;      // [M] the membrane's entry in its tile, ~entry on the partner's side, kPlainNone on the boundary
+  const int* mem_gate;     // [M] (gated) entry whose |vgj| gates the membrane
+  const int* cell_ptr;     // [C + 1]
+  const int* m2c;          // [M]
+  const double* mem_w;     // [M] gj_weight * mem_sa
+  const double* mem_sa;    // [M]
+  const double* dsa;       // [I][C] sum of Dm_i * mem_sa over the cell's membranes
+  const double* sa;        // [C] sum of mem_sa
+  const double* ivol;      // [C] 1 / cell_vol
+  const double* diviterm;  // [C]
+};
+
+struct PlainRun {
+  double* vm[2];           // Vmem [M], read from [0] first
+  double* ccm[2];          // membrane-side concentrations [I][C]
+  int n_steps;             // resident: steps of this launch
+  int nc_max, ne_max, nm_max;   // largest tile: cells, entries, membranes (shared memory)
+  double* part;            // [ntile][I] tile parts of the environment exchange (resident: two copies)
+  double* gpart;           // [groups + ...][I] group parts and the levels above them
+  unsigned* ticket;        // [groups + ncl] zero between steps
+  double* cenv;            // [ncl][I]
+  const double* env_scale; // [ncl]
+  unsigned* ctl;           // resident: barrier counter, timeout flag
+  long long timeout_ns;
+};
+
+// Shared memory of one CTA, in doubles, for the largest tile.
+struct PlainSmem {
+  int q, v, cm, cc, x, s1, k, env, lvl, ga, gg, total;
+  __host__ __device__ PlainSmem(int nc, int ne, int nm, int I, bool gated) {
+    int o = 0;
+    auto take = [&](int n) { const int at = o; o += n; return at; };
+    q = take(ne * I);
+    v = take(nc);
+    cm = take(nc * I);
+    cc = take(nc * I);
+    x = take(nc * I);
+    s1 = take(nc * I);
+    k = take(nc * 7);
+    env = take(kMaxIons);
+    lvl = take(8 * (kPlainT / 32));
+    ga = take(gated ? 2 * ne : 0);
+    gg = take(gated ? nm * I : 0);
+    total = o;
+  }
+};
+enum PlainCell { PK_K1 = 0, PK_E1, PK_K2, PK_E2, PK_FNA, PK_DTV, PK_FCA };
+
+// BETSE's six-ion set as constants (ZP = 1) or the parameters' ions (ZP = 0)
+template <int ZP> struct PlainIons {
+  __device__ static int n(const StepConst& k) { return k.I; }
+  __device__ static int zc(const StepConst& k, int i) { return k.zcode[i]; }
+  static constexpr int NI = kMaxIons;
+};
+template <> struct PlainIons<1> {
+  __device__ static constexpr int n(const StepConst&) { return 6; }
+  __device__ static constexpr int zc(const StepConst&, int i) { return i < 2 ? 1 : i == 3 ? 2 : -1; }
+  static constexpr int NI = 6;
+};
+
+// The flux factor of charge code zc for a side A -> B: ghk_flux without Dc,
+// from kr = a1 / d / expm1(-a1) and kr2 = 2 kr / (2 + expm1(-a1)).
+__device__ __forceinline__ double plain_ghk(int zc, double zval, double v_nonce, double F_RT, double inv_d, double kr,
+                                            double kr2, double e1, double e2, double cA, double cB) {
+  switch (zc) {
+    case 1: return kr * (cB - cA * e1);
+    case -1: return kr * (cB * e1 - cA);
+    case 2: return kr2 * (cB - cA * e2);
+    case -2: return kr2 * (cB * e2 - cA);
+    default: {
+      const double a = ((zval + kNonce) * v_nonce) * F_RT;
+      const double ea = exp(-a), den = -expm1(-a);
+      return -(a * inv_d) * ((cB - cA * ea) / den);
+    }
+  }
+}
+
+// w with its sign flipped when s is negative
+__device__ __forceinline__ double signed_like(double w, int s) {
+  return __hiloint2double(__double2hiint(w) ^ (s & 0x80000000), __double2loint(w));
+}
+
+// Sums of eight quantities over the 32 lanes of a warp, every pair of
+// neighbouring lanes first (the tree of aligned powers of two): three
+// exchange rounds that halve the quantities a lane keeps, then two plain
+// ones, nine additions in all.  Lane l returns quantity
+// 4 (l & 1) + 2 ((l >> 1) & 1) + ((l >> 2) & 1).
+__device__ __forceinline__ double warp_tree8(const double (&a)[8]) {
+  const int lane = threadIdx.x & 31;
+  double b[4], c[2], d;
+  const bool h1 = lane & 1, h2 = lane & 2, h4 = lane & 4;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const double keep = h1 ? a[j + 4] : a[j], send = h1 ? a[j] : a[j + 4];
+    b[j] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const double keep = h2 ? b[j + 2] : b[j], send = h2 ? b[j] : b[j + 2];
+    c[j] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+  }
+  {
+    const double keep = h4 ? c[1] : c[0], send = h4 ? c[0] : c[1];
+    d = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+  }
+  d += __shfl_xor_sync(0xffffffffu, d, 8);
+  d += __shfl_xor_sync(0xffffffffu, d, 16);
+  return d;
+}
+__device__ __forceinline__ int tree8_ion() {
+  const int lane = threadIdx.x & 31;
+  return 4 * (lane & 1) + 2 * ((lane >> 1) & 1) + ((lane >> 2) & 1);
+}
+
+// rows [0, n) of src ([.][I]), 32 at a time, into dst rows of their sums:
+// warps of the CTA in turn.  The caller synchronises.
+__device__ __forceinline__ void tree_rows(const double* src, int n, int I, double* dst, int stride_dst) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int c = threadIdx.x >> 5; c * 32 < n; c += nw) {
+    double a[8];
+    const int r = c * 32 + lane;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] = (i < I && r < n) ? __ldcg(src + (size_t)r * I + i) : 0.0;
+    const double s = warp_tree8(a);
+    const int i = tree8_ion();
+    if (lane < 8 && i < I) dst[(size_t)c * stride_dst + i] = s;
+  }
+}
+
+template <int ZP, bool GATED, bool RES>
+__global__ void __launch_bounds__(kPlainT, RES ? 1 : 3)
+k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r) {
+  using IS = PlainIons<ZP>;
+  constexpr int T = kPlainT, NI = IS::NI;
+  extern __shared__ double sm[];
+  __shared__ int s_flag;
+  const int I = IS::n(k);
+  const PlainSmem L(r.nc_max, r.ne_max, r.nm_max, I, GATED);
+  double *sQ = sm + L.q, *sv = sm + L.v, *scm = sm + L.cm, *scc = sm + L.cc, *sx = sm + L.x, *s1 = sm + L.s1,
+         *sk = sm + L.k, *senv = sm + L.env, *slvl = sm + L.lvl, *sga = sm + L.ga, *sgg = sm + L.gg;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, b = blockIdx.x;
+
+#if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 900)
+  if (!RES) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+  }
+#endif
+  const int2 tl = g.tile[b];
+  const int c0 = tl.x, nc = tl.y;
+  const int cl = g.tile_cl[b];
+  const int m0 = g.cell_ptr[c0], m1 = g.cell_ptr[c0 + nc];
+  const int e0 = g.ent_ptr[b], ne = g.ent_ptr[b + 1] - e0, nl = g.n_local[b];
+  const double pcoef = p.pump_coef[cl];
+  const double *vin = r.vm[0], *cin = r.ccm[0];
+  double *vout = r.vm[1], *cout = r.ccm[1];
+
+  // ---- the tile's state
+  for (int q = t; q < nc * I; q += T) {
+    const int lc = q / I, i = q - lc * I;
+    scm[q] = cin[(size_t)i * g.C + c0 + lc];
+    scc[q] = p.cc[(size_t)i * g.C + c0 + lc];
+  }
+  for (int q = t; q < nc; q += T) sv[q] = vin[g.cell_ptr[c0 + q]];
+  if (t < I) senv[t] = r.cenv[(size_t)cl * I + t];
+  if (t < 8 * (T / 32)) slvl[t] = 0.0;
+  __syncthreads();
+
+  // junction entry e: Q of every ion from the own side into the partner
+  auto entry = [&](int e, bool halo) {
+    const int4 en = g.ent[e0 + e];
+    const double v1 = sv[en.x] + kNonce;
+    const double vn = halo ? __ldcg(vin + en.z) : sv[en.y];
+    double cB[NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      if (i < I) cB[i] = halo ? __ldcg(cin + (size_t)i * g.C + en.y) : scm[en.y * I + i];
+    const double vgj = (vn + kNonce) - v1;        // update_gj, sim.py:2166
+    const double vg1 = vgj + kNonce;
+    GhkShared<double> s;
+    s.init(vg1, k.F_RT);
+    const double kr = s.a1 * k.inv_gj_len * s.r, kr2 = 2.0 * kr * s.q2, e2 = s.e1 * s.e1;
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      if (i < I)
+        sQ[e * I + i] = plain_ghk(IS::zc(k, i), k.z[i], vg1, k.F_RT, k.inv_gj_len, kr, kr2, s.e1, e2,
+                                  scm[en.x * I + i], cB[i]);
+    if (GATED) {
+      // Gap_Junction.run (channels/gap_junction.py:52-81): one implicit Euler
+      // update per ion with these two coefficients (phase G)
+      const double V1 = 1.0e3 * fabs(vgj);
+      const double al = kGjLambda * exp(-kGjA1 * (V1 - k.gj_vth));
+      double be = kGjLambda * exp(kGjA2 * (V1 - k.gj_vth));
+      be = be / (1.0 + 50.0 * be);
+      sga[2 * e] = k.gj_dt_ms * (al + be * k.gj_min);
+      sga[2 * e + 1] = 1.0 / (1.0 + al * k.gj_dt_ms + be * k.gj_dt_ms);
+    }
+  };
+  // cell lc: the shared exponentials of its Vmem
+  auto cell_exp = [&](int lc) {
+    GhkShared<double> s;
+    s.init(sv[lc] + kNonce, k.F_RT);
+    const double kr = s.a1 * k.inv_tm * s.r;
+    double* o = sk + lc * 7;
+    o[PK_K1] = kr;
+    o[PK_E1] = s.e1;
+    o[PK_K2] = 2.0 * kr * s.q2;
+    o[PK_E2] = s.e1 * s.e1;
+    o[PK_DTV] = k.dt * g.ivol[c0 + lc];
+  };
+  // cell lc: its pumps, times the cell's membrane area
+  auto cell_pump = [&](int lc) {
+    double* o = sk + lc * 7;
+    const double sa = g.sa[c0 + lc], e1 = o[PK_E1];
+    const double* cm = scm + lc * I;
+    double fna = 0.0;
+    if (pcoef != 0.0)                             // Na/K-ATPase (sim.py:1196-1234)
+      fna = pump_fna<double>(k, pcoef, e1, cm[k.iNa], senv[k.iNa], cm[k.iK], senv[k.iK]);
+    o[PK_FNA] = fna * sa;
+    if (k.iCa >= 0)                               // ca_handler (sim.py:2126-2155)
+      o[PK_FCA] = pump_fca<double>(k, e1, scc[lc * I + k.iCa], senv[k.iCa]) * sa;
+  };
+
+  const int nlp = (nl + 31) & ~31;                // whole warps of local entries, then the cells
+  unsigned bad = 0, neg = 0, nanv = 0;
+  int step = 0;
+  const int n_steps = RES ? r.n_steps : 1;
+  for (; step < n_steps; ++step) {
+    // ---- A: what needs only the tile
+    for (int q = t; q < nlp + nc; q += T) {
+      if (q < nlp) {
+        if (q < nl) entry(q, false);
+      } else {
+        cell_exp(q - nlp);
+        if (!RES || step == 0) cell_pump(q - nlp);
+      }
+    }
+    if (RES && step > 0) {
+      // the other tiles' step: the environment (every CTA adds the same tile
+      // parts in the same tree), then the pumps
+      if (!res_wait(r.ctl, (unsigned)step * gridDim.x, r.timeout_ns, &s_flag)) break;
+      const double* part = r.part + (size_t)(step & 1) * g.ntile * I;
+      tree_rows(part, g.ntile, I, slvl, 8);
+    }
+    for (int q = nl + t; q < ne; q += T) entry(q, true);
+    __syncthreads();
+    if (RES && step > 0) {
+      if (t < I) {
+        // at most eight rows of 32 tiles (the launch rule)
+        const double a = (slvl[t] + slvl[8 + t]) + (slvl[16 + t] + slvl[24 + t]);
+        const double c = (slvl[32 + t] + slvl[40 + t]) + (slvl[48 + t] + slvl[56 + t]);
+        senv[t] = senv[t] - (a + c) * r.env_scale[cl];
+      }
+      __syncthreads();
+      for (int q = t; q < nc; q += T) cell_pump(q);
+      __syncthreads();
+    }
+    // ---- G: the gated open fractions, one lane per membrane
+    if (GATED) {
+      for (int m = m0 + t; m < m1; m += T) {
+        const int e = g.mem_gate[m];
+        const double ga = sga[2 * e], gr = sga[2 * e + 1], sa = g.mem_sa[m];
+        double gg = p.gjo[m];
+        for (int i = 0; i < I; ++i) {
+          gg = k.gj_block * ((gg + ga) * gr);
+          sgg[(m - m0) * I + i] = gg * sa;
+        }
+        p.gjo[m] = gg;
+      }
+      __syncthreads();
+    }
+    // ---- C: lane per (cell, ion): update_all_concs
+    const bool last = step + 1 == n_steps;
+    for (int q = t; q < nc * I; q += T) {
+      const int lc = q / I, i = q - lc * I, c = c0 + lc;
+      const int a0 = g.cell_ptr[c], a1 = g.cell_ptr[c + 1];
+      double s2 = 0.0;
+      for (int m = a0; m < a1; ++m) {
+        const int me = g.mem_ent[m];
+        if (me == kPlainNone) continue;
+        const double w = GATED ? sgg[(m - m0) * I + i] : g.mem_w[m];
+        s2 += signed_like(w, ~me) * sQ[(me >= 0 ? me : ~me) * I + i];   // -w on the own side
+      }
+      const double* o = sk + lc * 7;
+      double S = g.dsa[(size_t)i * g.C + c] * plain_ghk(IS::zc(k, i), k.z[i], sv[lc] + kNonce, k.F_RT, k.inv_tm,
+                                                       o[PK_K1], o[PK_K2], o[PK_E1], o[PK_E2], senv[i], scm[q]);
+      if (i == k.iNa) S = o[PK_FNA] + S;
+      else if (i == k.iK) S = -(2.0 / 3.0) * o[PK_FNA] + S;
+      if (i == k.iCa) S = S + o[PK_FCA];
+      s1[q] = S;
+      double x = scc[q] + S * o[PK_DTV];              // update_Co, sim_toolbox.py:1182-1183
+      sx[q] = x;
+      cout[(size_t)i * g.C + c] = x;        // cc_at_mem = cX_cell[mem_to_cells]
+      const double dg = GATED ? k.dgj_gs[i] : k.dgj_gs[i] * k.gj_block;
+      x = x + (dg * s2) * o[PK_DTV];                  // gap-junction term, sim.py:2105-2108
+      const int hx = __double2hiint(x);               // integer tests: no FP64 pipe
+      const bool nan = (hx & 0x7fffffff) > 0x7ff00000 || ((hx & 0x7fffffff) == 0x7ff00000 && __double2loint(x));
+      bad += nan;
+      if (hx < 0 && !nan && ((hx & 0x7fffffff) | __double2loint(x))) { x = 0.0; ++neg; }   // no_negs
+      scc[q] = x;
+      if (last) p.cc[(size_t)i * g.C + c] = x;
+    }
+    __syncthreads();
+    // ---- D: Vmem (the last warps) and the tile's part of the environment
+    for (int lc = T - 1 - t; lc < nc; lc += T) {
+      double rho = 0.0;                               // rho_cells, ion_current.py:19
+#pragma unroll
+      for (int i = 0; i < NI; ++i)
+        if (i < I) rho += k.zF[i] * scc[lc * I + i];
+      const double v = k.inv_cm * (rho * g.diviterm[c0 + lc]);   // sim.py:2027-2029
+      sv[lc] = v;
+      const int a0 = g.cell_ptr[c0 + lc];
+      if (v != v) nanv += g.cell_ptr[c0 + lc + 1] - a0;
+      if (RES) vout[a0] = v;                 // what the other tiles read
+    }
+    double* part = r.part + (RES ? (size_t)((step + 1) & 1) * g.ntile * I : (size_t)0);
+    for (int i = warp; i < I; i += T / 32) {
+      // lane l: cells [l, l + 1) ... or a run of 2 or 4, pairs first
+      double a;
+      auto at = [&](int lc) { return lc < nc ? s1[lc * I + i] : 0.0; };
+      if (r.nc_max <= 32) a = at(lane);
+      else if (r.nc_max <= 64) a = at(2 * lane) + at(2 * lane + 1);
+      else a = (at(4 * lane) + at(4 * lane + 1)) + (at(4 * lane + 2) + at(4 * lane + 3));
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (lane == 0) part[(size_t)b * I + i] = a;
+    }
+    if (RES) {
+      for (int q = t; q < nc * I; q += T) scm[q] = sx[q];
+      double* w = vout; vout = const_cast<double*>(vin); vin = w;
+      w = cout; cout = const_cast<double*>(cin); cin = w;
+      __syncthreads();
+      if (t == 0) {
+        __threadfence();
+        res_arrive(r.ctl);
+      }
+    }
+  }
+  if (bad) atomicAdd(&p.status[1], (unsigned long long)bad);
+  if (neg) atomicAdd(&p.status[2], (unsigned long long)neg);
+  if (nanv) atomicAdd(&p.status[0], (unsigned long long)nanv);
+
+  if (RES) {
+    if (step < n_steps) return;                       // the barrier gave up
+    // Vmem of every membrane, and the environment of the last step (CTA 0)
+    double* vfin = const_cast<double*>(vin);
+    for (int m = m0 + t; m < m1; m += T) vfin[m] = sv[g.m2c[m] - c0];
+    if (b == 0) {
+      if (!res_wait(r.ctl, (unsigned)step * gridDim.x, r.timeout_ns, &s_flag)) return;
+      tree_rows(r.part + (size_t)(step & 1) * g.ntile * I, g.ntile, I, slvl, 8);
+      __syncthreads();
+      if (t < I) {
+        const double a = (slvl[t] + slvl[8 + t]) + (slvl[16 + t] + slvl[24 + t]);
+        const double c = (slvl[32 + t] + slvl[40 + t]) + (slvl[48 + t] + slvl[56 + t]);
+        r.cenv[t] = senv[t] - (a + c) * r.env_scale[0];
+      }
+    }
+    return;
+  }
+
+  // ---- streaming: Vmem of every membrane, then the environment by tickets
+  __syncthreads();
+  for (int m = m0 + t; m < m1; m += T) vout[m] = sv[g.m2c[m] - c0];
+  const int ct0 = g.cl_tile[cl], nt = g.cl_tile[cl + 1] - ct0;
+  const int grp = (b - ct0) >> 5, ngrp = (nt + 31) >> 5;
+  const int g0 = g.cl_group[cl];
+  unsigned* tk = r.ticket + g0 + cl;                  // the cluster's groups, then its own counter
+  if (t == 0) {
+    __threadfence();
+    const unsigned n = (unsigned)min(32, nt - 32 * grp);
+    s_flag = atomicAdd(&tk[grp], 1u) == n - 1u;
+  }
+  __syncthreads();
+  if (!s_flag) return;
+  __threadfence();
+  // rows of parts, level by level: 32 tiles -> group -> 32 groups -> ...
+  double* lv = r.gpart + (size_t)(2 * g0 + 8 * cl) * I;
+  {
+    const double* src = r.part + (size_t)(ct0 + 32 * grp) * I;
+    if (warp == 0) {
+      double a[8];
+      const int n = min(32, nt - 32 * grp);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = (i < I && lane < n) ? __ldcg(src + (size_t)lane * I + i) : 0.0;
+      const double s = warp_tree8(a);
+      const int i = tree8_ion();
+      if (lane < 8 && i < I) lv[(size_t)grp * I + i] = s;
+    }
+  }
+  __syncthreads();
+  if (t == 0) {
+    tk[grp] = 0u;
+    __threadfence();
+    s_flag = atomicAdd(&tk[ngrp], 1u) == (unsigned)ngrp - 1u;
+  }
+  __syncthreads();
+  if (!s_flag) return;
+  __threadfence();
+  int n = ngrp;
+  while (n > 1) {
+    double* up = lv + (size_t)n * I;
+    tree_rows(lv, n, I, up, I);
+    __threadfence_block();
+    __syncthreads();
+    lv = up;
+    n = (n + 31) >> 5;
+  }
+  if (t < I) {
+    double* ce = r.cenv + (size_t)cl * I + t;
+    *ce = *ce - __ldcg(lv + t) * r.env_scale[cl];     // sim_toolbox.py:1196-1205
+  }
+  if (t == 0) tk[ngrp] = 0u;
+}
+
+// sum of Dm_i * mem_sa over the cell's membranes, lane per (ion, cell)
+static __global__ void k_plain_dsa(int C, int M, int I, const int* __restrict__ cell_ptr,
+                                   const double* __restrict__ Dm, const double* __restrict__ mem_sa, double* dsa) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
+  if (c >= C) return;
+  double s = 0.0;
+  for (int m = cell_ptr[c]; m < cell_ptr[c + 1]; ++m) s += Dm[(size_t)i * M + m] * mem_sa[m];
+  dsa[(size_t)i * C + c] = s;
+}
+
+// the membranes' junction weights times area, the cells' areas and 1 / cell_vol
+static __global__ void k_plain_static(int C, const int* __restrict__ cell_ptr, const double* __restrict__ gj_w,
+                                      const double* __restrict__ mem_sa, const double* __restrict__ cell_vol,
+                                      double* mem_w, double* sa, double* ivol) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= C) return;
+  double s = 0.0;
+  for (int m = cell_ptr[c]; m < cell_ptr[c + 1]; ++m) {
+    mem_w[m] = gj_w[m] * mem_sa[m];
+    s += mem_sa[m];
+  }
+  sa[c] = s;
+  ivol[c] = 1.0 / cell_vol[c];
+}
+
+// launchers (bx_step_f64_small.cu)
+cudaError_t launch_plain_step(bool six, bool gated, cudaStream_t s, const PlainGeom& g, const StepPtrs& p,
+                              const StepConst& k, const PlainRun& r);
+cudaError_t launch_plain_resident(bool six, bool gated, cudaStream_t s, const PlainGeom& g, const StepPtrs& p,
+                                  const StepConst& k, const PlainRun& r);
+// CTAs of the resident form that fit one SM with this much shared memory (0: none)
+cudaError_t plain_resident_per_sm(bool six, bool gated, size_t smem, int* per_sm);
+// the shared-memory limit of both forms, raised once per device
+cudaError_t plain_smem_attr(bool six, bool gated, size_t smem);
+
+}  // namespace bx

@@ -30,7 +30,8 @@ __device__ __forceinline__ double state_phib(const StateIO& io, int m) {
 
 // The checks of bx_state_upload, one thread per membrane: flag[0] when
 // cc_at_mem differs from its cell's first membrane (a NaN differs too), flag[1]
-// (with check_vm, the split form) when vm + Phi_b is not uniform over the cell.
+// when vm + Phi_b is not uniform over the cell (check_vm 1, the split form: to
+// rounding; 2, the plain form: bit for bit, which its factored step needs).
 __global__ void k_state_check(StateIO io, const double* __restrict__ vm, const double* __restrict__ cam,
                               int check_vm, int* flag) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
@@ -41,7 +42,9 @@ __global__ void k_state_check(StateIO io, const double* __restrict__ vm, const d
     if (cam[(size_t)i * io.M + m] != cam[(size_t)i * io.M + f]) { atomicOr(&flag[0], 1); break; }
   if (check_vm) {
     const double v0 = vm[f] + state_phib(io, f), v = vm[m] + state_phib(io, m);
-    if (fabs(v - v0) > 1e-12 * fabs(v0) + 1e-18) atomicOr(&flag[1], 1);
+    // (a polarizable state differs everywhere: no more atomics once it is known)
+    if (check_vm == 2 ? !(v == v0) : fabs(v - v0) > 1e-12 * fabs(v0) + 1e-18)
+      if (!*(volatile int*)&flag[1]) atomicOr(&flag[1], 1);
   }
 }
 
