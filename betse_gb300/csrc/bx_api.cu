@@ -112,7 +112,7 @@ struct bx_cluster {
   // ---- geometry (device)
   int *d_cell_ptr = nullptr, *d_m2c = nullptr, *d_nn = nullptr, *d_nn_cell = nullptr,
       *d_map_env = nullptr, *d_blk = nullptr, *d_blk_cl = nullptr, *d_cl_blk = nullptr,
-      *d_env_ptr = nullptr, *d_env_mem = nullptr;
+      *d_env_ptr = nullptr, *d_env_slot = nullptr;
   uint8_t *d_bflag = nullptr, *d_touched = nullptr, *d_lcell = nullptr;
   double *d_mem_sa = nullptr, *d_gj_w = nullptr, *d_nx = nullptr, *d_ny = nullptr, *d_swm = nullptr,
          *d_swo = nullptr, *d_cell_vol = nullptr, *d_cell_sa = nullptr, *d_diviterm = nullptr;
@@ -147,7 +147,7 @@ struct bx_cluster {
   // ---- factored plain step (bx_plain.cuh)
   bool vm_uniform = false;         // Vmem is one value per cell (the factored step needs it)
   int pl_pin = 0;                  // cells per tile pinned by a launch configuration (0: by size)
-  int pl_nc = 0, pl_ntile = 0, pl_ngroup = 0, pl_ne = 0, pl_nm = 0;   // cells per tile, tiles, groups, largest tile
+  int pl_nc = 0, pl_ntile = 0, pl_ne = 0, pl_nm = 0;   // cells per tile, tiles, largest tile
   bool pl_res = false;             // the resident form fits: one tile per co-resident CTA
   unsigned char* pl_base = nullptr;   // the one allocation that the pl_ pointers point into
   int2* pl_tile = nullptr;
@@ -223,7 +223,7 @@ namespace {
 void free_all(bx_cluster* h) {
   void* ptrs[] = {
       h->d_cell_ptr, h->d_m2c, h->d_nn, h->d_nn_cell, h->d_map_env, h->d_blk, h->d_blk_cl, h->d_cl_blk,
-      h->d_env_ptr, h->d_env_mem, h->d_bflag, h->d_touched, h->d_lcell, h->d_mem_sa, h->d_gj_w, h->d_nx,
+      h->d_env_ptr, h->d_env_slot, h->d_bflag, h->d_touched, h->d_lcell, h->d_mem_sa, h->d_gj_w, h->d_nx,
       h->d_ny, h->d_swm, h->d_swo, h->d_cell_vol, h->d_cell_sa, h->d_diviterm, h->d_mem_sa_f,
       h->d_gj_w_f, h->d_gjw0_f, h->d_dtv, h->d_dvc, h->d_Dm, h->d_Dm_f, h->d_vm[0], h->d_vm[1],
       h->d_ccm[0], h->d_ccm[1], h->d_cc, h->s_cc2, h->s_rec[0], h->s_rec[1], h->s_count,
@@ -390,6 +390,7 @@ bx::DevGeom dev_geom(const bx_cluster* h) {
   g.sw_mem = h->d_swm; g.sw_o = h->d_swo; g.cell_vol = h->d_cell_vol; g.cell_sa = h->d_cell_sa;
   g.diviterm = h->d_diviterm; g.blk_cell = h->d_blk; g.blk_cluster = h->d_blk_cl;
   g.R_rads = h->d_Rrads;
+  g.env_slot = h->d_env_slot;
   return g;
 }
 
@@ -431,6 +432,7 @@ bx::SplitPtrs split_ptrs(bx_cluster* h, int parity) {
   p.o_drho = h->o_drho;
   p.cenv_grid = h->ecm ? h->d_cenv : nullptr;
   p.mfs = h->d_mem_flux_sa;
+  p.env_slot = h->d_env_slot;
   p.gjo = h->t_gjo;
   p.o_gjopen = h->o_gjopen;
   p.ca_env = ca_env_ptr(h);
@@ -452,11 +454,11 @@ bool fact_eligible(const bx_cluster* h, bool out) {
   return h->mode == MODE_SPLIT && !out && !h->phib_nonzero && !h->ecm && !h->vgj && !h->ca;
 }
 
-// The plain form's factored step (bx_plain.cuh) needs one Vmem and one
-// environment per cell: no Phi_b, no extracellular spaces, no polarizability,
-// no outputs.
+// The plain form's factored step (bx_plain.cuh) needs one Vmem per cell: no
+// Phi_b, no polarizability, no outputs; with extracellular spaces no Ca-ATPase
+// (which reads the grid between its update and the scatter).
 bool plain_factored(const bx_cluster* h, bool out) {
-  return h->mode == MODE_PLAIN && !out && !h->phib_nonzero && !h->ecm && !h->polar;
+  return h->mode == MODE_PLAIN && !out && !h->phib_nonzero && !h->polar && !(h->ecm && h->ca);
 }
 
 bool is_betse_six_ions(const bx_cluster* h) {
@@ -529,13 +531,31 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), unsigned grid, unsigned block, cu
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+// The grid's Nernst-Planck flux in nthreads-wide blocks of the cell kernel's
+// launch (with the Ca-ATPase it has run before, and with sharpness < 1 the
+// split form's stencil is FP64: a launch of its own)
+bx::EnvNp env_np(const bx_cluster* h, int nthreads) {
+  bx::EnvNp n{};
+  if (!h->ecm) return n;
+  n.cenv = h->d_cenv; n.Denv = h->d_Denv; n.Ex = h->d_Ex; n.Ey = h->d_Ey; n.fx = h->d_fx; n.fy = h->d_fy;
+  n.e = make_env_const(h);
+  if (nthreads) n.nblk = (h->G * h->I + nthreads - 1) / nthreads;
+  return n;
+}
+bool env_flux_in_cell_launch(const bx_cluster* h, bool out) {
+  if (!h->ecm || h->ca) return false;
+  return h->mode == MODE_SPLIT ? !(h->par.sharpness < 1.0) : h->vm_uniform && plain_factored(h, out);
+}
+
 template <int TPB, bool OUT, bool PHIB, bool ECM>
 cudaError_t launch_split_t(bx_cluster* h, int parity, cudaStream_t s) {
+  const bx::EnvNp en = env_np(h, ECM && env_flux_in_cell_launch(h, OUT) ? TPB : 0);
+  const unsigned grid = (unsigned)(h->nblk + en.nblk);
   if (is_betse_six_ions(h))
-    return launch_pdl(bx::k_split_step<TPB, kRec, 1, OUT, PHIB, ECM>, (unsigned)h->nblk, TPB, s, split_geom(h),
-                      split_ptrs(h, parity), make_split_const(h));
-  return launch_pdl(bx::k_split_step<TPB, kRec, 0, OUT, PHIB, ECM>, (unsigned)h->nblk, TPB, s, split_geom(h),
-                    split_ptrs(h, parity), make_split_const(h));
+    return launch_pdl(bx::k_split_step<TPB, kRec, 1, OUT, PHIB, ECM>, grid, TPB, s, split_geom(h),
+                      split_ptrs(h, parity), make_split_const(h), en);
+  return launch_pdl(bx::k_split_step<TPB, kRec, 0, OUT, PHIB, ECM>, grid, TPB, s, split_geom(h),
+                    split_ptrs(h, parity), make_split_const(h), en);
 }
 
 template <int TPB, bool OUT, bool PHIB>
@@ -795,6 +815,7 @@ cudaError_t launch_plain(bx_cluster* h, int parity, int n, bool resident, cudaSt
   g.mem_ent = h->pl_mem_ent; g.mem_gate = h->pl_mem_gate; g.cell_ptr = h->d_cell_ptr; g.m2c = h->d_m2c;
   g.mem_w = h->pl_mem_w; g.mem_sa = h->d_mem_sa; g.dsa = h->pl_dsa; g.sa = h->pl_sa; g.ivol = h->pl_ivol;
   g.diviterm = h->d_diviterm;
+  g.map_env = h->d_map_env; g.env_slot = h->d_env_slot; g.G = h->G;
   bx::PlainRun r{};
   r.vm[0] = h->d_vm[parity]; r.vm[1] = h->d_vm[parity ^ 1];
   r.ccm[0] = h->d_ccm[parity]; r.ccm[1] = h->d_ccm[parity ^ 1];
@@ -806,7 +827,7 @@ cudaError_t launch_plain(bx_cluster* h, int parity, int n, bool resident, cudaSt
   const bx::StepPtrs p = step_ptrs(h, parity);
   const bool six = is_betse_six_ions(h);
   return resident ? bx::launch_plain_resident(six, h->vgj, s, g, p, k, r)
-                  : bx::launch_plain_step(six, h->vgj, s, g, p, k, r);
+                  : bx::launch_plain_step(six, h->vgj, h->ecm, s, g, p, k, r, env_np(h, h->ecm ? bx::kPlainT : 0));
 }
 
 // The extracellular grid of one step (update_ecm, update_Co's ECM term, get_current's E_env).
@@ -818,57 +839,56 @@ cudaError_t launch_plain(bx_cluster* h, int parity, int n, bool resident, cudaSt
 cudaError_t enqueue_env_pre(bx_cluster* h, cudaStream_t s) {
   bx::EnvConst ec = make_env_const(h);
   const int gi = env_grid(h->G * h->I);
-  bx::k_env_np_flux<double><<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_Denv, h->d_Ex, h->d_Ey, h->d_fx, h->d_fy, ec);
+  bx::k_env_np_flux<double><<<gi, kEnvTPB, 0, s>>>(env_np(h, 0));
   bx::k_env_update<false><<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_fx, h->d_fy, h->d_env_ptr,
-                                                h->d_env_mem, h->d_mem_flux_sa, h->M, ec);
+                                                h->d_mem_flux_sa, ec);
   h->launches += 2;
   if (h->par.sharpness < 1.0) {
-    bx::k_env_integrate_scatter<false><<<gi, kEnvTPB, 0, s>>>(h->d_cnew, h->d_tmp2, h->d_env_ptr, h->d_env_mem,
-                                                             h->d_mem_flux_sa, h->M, ec);
+    bx::k_env_integrate_scatter<false><<<gi, kEnvTPB, 0, s>>>(h->d_cnew, h->d_tmp2, h->d_env_ptr, h->d_mem_flux_sa, ec);
     h->launches += 1;
   }
   return cudaGetLastError();
 }
 
-cudaError_t enqueue_env(bx_cluster* h, bool out, cudaStream_t s) {
+// flux_done: the cell kernel's launch has computed the Nernst-Planck flux
+cudaError_t enqueue_env(bx_cluster* h, bool out, bool flux_done, cudaStream_t s) {
   bx::EnvConst ec = make_env_const(h);
   const int gg = env_grid(h->G);
   const int gi = env_grid(h->G * h->I);   // one thread per (ion, grid cell)
+  const bool split = h->mode == MODE_SPLIT && !(h->par.sharpness < 1.0);   // FP32 stencils around FP64 state
+  if (!flux_done && !h->ca) {
+    if (split) bx::k_env_np_flux<float><<<gi, kEnvTPB, 0, s>>>(env_np(h, 0));
+    else bx::k_env_np_flux<double><<<gi, kEnvTPB, 0, s>>>(env_np(h, 0));
+    h->launches += 1;
+  }
   if (h->ca) {
     const double* src = (h->par.sharpness < 1.0) ? h->d_cnew : h->d_tmp2;
-    bx::k_env_scatter_add<<<gi, kEnvTPB, 0, s>>>(h->d_cenv, src, h->d_env_ptr, h->d_env_mem,
-                                                h->d_mem_flux_sa, h->M, ec);
+    bx::k_env_scatter_add<<<gi, kEnvTPB, 0, s>>>(h->d_cenv, src, h->d_env_ptr, h->d_mem_flux_sa, ec);
     h->launches += 1;
   } else if (h->par.sharpness < 1.0) {
-    bx::k_env_np_flux<double><<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_Denv, h->d_Ex, h->d_Ey, h->d_fx, h->d_fy, ec);
     bx::k_env_update<false><<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_fx, h->d_fy, h->d_env_ptr,
-                                                  h->d_env_mem, h->d_mem_flux_sa, h->M, ec);
-    bx::k_env_integrate_scatter<true><<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_env_ptr,
-                                                            h->d_env_mem, h->d_mem_flux_sa, h->M, ec);
-    h->launches += 3;
+                                                  h->d_mem_flux_sa, ec);
+    bx::k_env_integrate_scatter<true><<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_env_ptr, h->d_mem_flux_sa, ec);
+    h->launches += 2;
   } else {
-    // the common configuration: flux, then update + charge fused, then the
-    // fields in one tiled launch (4 launches per step with the cell kernel);
-    // the split form runs these stencils in FP32 around FP64 state
-    const unsigned gc = (unsigned)(((size_t)h->G * 8 + 255) / 256);
-    const dim3 gt((unsigned)((h->nx + bx::kEnvTX - 1) / bx::kEnvTX), (unsigned)((h->ny + bx::kEnvTY - 1) / bx::kEnvTY));
+    // the common configuration: update + charge fused, then the fields in one
+    // tiled launch (with the cell kernel's, which computes the flux too, three
+    // dependent launches a step)
+    const unsigned gc = (unsigned)((h->G + bx::kEnvUpCells - 1) / bx::kEnvUpCells);
+    const unsigned ntx = (unsigned)((h->nx + bx::kEnvTX - 1) / bx::kEnvTX),
+                   nty = (unsigned)((h->ny + bx::kEnvTY - 1) / bx::kEnvTY);
     const double* phib = h->phib_nonzero ? h->d_phib : nullptr;
     double* rho = out ? h->d_rho_env : nullptr;
-    if (h->mode == MODE_SPLIT) {
-      bx::k_env_np_flux<float><<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_Denv, h->d_Ex, h->d_Ey, h->d_fx, h->d_fy, ec);
-      bx::k_env_update_charge<float><<<gc, 256, 0, s>>>(h->d_cenv, h->d_fx, h->d_fy, h->d_env_ptr, h->d_env_mem,
-                                                        h->d_mem_flux_sa, h->M, h->d_touched, h->d_vsrc, rho, ec);
-      bx::k_env_fields_tile<float><<<gt, bx::kEnvTX * bx::kEnvTY, 0, s>>>(h->d_vsrc, phib, h->d_venv, ec.screen,
-                                                                         h->d_Ex, h->d_Ey, ec);
-    } else {
-      bx::k_env_np_flux<double><<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_Denv, h->d_Ex, h->d_Ey, h->d_fx, h->d_fy, ec);
-      bx::k_env_update_charge<double><<<gc, 256, 0, s>>>(h->d_cenv, h->d_fx, h->d_fy, h->d_env_ptr, h->d_env_mem,
-                                                         h->d_mem_flux_sa, h->M, h->d_touched, h->d_vsrc, rho, ec);
-      bx::k_env_fields_tile<double><<<gt, bx::kEnvTX * bx::kEnvTY, 0, s>>>(h->d_vsrc, phib, h->d_venv, ec.screen,
-                                                                          h->d_Ex, h->d_Ey, ec);
-    }
-    h->launches += 3;
-    return cudaGetLastError();
+    auto update = split ? bx::k_env_update_charge<float> : bx::k_env_update_charge<double>;
+    auto fields = split ? bx::k_env_fields_tile<float> : bx::k_env_fields_tile<double>;
+    cudaError_t e = launch_pdl(update, gc, bx::kEnvUpT, s, h->d_cenv, (const double*)h->d_fx, (const double*)h->d_fy,
+                               (const int*)h->d_env_ptr, (const double*)h->d_mem_flux_sa,
+                               (const uint8_t*)h->d_touched, h->d_vsrc, rho, ec);
+    if (e != cudaSuccess) return e;
+    e = launch_pdl(fields, ntx * nty, bx::kEnvTX * bx::kEnvTY, s, (const double*)h->d_vsrc, phib, h->d_venv, ec.screen,
+                   h->d_Ex, h->d_Ey, ec, (int)ntx);
+    h->launches += 2;
+    return e;
   }
   bx::k_env_charge<<<gg, kEnvTPB, 0, s>>>(h->d_cenv, h->d_touched, h->d_vsrc, out ? h->d_rho_env : nullptr, ec);
   h->launches += 1;
@@ -891,7 +911,7 @@ cudaError_t enqueue_step(bx_cluster* h, int parity, bool out, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     h->launches += 1;
     if (h->ecm) {
-      e = enqueue_env(h, out, s);
+      e = enqueue_env(h, out, env_flux_in_cell_launch(h, out), s);
     } else {
       e = launch_split_env(h, s);
       h->launches += 1;
@@ -922,7 +942,8 @@ cudaError_t enqueue_step(bx_cluster* h, int parity, bool out, cudaStream_t s) {
   }
   if (h->vm_uniform && plain_factored(h, out)) {
     h->launches++;
-    return launch_plain(h, parity, 1, false, s);
+    e = launch_plain(h, parity, 1, false, s);
+    return e != cudaSuccess || !h->ecm ? e : enqueue_env(h, out, true, s);
   }
   e = launch_cell(h, parity, out, s);
   if (e != cudaSuccess) return e;
@@ -933,14 +954,13 @@ cudaError_t enqueue_step(bx_cluster* h, int parity, bool out, cudaStream_t s) {
     h->launches++;
     return cudaGetLastError();
   }
-  return enqueue_env(h, out, s);
+  return enqueue_env(h, out, false, s);
 }
 
 int launches_per_step(const bx_cluster* h) {
-  if (plain_factored(h, false)) return 1;
-  if (!h->ecm) return 2;
+  if (!h->ecm) return plain_factored(h, false) ? 1 : 2;
   if (h->ca) return h->par.sharpness < 1.0 ? 9 : 8;
-  return h->par.sharpness < 1.0 ? 8 : 4;
+  return (h->par.sharpness < 1.0 ? 8 : 4) - (env_flux_in_cell_launch(h, false) ? 1 : 0);
 }
 
 int upload_fact_cst(bx_cluster* h);
@@ -1195,26 +1215,31 @@ int build_split_layout(bx_cluster* h, const std::vector<int>& blk) {
   return upload_param_arrays(h);
 }
 
-// sum of Dm_i * mem_sa of every cell, on the handle's stream
+// sum of Dm_i * mem_sa of every cell (ECM: Dm_i * mem_sa of every membrane),
+// on the handle's stream
 cudaError_t plain_dsa(bx_cluster* h) {
+  if (h->ecm)
+    bx::k_plain_dsam<<<(h->M + 255) / 256, 256, 0, h->stream>>>(h->M, h->I, h->d_Dm, h->d_mem_sa, h->pl_dsa);
+  else
   bx::k_plain_dsa<<<dim3((unsigned)((h->C + 255) / 256), (unsigned)h->I), 256, 0, h->stream>>>(
       h->C, h->M, h->I, h->d_cell_ptr, h->d_Dm, h->d_mem_sa, h->pl_dsa);
   return cudaGetLastError();
 }
 
 // Tiles, junction entries and buffers of the factored plain step.  Cells per
-// tile (a power of two):
+// tile:
 //   pinned    by the launch configuration (a quarter of its membrane slots);
-//   resident  the smallest of 2 to 64 whose tiles fit one a SM (one cluster):
-//             small clusters spread over every SM and keep their state there;
+//   resident  the smallest power of two from 2 to 64 whose tiles fit one a SM
+//             (one cluster): small clusters spread over every SM and keep their
+//             state there;
 //   else      64, halved while fewer than two tiles an SM would be left.
+// Halved further while a tile's shared memory would exceed kPlainSmemMax (cells with very
+// many membranes).
 // Measured us per step, cells per tile 8 / 16 / 32 / 64 (r: resident):
 // 2,878 cells 15.1 / 16.6 / 10.9r / 13.7r, 6,069 cells 25.6 / 17.2 / 20.9 /
 // 13.6r, 9,918 cells 37.5 / 28.3 / 21.2 / 30.7 (so at 64 the resident rule
 // stops where the tiles exceed the SMs), 20,432 cells 67.6 / 42.6 / 37.3 /
 // 33.0, 100,043 cells 293 / 176 / 121 / 108.
-// Halved further while a tile's shared memory would exceed kPlainSmemMax (cells with
-// very many membranes).
 constexpr size_t kPlainSmemMax = 100 * 1024;
 int build_plain_layout(bx_cluster* h) {
   const int C = h->C, M = h->M, I = h->I, ncl = h->ncl;
@@ -1227,7 +1252,7 @@ int build_plain_layout(bx_cluster* h) {
     return n;
   };
   int nc = 64;
-  bool want_res = ncl == 1;
+  bool want_res = ncl == 1 && !h->ecm;
   if (h->pl_pin) {
     nc = h->pl_pin;
   } else if (want_res && tiles_of(64) <= h->sm_count) {
@@ -1291,23 +1316,23 @@ int build_plain_layout(bx_cluster* h) {
       cl_tile[cl + 1] = (int)tile.size();
       cl_group[cl + 1] = cl_group[cl] + (cl_tile[cl + 1] - cl_tile[cl] + 31) / 32;
     }
-    const size_t smem = sizeof(double) * (size_t)bx::PlainSmem(nc, ne_max, nm_max, I, h->vgj).total;
+    const size_t smem = sizeof(double) * (size_t)bx::PlainSmem(nc, ne_max, nm_max, I, h->vgj, h->ecm).total;
     if (smem <= kPlainSmemMax || nc == 1) break;
   }
   const int nt = (int)tile.size(), ng = cl_group[ncl];
   const bool six = is_betse_six_ions(h);
-  const size_t smem = sizeof(double) * (size_t)bx::PlainSmem(nc, ne_max, nm_max, I, h->vgj).total;
+  const size_t smem = sizeof(double) * (size_t)bx::PlainSmem(nc, ne_max, nm_max, I, h->vgj, h->ecm).total;
   int per_sm = 0, coop = 0;
   BX_CU(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->dev));
   if (smem > kPlainSmemMax) return fail(BX_EINVAL, "a cell's junctions do not fit the shared memory of one SM");
   // one limit for every handle, so that handles of different sizes never undercut each other
-  BX_CU(bx::plain_smem_attr(six, h->vgj, kPlainSmemMax));
+  BX_CU(bx::plain_smem_attr(six, h->vgj, h->ecm, kPlainSmemMax));
   h->pl_res = false;
-  if (want_res && coop && nt <= 256) {                // 256: the environment tree of the resident form
+  if (want_res && coop && nt <= 32 * bx::kPlainRows) {   // the environment tree of the resident form
     BX_CU(bx::plain_resident_per_sm(six, h->vgj, smem, &per_sm));
     h->pl_res = nt <= per_sm * h->sm_count;
   }
-  h->pl_nc = nc; h->pl_ntile = nt; h->pl_ngroup = ng; h->pl_ne = ne_max; h->pl_nm = nm_max;
+  h->pl_nc = nc; h->pl_ntile = nt; h->pl_ne = ne_max; h->pl_nm = nm_max;
   h->pl_nent = (int64_t)ent.size();
   // one allocation and one copy: the tables (and the zeroed counters), then
   // what the device fills
@@ -1321,7 +1346,7 @@ int build_plain_layout(bx_cluster* h) {
                o_ctl = take(2 * sizeof(unsigned)), host_bytes = off, o_part = take((size_t)2 * nt * I * sizeof(double)),
                o_gp = take((size_t)(2 * ng + 8 * ncl) * I * sizeof(double)), o_mw = take((size_t)M * sizeof(double)),
                o_sa = take((size_t)C * sizeof(double)), o_iv = take((size_t)C * sizeof(double)),
-               o_dsa = take((size_t)I * C * sizeof(double));
+               o_dsa = take((size_t)I * (h->ecm ? M : C) * sizeof(double));
   std::vector<unsigned char> blob(host_bytes, 0);
   auto put = [&](size_t at, const void* src, size_t bytes) { if (bytes) std::memcpy(blob.data() + at, src, bytes); };
   put(o_tile, tile.data(), nt * sizeof(int2));
@@ -1411,7 +1436,7 @@ int build_partition(bx_cluster* h, int tpb) {
   h->graph_valid = false;
   ++h->layout_gen;
   if (h->mode == MODE_SPLIT) return build_split_layout(h, blk);
-  return h->ecm || h->polar ? BX_OK : build_plain_layout(h);
+  return h->polar || (h->ecm && h->ca) ? BX_OK : build_plain_layout(h);
 }
 
 int create_impl(const bx_geom* gs, const bx_params* ps, int ncl, int precision, bx_handle* out) {
@@ -1509,14 +1534,14 @@ int create_impl(const bx_geom* gs, const bx_params* ps, int ncl, int precision, 
   h->h_gjw = gjw;
   h->h_bflag = bflag; h->h_nn = nn;
 
-  // environment CSR (grid cell -> its membranes, ascending) for the ECM scatter
-  std::vector<int> env_ptr(G + 1, 0), env_mem(M);
+  // environment rows (grid cell -> its membranes, ascending) for the ECM scatter
+  std::vector<int> env_ptr(G + 1, 0), env_slot(h->ecm ? M : 0);
   std::vector<uint8_t> touched(G, 0);
   if (h->ecm) {
     for (int m = 0; m < M; ++m) env_ptr[map_env[m] + 1]++;
     for (int k = 0; k < G; ++k) env_ptr[k + 1] += env_ptr[k];
     std::vector<int> fill(env_ptr.begin(), env_ptr.end() - 1);
-    for (int m = 0; m < M; ++m) env_mem[fill[map_env[m]]++] = m;
+    for (int m = 0; m < M; ++m) env_slot[m] = fill[map_env[m]]++;
     for (int k = 0; k < G; ++k) touched[k] = env_ptr[k + 1] > env_ptr[k];
     double s = 0.0;
     for (int m = 0; m < M; ++m) s += gs[0].mem_sa_per_env[map_env[m]];
@@ -1573,9 +1598,9 @@ int create_impl(const bx_geom* gs, const bx_params* ps, int ncl, int precision, 
   }
   if (h->ecm) {
     ALLOC(h->d_env_ptr, G + 1); H2D(h->d_env_ptr, env_ptr.data(), G + 1);
-    ALLOC(h->d_env_mem, M); H2D(h->d_env_mem, env_mem.data(), M);
+    ALLOC(h->d_env_slot, M); H2D(h->d_env_slot, env_slot.data(), M);
     ALLOC(h->d_touched, G); H2D(h->d_touched, touched.data(), G);
-    ALLOC(h->d_mem_flux_sa, (size_t)I * M);
+    ALLOC(h->d_mem_flux_sa, (size_t)bx::kMfs * M);
     ALLOC(h->d_Denv, (size_t)I * G);
     ALLOC(h->d_Ex, G); ALLOC(h->d_Ey, G);
     ALLOC(h->d_fx, (size_t)I * G); ALLOC(h->d_fy, (size_t)I * G);
@@ -2139,7 +2164,10 @@ int64_t bx_cell_kernel_bytes(bx_handle h) {
     // factored plain step: per cell cc in+out, membrane-side concentrations in+out, dsa (8I each),
     // area, 1/vol, diviterm, row pointer, Vmem in; per membrane the entry, the weight and Vmem out
     // (gating: area, open fraction in+out, gate entry); per entry 16; per tile the environment part
-    return C * (40 * I + 36) + M * (20 + (h->vgj ? 28 : 0)) + h->pl_nent * 16 + (int64_t)h->pl_ntile * (8 * I + 24);
+    // (ECM: instead of dsa per membrane Dm * area, the environment, the exported f*sa, two indices and the area)
+    const int64_t ecm = h->ecm ? M * (24 * I + 16) - C * 8 * I : 0;
+    return C * (40 * I + 36) + M * (20 + (h->vgj ? 28 : 0)) + h->pl_nent * 16 + (int64_t)h->pl_ntile * (8 * I + 24) +
+           ecm;
   }
   const int64_t w = 8;  // Dm, mem_sa, gj_w width
   // membrane: Dm, vm in+out, m2c, nn, nn_cell, bflag, mem_sa, gj_w (+ map_env and the f*sa

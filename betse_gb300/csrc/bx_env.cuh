@@ -5,65 +5,14 @@
 // thread per grid cell; the work is a few hundred bytes per cell, HBM- or
 // launch-bound, and runs inside the step's CUDA graph.
 #pragma once
+#include "bx_env_np.cuh"
 #include "bx_kernels.cuh"
 
 namespace bx {
 
-struct EnvConst {
-  int I, ny, nx, G;
-  double delta, inv_delta, inv_2delta, dt, sharpness;
-  double np_alpha[kMaxIons];   // z q / (kb T)  (times D_env per cell)
-  double zF[kMaxIons];
-  double c_bound[kMaxIons];
-  double surf_scale;           // cell_height delta^2 / mean(memSa_per_envSquare[map])
-  double inv_koeoer;           // 1 / (ko_env eo er)
-  double screen;               // (2/(ko_env delta)) (cell_radius/true_cell_size)
-  double inv_h_d2;             // 1 / (cell_height delta^2)
-  double gw[9];                // Gaussian taps, sigma 1, radius 4
-};
-
-__device__ __forceinline__ bool on_edge(int i, int j, int ny, int nx) {
-  return i == 0 || j == 0 || i == ny - 1 || j == nx - 1;
-}
-
-// Boundary-set concentration (update_ecm sets the four edges, sim.py:2214-2217)
-__device__ __forceinline__ double cb_at(const double* c, const EnvConst& e, int ion, int i, int j) {
-  return on_edge(i, j, e.ny, e.nx) ? e.c_bound[ion] : c[(size_t)ion * e.G + i * e.nx + j];
-}
-
-// Nernst-Planck flux on the grid (update_ecm, sim.py:2219-2242;
-// stb.nernst_planck_flux, sim_toolbox.py:385-413) with fd.gradient
-// (finitediff.py:1236-1266).  E_env is the previous update_V's field.
-// The grid kernels multiply by 1/delta and 1/(2 delta) where the reference
-// divides (a difference of at most one rounding): an FP64 division costs
-// GB300 several FP64-pipe operations, and the stencils are otherwise cheap.
-// R = float is the split form's stencil: the concentration differences are
-// taken in FP64 (the state) and scaled, with the drift term, in FP32.
-// One thread per (ion, grid cell): t = ion*G + k.
 template <typename R>
-__global__ void k_env_np_flux(const double* __restrict__ cenv, const double* __restrict__ Denv,
-                              const double* __restrict__ Ex, const double* __restrict__ Ey,
-                              double* fx, double* fy, EnvConst e) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= e.I * e.G) return;
-  const int ion = t / e.G, k = t - ion * e.G;
-  const int i = k / e.nx, j = k - i * e.nx;
-  {
-    const double c0 = cb_at(cenv, e, ion, i, j);
-    const R inv_d = (R)e.inv_delta, inv_2d = (R)e.inv_2delta;
-    R gcx, gcy;
-    if (j == 0) gcx = (R)(cb_at(cenv, e, ion, i, 1) - c0) * inv_d;
-    else if (j == e.nx - 1) gcx = (R)(c0 - cb_at(cenv, e, ion, i, j - 1)) * inv_d;
-    else gcx = -(R)(cb_at(cenv, e, ion, i, j - 1) - cb_at(cenv, e, ion, i, j + 1)) * inv_2d;
-    if (i == 0) gcy = (R)(cb_at(cenv, e, ion, 1, j) - c0) * inv_d;
-    else if (i == e.ny - 1) gcy = (R)(c0 - cb_at(cenv, e, ion, i - 1, j)) * inv_d;
-    else gcy = -(R)(cb_at(cenv, e, ion, i - 1, j) - cb_at(cenv, e, ion, i + 1, j)) * inv_2d;
-    const R D = (R)Denv[(size_t)ion * e.G + k];
-    const R alpha = D * (R)e.np_alpha[ion];
-    const R gvx = -(R)Ex[k], gvy = -(R)Ey[k];
-    fx[(size_t)ion * e.G + k] = (double)(-D * gcx - alpha * gvx * (R)c0);
-    fy[(size_t)ion * e.G + k] = (double)(-D * gcy - alpha * gvy * (R)c0);
-  }
+__global__ void k_env_np_flux(EnvNp a) {
+  env_np_flux<R>(a, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // fd.diff with the reference's flipped one-sided edge signs (finitediff.py:1268-1303)
@@ -105,8 +54,7 @@ __device__ __forceinline__ void env_charge_out(int k, double rho, const uint8_t*
 template <bool FUSE_SCATTER>
 __global__ void k_env_update(double* cenv, double* tmp, const double* __restrict__ fx,
                              const double* __restrict__ fy, const int* __restrict__ env_ptr,
-                             const int* __restrict__ env_mem, const double* __restrict__ mem_flux_sa,
-                             int M, EnvConst e) {
+                             const double* __restrict__ mem_flux_sa, EnvConst e) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= e.I * e.G) return;
   const int ion = t / e.G, k = t - ion * e.G;
@@ -118,7 +66,7 @@ __global__ void k_env_update(double* cenv, double* tmp, const double* __restrict
     double c = cb_at(cenv, e, ion, i, j) + div * e.dt;
     if (FUSE_SCATTER) {
       double s = 0.0;
-      for (int q = env_ptr[k]; q < env_ptr[k + 1]; ++q) s += -mem_flux_sa[(size_t)ion * M + env_mem[q]];
+      for (int q = env_ptr[k]; q < env_ptr[k + 1]; ++q) s += -mem_flux_sa[(size_t)q * kMfs + ion];
       c = c + (s * e.inv_h_d2) * e.dt;
       cenv[(size_t)ion * e.G + k] = c;
     } else {
@@ -143,8 +91,8 @@ __global__ void k_env_charge(const double* __restrict__ cenv, const uint8_t* __r
 // then a separate buffer).  One thread per (ion, grid cell).
 template <bool SCATTER = true>
 __global__ void k_env_integrate_scatter(double* cenv, const double* __restrict__ tmp,
-                                        const int* __restrict__ env_ptr, const int* __restrict__ env_mem,
-                                        const double* __restrict__ mem_flux_sa, int M, EnvConst e) {
+                                        const int* __restrict__ env_ptr,
+                                        const double* __restrict__ mem_flux_sa, EnvConst e) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= e.I * e.G) return;
   const int ion = t / e.G, k = t - ion * e.G;
@@ -167,7 +115,7 @@ __global__ void k_env_integrate_scatter(double* cenv, const double* __restrict__
       return;
     }
     double s = 0.0;
-    for (int q = env_ptr[k]; q < env_ptr[k + 1]; ++q) s += -mem_flux_sa[(size_t)ion * M + env_mem[q]];
+    for (int q = env_ptr[k]; q < env_ptr[k + 1]; ++q) s += -mem_flux_sa[(size_t)q * kMfs + ion];
     cenv[(size_t)ion * e.G + k] = F + (s * e.inv_h_d2) * e.dt;
   }
 }
@@ -176,13 +124,13 @@ __global__ void k_env_integrate_scatter(double* cenv, const double* __restrict__
 // Nernst-Planck update (and smoothing): update_Co's ECM term
 // (sim_toolbox.py:1185-1200), the same arithmetic as the fused kernels.
 __global__ void k_env_scatter_add(double* cenv, const double* __restrict__ src,
-                                  const int* __restrict__ env_ptr, const int* __restrict__ env_mem,
-                                  const double* __restrict__ mem_flux_sa, int M, EnvConst e) {
+                                  const int* __restrict__ env_ptr,
+                                  const double* __restrict__ mem_flux_sa, EnvConst e) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= e.I * e.G) return;
   const int ion = t / e.G, k = t - ion * e.G;
   double s = 0.0;
-  for (int q = env_ptr[k]; q < env_ptr[k + 1]; ++q) s += -mem_flux_sa[(size_t)ion * M + env_mem[q]];
+  for (int q = env_ptr[k]; q < env_ptr[k + 1]; ++q) s += -mem_flux_sa[(size_t)q * kMfs + ion];
   cenv[t] = src[t] + (s * e.inv_h_d2) * e.dt;
 }
 
@@ -243,58 +191,58 @@ __global__ void k_env_neg_grad(const double* __restrict__ F, double scale, doubl
 // the GPU, the same arithmetic term by term.
 // ---------------------------------------------------------------------------
 
-// k_env_update<true> and k_env_charge in one launch.  Eight lanes per grid
-// cell (lane = ion, I <= 8): each lane advances its ion's concentration in
-// place (it reads only fluxes and its own cell's value), then the cell's
-// group sums F z_i c_i over the ions in order through shuffles.
+// The concentration update, the membrane exchange and the environment charge
+// in one launch: kEnvUpCells grid cells per CTA, a lane per (cell, ion) with the
+// ions of a cell contiguous.  Each lane advances its ion's concentration in
+// place (it reads only fluxes and its own cell's value); then a lane per cell
+// adds F z_i c_i over the ions in order.
 // R = float (split form): the divergence of the FP32 fluxes in FP32; the
 // concentration, the membrane exchange and the charge stay FP64.
+// Bound by the FP64 pipe in both forms, so what counts is full lanes: with
+// eight lanes a cell and the charge summed by shuffles in all of them, 20 FP64
+// warp instructions per four cells took 24 us (split) and 22 us (FP64) on
+// 200 x 200 cells; as written 15.0 and 12.8 us (a launch by itself).
+constexpr int kEnvUpT = 192, kEnvUpCells = 32;
 template <typename R>
-__global__ void __launch_bounds__(256) k_env_update_charge(double* cenv, const double* __restrict__ fx,
-                                                           const double* __restrict__ fy,
-                                                           const int* __restrict__ env_ptr,
-                                                           const int* __restrict__ env_mem,
-                                                           const double* __restrict__ mem_flux_sa, int M,
-                                                           const uint8_t* __restrict__ touched, double* vsrc,
-                                                           double* rho_env, EnvConst e) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = t >> 3, ion = t & 7;
-  const bool live = k < e.G && ion < e.I;
-  double zc = 0.0;
-  if (live) {
+__global__ void __launch_bounds__(kEnvUpT) k_env_update_charge(double* cenv, const double* __restrict__ fx,
+                                                               const double* __restrict__ fy,
+                                                               const int* __restrict__ env_ptr,
+                                                               const double* __restrict__ mem_flux_sa,
+                                                               const uint8_t* __restrict__ touched, double* vsrc,
+                                                               double* rho_env, EnvConst e) {
+  __shared__ double zc[kEnvUpCells * kMaxIons];
+  grid_wait();
+  const int k0 = blockIdx.x * kEnvUpCells, nk = min(kEnvUpCells, e.G - k0);
+  for (int q = threadIdx.x; q < nk * e.I; q += kEnvUpT) {
+    const int lk = q / e.I, ion = q - lk * e.I, k = k0 + lk;
     const int i = k / e.nx, j = k - i * e.nx;
     const double* fxi = fx + (size_t)ion * e.G;
     const double* fyi = fy + (size_t)ion * e.G;
     const R div = ddx_neg<R>(fxi, e, i, j) + ddy_neg<R>(fyi, e, i, j);
     double c = cb_at(cenv, e, ion, i, j) + (double)(div * (R)e.dt);
-    // the membrane exchange: indices, then values, four at a time (the
-    // loads of a batch are independent), added in list order
+    // the membrane exchange, four rows at a time (their loads are
+    // independent), added in list order; a cell's lanes read a row together
     double s = 0.0;
     const int q1 = env_ptr[k + 1];
-    const double* mf = mem_flux_sa + (size_t)ion * M;
     for (int q0 = env_ptr[k]; q0 < q1; q0 += 4) {
-      int mm[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) mm[u] = q0 + u < q1 ? env_mem[q0 + u] : -1;
       double fv[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) fv[u] = mm[u] >= 0 ? mf[mm[u]] : 0.0;
+      for (int u = 0; u < 4; ++u) fv[u] = q0 + u < q1 ? mem_flux_sa[(size_t)(q0 + u) * kMfs + ion] : 0.0;
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (mm[u] >= 0) s += -fv[u];
+        if (q0 + u < q1) s += -fv[u];
     }
     c = c + (s * e.inv_h_d2) * e.dt;
     cenv[(size_t)ion * e.G + k] = c;
-    zc = e.zF[ion] * c;
+    zc[q] = e.zF[ion] * c;
   }
-  // the group of cell k: lanes 8 (k mod 4) .. +7 of this warp
-  const int base = threadIdx.x & 24;
-  double rho = 0.0;
-  for (int q = 0; q < e.I; ++q) {
-    const double v = __shfl_sync(0xffffffffu, zc, base + q);
-    rho += v;
+  __syncthreads();
+  if (threadIdx.x < nk) {
+    double rho = 0.0;
+    for (int q = 0; q < e.I; ++q) rho += zc[threadIdx.x * e.I + q];
+    env_charge_out(k0 + threadIdx.x, rho, touched, vsrc, rho_env, e);
   }
-  if (live && ion == 0) env_charge_out(k, rho, touched, vsrc, rho_env, e);
+  grid_release();
 }
 
 // k_env_gauss_y, k_env_gauss_x (+ Phi_b) and k_env_neg_grad in one launch:
@@ -309,11 +257,13 @@ template <typename R>
 __global__ void __launch_bounds__(kEnvTX * kEnvTY) k_env_fields_tile(const double* __restrict__ vsrc,
                                                                      const double* __restrict__ phib,
                                                                      double* venv, double scale, double* Ex,
-                                                                     double* Ey, EnvConst e) {
+                                                                     double* Ey, EnvConst e, int ntx) {
   __shared__ R src[kEnvSY][kEnvSX];
   __shared__ R gy[kEnvVY][kEnvSX];
   __shared__ R v[kEnvVY][kEnvVX];
-  const int i0 = blockIdx.y * kEnvTY - 1 - 4, j0 = blockIdx.x * kEnvTX - 1 - 4;   // src tile origin
+  grid_wait();
+  const int by = blockIdx.x / ntx, bx_ = blockIdx.x - by * ntx;
+  const int i0 = by * kEnvTY - 1 - 4, j0 = bx_ * kEnvTX - 1 - 4;   // src tile origin
   const int nt = blockDim.x;
   for (int q = threadIdx.x; q < kEnvSY * kEnvSX; q += nt) {
     const int a = q / kEnvSX, b = q - a * kEnvSX, i = i0 + a, j = j0 + b;
@@ -348,8 +298,8 @@ __global__ void __launch_bounds__(kEnvTX * kEnvTY) k_env_fields_tile(const doubl
   __syncthreads();
   // E = -gradient(scale * v_env), one-sided on the grid edges
   const int a = threadIdx.x / kEnvTX + 1, b = threadIdx.x % kEnvTX + 1;
-  const int i = blockIdx.y * kEnvTY + a - 1, j = blockIdx.x * kEnvTX + b - 1;
-  if (i >= e.ny || j >= e.nx) return;
+  const int i = by * kEnvTY + a - 1, j = bx_ * kEnvTX + b - 1;
+  if (i >= e.ny || j >= e.nx) return;   // (an exited thread has released)
   const int k = i * e.nx + j;
   venv[k] = (double)v[a][b];
   const R sc = (R)scale, inv_d = (R)e.inv_delta, inv_2d = (R)e.inv_2delta;
@@ -363,6 +313,7 @@ __global__ void __launch_bounds__(kEnvTX * kEnvTY) k_env_fields_tile(const doubl
   else gyy = -(f(-1, 0) - f(1, 0)) * inv_2d;
   Ex[k] = (double)(-gx);
   Ey[k] = (double)(-gyy);
+  grid_release();
 }
 
 // ---------------------------------------------------------------------------

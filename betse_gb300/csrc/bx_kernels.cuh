@@ -46,6 +46,7 @@ struct DevGeom {
   const int* blk_cell;    // [nblk+1]
   const int* blk_cluster; // [nblk] cluster of each CTA (batched sweeps)
   const double* R_rads;   // [M] membrane distance from the cell centre (cell polarizability)
+  const int* env_slot;    // [M] row of each membrane in mem_flux_sa (ECM)
 };
 
 // Per-step constants (kernel parameter, passed by value).
@@ -92,7 +93,7 @@ struct StepPtrs {
   const double* pump_coef;                 // [ncl] -3 block alpha_NaK (0 = pump off)
   const double* phib;                      // [G] or nullptr
   double* env_part;                        // [nblk][I] partial sums (no ECM)
-  double* mem_flux_sa;                     // [I][M] f_mem*sa (ECM scatter input)
+  double* mem_flux_sa;                     // [M][8] f_mem*sa by env_slot (ECM scatter input)
   unsigned long long* status;              // [4]: nan_vm, nan_conc, neg clamps, spare
   double* gjo;                             // [M] gap-junction open fraction (vgj), in place
   const double* ca_env;                    // [G] Ca2+ of the environment after this step's
@@ -313,7 +314,7 @@ k_cell_step(DevGeom g, StepPtrs p, StepConst k) {
       const double a = (double)(f * msa_t);
       sA[i * TPB + t] = a;
       sB[i * TPB + t] = (double)(-fg * msa_t);
-      if (ECM) p.mem_flux_sa[(size_t)i * g.M + m] = a;
+      if (ECM) p.mem_flux_sa[(size_t)g.env_slot[m] * 8 + i] = a;
       else env_acc[i] = a;
       if (OUT) { fmem_o[i] = f; fgj_o[i] = fg; }
       if (k.polar) { jm += k.zF[i] * (double)f; jg += k.zF[i] * (double)fg; }

@@ -16,11 +16,11 @@
 // about 400 FP64 thread instructions a cell against 1900.  Everything stays
 // FP64; only the order of the sums differs (one rounding per term).
 // Measured per step (k_cell_step with k_env_mix before): 100k cells 403 ->
-// 108 us, 20k cells 85 -> 33 us, 2900 cells 41 -> 10.9 us, 185 cells
+// 100 us, 20k cells 85 -> 33 us, 2900 cells 41 -> 11.1 us, 185 cells
 // 40 -> 10.3 us (12.5 with the one-lane-per-ion kernel that this one replaced).
 //
-// One CTA advances one tile: NC consecutive cells of one cluster (NC a power
-// of two), in phases separated by bar.sync:
+// One CTA advances one tile: NC consecutive cells of one cluster, in phases
+// separated by bar.sync:
 //   A  lane per junction ("entry"): the shared exponentials and Q of every ion;
 //      lane per cell: the shared exponentials and the pumps
 //   G  (voltage-gated junctions) lane per membrane: the open fraction, once
@@ -34,12 +34,19 @@
 //
 // The environment sum runs over a binary tree of the cluster's cell indices
 // (aligned powers of two, missing leaves zero), so its rounding depends
-// neither on the tile size nor on what else is in a batch.
+// neither on the tile size nor on what else is in a batch (NC is a power of two).
 //
 // Two launches of the same body (build_plain_layout chooses):
 //   streaming   one step per launch (programmatic dependent launch); the last
 //               tile of every 32 adds their parts, the last such group of the
 //               cluster the groups' (ticket counters), and mixes the environment
+//   (extracellular spaces: streaming, one launch a step before the grid's own,
+//   without the environment sum.  The environment differs from membrane to
+//   membrane, so a phase M, lane per membrane, gathers it and evaluates the
+//   pump, and phase C forms each membrane's flux from two factors per cell and
+//   ion, f sa = Dm sa (P - Q c_env): five FP64 instructions a membrane and ion.
+//   The last blocks of the launch compute the grid's Nernst-Planck flux.
+//   20,400 cells on 200 x 200: step 126 -> 58.8 us; 4975 on 100 x 100: 44 -> 28)
 //   resident    many steps per cooperative launch, one tile per CTA, all of
 //               them co-resident: the state stays in shared memory, tiles
 //               exchange Vmem and concentrations through L2 and meet once a
@@ -47,6 +54,7 @@
 //               and the junctions inside the tile are evaluated while the
 //               barrier completes.
 #pragma once
+#include "bx_env_np.cuh"
 #include "bx_kernels.cuh"
 #include "bx_sync.cuh"
 
@@ -54,6 +62,7 @@ namespace bx {
 
 constexpr int kPlainT = 256;            // threads per CTA
 constexpr int kPlainNone = INT32_MIN;   // mem_ent: no junction
+constexpr int kPlainRows = 8;           // resident: most rows of 32 tiles (the environment tree adds eight)
 
 struct PlainGeom {
   int C, M, ntile;
@@ -70,10 +79,13 @@ struct PlainGeom {
   const int* m2c;          // [M]
   const double* mem_w;     // [M] gj_weight * mem_sa
   const double* mem_sa;    // [M]
-  const double* dsa;       // [I][C] sum of Dm_i * mem_sa over the cell's membranes
+  const double* dsa;       // [I][C] sum of Dm_i * mem_sa over the cell's membranes (ECM: [M][I] Dm_i * mem_sa)
   const double* sa;        // [C] sum of mem_sa
   const double* ivol;      // [C] 1 / cell_vol
   const double* diviterm;  // [C]
+  const int* map_env;      // [M] (ECM)
+  const int* env_slot;     // [M] (ECM) row of the exported f*sa
+  int G;
 };
 
 struct PlainRun {
@@ -91,9 +103,10 @@ struct PlainRun {
 };
 
 // Shared memory of one CTA, in doubles, for the largest tile.
+constexpr int kPlainCell = 9;           // doubles of a cell's shared factors
 struct PlainSmem {
-  int q, v, cm, cc, x, s1, k, env, lvl, ga, gg, total;
-  __host__ __device__ PlainSmem(int nc, int ne, int nm, int I, bool gated) {
+  int q, v, cm, cc, x, s1, k, env, lvl, ga, gg, en, pm, total;
+  __host__ __device__ PlainSmem(int nc, int ne, int nm, int I, bool gated, bool ecm) {
     int o = 0;
     auto take = [&](int n) { const int at = o; o += n; return at; };
     q = take(ne * I);
@@ -102,15 +115,17 @@ struct PlainSmem {
     cc = take(nc * I);
     x = take(nc * I);
     s1 = take(nc * I);
-    k = take(nc * 7);
+    k = take(nc * kPlainCell);
     env = take(kMaxIons);
-    lvl = take(8 * (kPlainT / 32));
+    lvl = take(8 * kPlainRows);
     ga = take(gated ? 2 * ne : 0);
     gg = take(gated ? nm * I : 0);
+    en = take(ecm ? nm * I : 0);
+    pm = take(ecm ? nm : 0);
     total = o;
   }
 };
-enum PlainCell { PK_K1 = 0, PK_E1, PK_K2, PK_E2, PK_FNA, PK_DTV, PK_FCA };
+enum PlainCell { PK_K1 = 0, PK_E1, PK_K2, PK_E2, PK_FNA, PK_DTV, PK_FCA, PK_PC, PK_PR };   // kPlainCell rows
 
 // BETSE's six-ion set as constants (ZP = 1) or the parameters' ions (ZP = 0)
 template <int ZP> struct PlainIons {
@@ -137,6 +152,23 @@ __device__ __forceinline__ double plain_ghk(int zc, double zval, double v_nonce,
       const double a = ((zval + kNonce) * v_nonce) * F_RT;
       const double ea = exp(-a), den = -expm1(-a);
       return -(a * inv_d) * ((cB - cA * ea) / den);
+    }
+  }
+}
+
+// The same flux as P - Q cA (factors per cell and ion).
+__device__ __forceinline__ void plain_pq(int zc, double zval, double v_nonce, double F_RT, double inv_d, double kr,
+                                         double kr2, double e1, double e2, double cB, double& P, double& Q) {
+  switch (zc) {
+    case 1: P = kr * cB; Q = kr * e1; break;
+    case -1: P = (kr * e1) * cB; Q = kr; break;
+    case 2: P = kr2 * cB; Q = kr2 * e2; break;
+    case -2: P = (kr2 * e2) * cB; Q = kr2; break;
+    default: {
+      const double a = ((zval + kNonce) * v_nonce) * F_RT;
+      const double r = -(a * inv_d) / -expm1(-a);
+      P = r * cB;
+      Q = r * exp(-a);
     }
   }
 }
@@ -193,25 +225,31 @@ __device__ __forceinline__ void tree_rows(const double* src, int n, int I, doubl
   }
 }
 
-template <int ZP, bool GATED, bool RES>
-__global__ void __launch_bounds__(kPlainT, RES ? 1 : 3)
-k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r) {
+// CTAs per SM: four (64 registers) at 100k cells 100.1 us a step against 108.1
+// with three (70 registers); extracellular spaces (78 registers) 59.6 us with
+// three, 60.6 with four, at 20,400 cells.
+template <int ZP, bool GATED, bool RES, bool ECM>
+__global__ void __launch_bounds__(kPlainT, RES ? 1 : (ECM ? 3 : 4))
+k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r, EnvNp en) {
+  static_assert(!(RES && ECM), "the grid's own launches separate the steps");
   using IS = PlainIons<ZP>;
   constexpr int T = kPlainT, NI = IS::NI;
   extern __shared__ double sm[];
   __shared__ int s_flag;
   const int I = IS::n(k);
-  const PlainSmem L(r.nc_max, r.ne_max, r.nm_max, I, GATED);
+  const PlainSmem L(r.nc_max, r.ne_max, r.nm_max, I, GATED, ECM);
   double *sQ = sm + L.q, *sv = sm + L.v, *scm = sm + L.cm, *scc = sm + L.cc, *sx = sm + L.x, *s1 = sm + L.s1,
-         *sk = sm + L.k, *senv = sm + L.env, *slvl = sm + L.lvl, *sga = sm + L.ga, *sgg = sm + L.gg;
+         *sk = sm + L.k, *senv = sm + L.env, *slvl = sm + L.lvl, *sga = sm + L.ga, *sgg = sm + L.gg, *sen = sm + L.en, *spm = sm + L.pm;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, b = blockIdx.x;
 
-#if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 900)
-  if (!RES) {
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+  // A streaming launch releases the next one as its CTAs exit: released at its
+  // start, the next step's CTAs take whatever room the SMs have and the load
+  // ends up uneven (20,400 cells 33.2 -> 41.5 us).
+  if (!RES) grid_wait();
+  if (ECM && b >= g.ntile) {
+    env_np_flux<double>(en, (b - g.ntile) * T + t);
+    return;   // (an exited CTA has released the next kernel)
   }
-#endif
   const int2 tl = g.tile[b];
   const int c0 = tl.x, nc = tl.y;
   const int cl = g.tile_cl[b];
@@ -228,8 +266,8 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r) {
     scc[q] = p.cc[(size_t)i * g.C + c0 + lc];
   }
   for (int q = t; q < nc; q += T) sv[q] = vin[g.cell_ptr[c0 + q]];
-  if (t < I) senv[t] = r.cenv[(size_t)cl * I + t];
-  if (t < 8 * (T / 32)) slvl[t] = 0.0;
+  if (!ECM && t < I) senv[t] = r.cenv[(size_t)cl * I + t];
+  for (int q = t; q < 8 * kPlainRows; q += T) slvl[q] = 0.0;
   __syncthreads();
 
   // junction entry e: Q of every ion from the own side into the partner
@@ -267,7 +305,7 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r) {
     GhkShared<double> s;
     s.init(sv[lc] + kNonce, k.F_RT);
     const double kr = s.a1 * k.inv_tm * s.r;
-    double* o = sk + lc * 7;
+    double* o = sk + lc * kPlainCell;
     o[PK_K1] = kr;
     o[PK_E1] = s.e1;
     o[PK_K2] = 2.0 * kr * s.q2;
@@ -276,9 +314,20 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r) {
   };
   // cell lc: its pumps, times the cell's membrane area
   auto cell_pump = [&](int lc) {
-    double* o = sk + lc * 7;
-    const double sa = g.sa[c0 + lc], e1 = o[PK_E1];
+    double* o = sk + lc * kPlainCell;
+    const double e1 = o[PK_E1];
     const double* cm = scm + lc * I;
+    if (ECM) {
+      // pump_fna with the cell's share in PC and PR: PC (k2 - PR nao^3) / (1 +
+      // k2), k2 = (ko / KmK)^2 (the quotient's ko^2 cancels against k2)
+      const double nai = cm[k.iNa] * 1e-3, ki = cm[k.iK] * 1e-3;
+      const double xna = cm[k.iNa] * k.inv_KmNa, c = k.inv_KmK * 1e3;
+      const double na3 = xna * xna * xna;
+      o[PK_PC] = pcoef * (na3 * k.atp_term) / ((1.0 + na3) * k.atp_den);
+      o[PK_PR] = (k.qnum_c * (ki * ki) * e1 * (c * c)) / (k.qden_c * (nai * nai * nai) * k.K0);
+      return;
+    }
+    const double sa = g.sa[c0 + lc];
     double fna = 0.0;
     if (pcoef != 0.0)                             // Na/K-ATPase (sim.py:1196-1234)
       fna = pump_fna<double>(k, pcoef, e1, cm[k.iNa], senv[k.iNa], cm[k.iK], senv[k.iK]);
@@ -312,13 +361,37 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r) {
     __syncthreads();
     if (RES && step > 0) {
       if (t < I) {
-        // at most eight rows of 32 tiles (the launch rule)
+        // kPlainRows rows of 32 tiles (the launch rule)
         const double a = (slvl[t] + slvl[8 + t]) + (slvl[16 + t] + slvl[24 + t]);
         const double c = (slvl[32 + t] + slvl[40 + t]) + (slvl[48 + t] + slvl[56 + t]);
         senv[t] = senv[t] - (a + c) * r.env_scale[cl];
       }
       __syncthreads();
       for (int q = t; q < nc; q += T) cell_pump(q);
+      __syncthreads();
+    }
+    // ---- M: each membrane's environment and pump
+    if (ECM) {
+      for (int m = m0 + t; m < m1; m += T) {
+        const int ge = g.map_env[m], lc = g.m2c[m] - c0;
+        double ce[NI];
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+          if (i < I) ce[i] = r.cenv[(size_t)i * g.G + ge];
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+          if (i < I) sen[(m - m0) * I + i] = ce[i];
+        double f = 0.0;
+        if (pcoef != 0.0) {
+          const double cna = r.cenv[(size_t)k.iNa * g.G + ge], cko = r.cenv[(size_t)k.iK * g.G + ge];
+          const double* o = sk + lc * kPlainCell;
+          const double nao = cna * 1e-3, xk = cko * k.inv_KmK, k2 = xk * xk;
+          f = o[PK_PC] * (k2 - o[PK_PR] * (nao * nao * nao)) / (1.0 + k2);
+          if ((__double2hiint(f) & 0x7ff00000) == 0x7ff00000 || cko == 0.0)   // a vanishing quotient: the
+            f = pump_fna<double>(k, pcoef, o[PK_E1], scm[lc * I + k.iNa], cna, scm[lc * I + k.iK], cko);   // reference's value
+        }
+        spm[m - m0] = f * g.mem_sa[m];
+      }
       __syncthreads();
     }
     // ---- G: the gated open fractions, one lane per membrane
@@ -340,19 +413,32 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r) {
     for (int q = t; q < nc * I; q += T) {
       const int lc = q / I, i = q - lc * I, c = c0 + lc;
       const int a0 = g.cell_ptr[c], a1 = g.cell_ptr[c + 1];
-      double s2 = 0.0;
+      const double* o = sk + lc * kPlainCell;
+      double s2 = 0.0, S = 0.0, P = 0.0, Q = 0.0, fp = 0.0;
+      if (ECM) {
+        plain_pq(IS::zc(k, i), k.z[i], sv[lc] + kNonce, k.F_RT, k.inv_tm, o[PK_K1], o[PK_K2], o[PK_E1], o[PK_E2],
+                 scm[q], P, Q);
+        fp = i == k.iNa ? 1.0 : i == k.iK ? -(2.0 / 3.0) : 0.0;
+      }
       for (int m = a0; m < a1; ++m) {
+        if (ECM) {
+          const int ml = m - m0;
+          const double a = g.dsa[(size_t)m * I + i] * (P - Q * sen[ml * I + i]) + fp * spm[ml];
+          p.mem_flux_sa[(size_t)g.env_slot[m] * kMfs + i] = a;
+          S += a;
+        }
         const int me = g.mem_ent[m];
         if (me == kPlainNone) continue;
         const double w = GATED ? sgg[(m - m0) * I + i] : g.mem_w[m];
         s2 += signed_like(w, ~me) * sQ[(me >= 0 ? me : ~me) * I + i];   // -w on the own side
       }
-      const double* o = sk + lc * 7;
-      double S = g.dsa[(size_t)i * g.C + c] * plain_ghk(IS::zc(k, i), k.z[i], sv[lc] + kNonce, k.F_RT, k.inv_tm,
-                                                       o[PK_K1], o[PK_K2], o[PK_E1], o[PK_E2], senv[i], scm[q]);
-      if (i == k.iNa) S = o[PK_FNA] + S;
-      else if (i == k.iK) S = -(2.0 / 3.0) * o[PK_FNA] + S;
-      if (i == k.iCa) S = S + o[PK_FCA];
+      if (!ECM) {
+        S = g.dsa[(size_t)i * g.C + c] * plain_ghk(IS::zc(k, i), k.z[i], sv[lc] + kNonce, k.F_RT, k.inv_tm, o[PK_K1],
+                                                 o[PK_K2], o[PK_E1], o[PK_E2], senv[i], scm[q]);
+        if (i == k.iNa) S = o[PK_FNA] + S;
+        else if (i == k.iK) S = -(2.0 / 3.0) * o[PK_FNA] + S;
+        if (i == k.iCa) S = S + o[PK_FCA];
+      }
       s1[q] = S;
       double x = scc[q] + S * o[PK_DTV];              // update_Co, sim_toolbox.py:1182-1183
       sx[q] = x;
@@ -379,17 +465,19 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r) {
       if (v != v) nanv += g.cell_ptr[c0 + lc + 1] - a0;
       if (RES) vout[a0] = v;                 // what the other tiles read
     }
-    double* part = r.part + (RES ? (size_t)((step + 1) & 1) * g.ntile * I : (size_t)0);
-    for (int i = warp; i < I; i += T / 32) {
-      // lane l: cells [l, l + 1) ... or a run of 2 or 4, pairs first
-      double a;
-      auto at = [&](int lc) { return lc < nc ? s1[lc * I + i] : 0.0; };
-      if (r.nc_max <= 32) a = at(lane);
-      else if (r.nc_max <= 64) a = at(2 * lane) + at(2 * lane + 1);
-      else a = (at(4 * lane) + at(4 * lane + 1)) + (at(4 * lane + 2) + at(4 * lane + 3));
+    if (!ECM) {
+      // lane l: cells [l, l + 1), or a run of 2 or 4, pairs first
+      double* part = r.part + (RES ? (size_t)((step + 1) & 1) * g.ntile * I : (size_t)0);
+      for (int i = warp; i < I; i += T / 32) {
+        double a;
+        auto at = [&](int lc) { return lc < nc ? s1[lc * I + i] : 0.0; };
+        if (r.nc_max <= 32) a = at(lane);
+        else if (r.nc_max <= 64) a = at(2 * lane) + at(2 * lane + 1);
+        else a = (at(4 * lane) + at(4 * lane + 1)) + (at(4 * lane + 2) + at(4 * lane + 3));
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (lane == 0) part[(size_t)b * I + i] = a;
+        for (int o = 1; o < 32; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane == 0) part[(size_t)b * I + i] = a;
+      }
     }
     if (RES) {
       for (int q = t; q < nc * I; q += T) scm[q] = sx[q];
@@ -427,6 +515,10 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r) {
   // ---- streaming: Vmem of every membrane, then the environment by tickets
   __syncthreads();
   for (int m = m0 + t; m < m1; m += T) vout[m] = sv[g.m2c[m] - c0];
+  if (ECM) {
+    grid_release();
+    return;
+  }
   const int ct0 = g.cl_tile[cl], nt = g.cl_tile[cl + 1] - ct0;
   const int grp = (b - ct0) >> 5, ngrp = (nt + 31) >> 5;
   const int g0 = g.cl_group[cl];
@@ -503,14 +595,22 @@ static __global__ void k_plain_static(int C, const int* __restrict__ cell_ptr, c
   ivol[c] = 1.0 / cell_vol[c];
 }
 
-// launchers (bx_step_f64_small.cu)
-cudaError_t launch_plain_step(bool six, bool gated, cudaStream_t s, const PlainGeom& g, const StepPtrs& p,
-                              const StepConst& k, const PlainRun& r);
+// Dm_i * mem_sa of every membrane, ion contiguous (ECM)
+static __global__ void k_plain_dsam(int M, int I, const double* __restrict__ Dm, const double* __restrict__ mem_sa,
+                                    double* dsam) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= M) return;
+  for (int i = 0; i < I; ++i) dsam[(size_t)m * I + i] = Dm[(size_t)i * M + m] * mem_sa[m];
+}
+
+// launchers (bx_step_f64_small.cu); ecm: with the grid's flux in en.nblk more blocks
+cudaError_t launch_plain_step(bool six, bool gated, bool ecm, cudaStream_t s, const PlainGeom& g, const StepPtrs& p,
+                              const StepConst& k, const PlainRun& r, const EnvNp& en);
 cudaError_t launch_plain_resident(bool six, bool gated, cudaStream_t s, const PlainGeom& g, const StepPtrs& p,
                                   const StepConst& k, const PlainRun& r);
 // CTAs of the resident form that fit one SM with this much shared memory (0: none)
 cudaError_t plain_resident_per_sm(bool six, bool gated, size_t smem, int* per_sm);
 // the shared-memory limit of both forms, raised once per device
-cudaError_t plain_smem_attr(bool six, bool gated, size_t smem);
+cudaError_t plain_smem_attr(bool six, bool gated, bool ecm, size_t smem);
 
 }  // namespace bx

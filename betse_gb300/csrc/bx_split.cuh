@@ -21,6 +21,7 @@
 //   per CTA        cluster id; per cluster the well-mixed environment and the
 //                  pump constant (batched parameter sweeps share one launch)
 #pragma once
+#include "bx_env_np.cuh"
 #include "bx_kernels.cuh"
 
 namespace bx {
@@ -153,7 +154,8 @@ struct SplitPtrs {
   const float* __restrict__ phib;          // [G] (PHIB)
   float* __restrict__ env_part;            // [nblk][I] per-tile partial sums
   const double* __restrict__ cenv_grid;    // [I][G] environment grid concentrations (ECM)
-  double* __restrict__ mfs;                // [I][M] f_mem*sa per membrane, natural order (ECM scatter)
+  double* __restrict__ mfs;                // [M][kMfs] f_mem*sa by env_slot (ECM scatter)
+  const int* __restrict__ env_slot;        // [M] (ECM)
   float* __restrict__ gjo;                 // [Q] gap-junction open fraction per slot (vgj), in place
   double* __restrict__ o_gjopen;           // [M] output steps with vgj: the open fraction
   const double* __restrict__ ca_env;       // [G] Ca2+ of the grid after this step's Nernst-Planck
@@ -230,7 +232,7 @@ template <> struct IonSet<1> {
 // grid scatter (update_Co's ECM term) instead of the well-mixed partials.
 template <int TPB, int REC, int ZP, bool OUT, bool PHIB, bool ECM = false>
 __global__ void __launch_bounds__(TPB, 2048 / TPB / 2)
-k_split_step(SplitGeom g, SplitPtrs p, SplitConst k) {
+k_split_step(SplitGeom g, SplitPtrs p, SplitConst k, EnvNp en) {
   using IS = IonSet<ZP>;
   constexpr int NI = IS::NI;
   __shared__ float sA[NI][TPB];
@@ -245,13 +247,20 @@ k_split_step(SplitGeom g, SplitPtrs p, SplitConst k) {
   const int q = b * TPB + t;                 // membrane slot
   const int s0 = b * kCellsPerCta;           // first cell slot of the tile
 
+  if (!ECM) grid_release();
+  if (ECM && b >= (int)gridDim.x - en.nblk) {
+    // the last blocks: the grid's Nernst-Planck flux, which needs only the
+    // previous step (beside the tiles it costs no launch and no wait)
 #if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 900)
-  cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
 #endif
+    env_np_flux<float>(en, (b - ((int)gridDim.x - en.nblk)) * TPB + t);
+    return;
+  }
   // ---- prologue: geometry and channel data (read-only during stepping)
   const int lc = g.lcell[q];
   const bool active = lc != 255;                // padding slots load nothing more
-  int cn = s0;
+  int cn = s0, erow = 0;
   float sa = 0.f, gw = 0.f;
   float dmv[NI];
 #pragma unroll
@@ -260,6 +269,7 @@ k_split_step(SplitGeom g, SplitPtrs p, SplitConst k) {
     cn = g.nn_slot[q];
     sa = g.mem_sa[q];
     gw = g.gjw[q] * k.gj_block;
+    if (ECM) erow = p.env_slot[g.tile_m0[b] + t];
 #pragma unroll
     for (int i = 0; i < NI; ++i)
       if (i < I) dmv[i] = p.Dm[(size_t)i * g.Q + q];
@@ -364,7 +374,7 @@ k_split_step(SplitGeom g, SplitPtrs p, SplitConst k) {
       const float fg = ghk_flux_fk(sg, ka_g, z, k.z[i], vgj1, k.F_RT, cin, nbr[i], dgjv, k.inv_gjl);
       sA[i][t] = f * sa;
       sB[i][t] = -fg * sa;
-      if (ECM) p.mfs[(size_t)i * g.M + g.tile_m0[b] + t] = (double)(f * sa);
+      if (ECM) p.mfs[(size_t)erow * kMfs + i] = (double)(f * sa);
       if (OUT) {
         const int mn = g.tile_m0[b] + t;
         p.o_fmem[(size_t)i * g.M + mn] = (double)f;
