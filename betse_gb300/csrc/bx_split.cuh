@@ -247,7 +247,6 @@ k_split_step(SplitGeom g, SplitPtrs p, SplitConst k, EnvNp en) {
   const int q = b * TPB + t;                 // membrane slot
   const int s0 = b * kCellsPerCta;           // first cell slot of the tile
 
-  if (!ECM) grid_release();
   if (ECM && b >= (int)gridDim.x - en.nblk) {
     // the last blocks: the grid's Nernst-Planck flux, which needs only the
     // previous step (beside the tiles it costs no launch and no wait)
