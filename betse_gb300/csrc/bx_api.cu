@@ -2805,9 +2805,12 @@ int bx_time_env_fields(bx_handle h, int n, double* ms_fields, double* ms_product
 // ---------------------------------------------------------------------------
 // Molecule and gene regulatory networks (bx_network.cuh)
 // ---------------------------------------------------------------------------
+constexpr int kNetSmemMax = 100 * 1024;   // dynamic shared memory of k_net_cell, k_net_gj
+
 struct bx_network {
   bx_cluster* h = nullptr;
-  int S = 0, R = 0, nblk = 0;
+  int S = 0, R = 0;
+  int ntile = 0, tile_cells = 0, tile_mems = 0;   // k_net_cell, k_net_gj: a CTA per tile
   bool any_ui = false, have_state = false, have_fluxes = false;
   bx::NetTables* d_tab = nullptr;
   double *d_gamma = nullptr, *d_Rr = nullptr /* gamma / R_rads */, *d_gmod = nullptr, *d_cc = nullptr, *d_cm = nullptr,
@@ -2860,25 +2863,26 @@ bx::NetArgs net_args(bx_network* n, int vm_parity) {
   a.dt = h->par.dt; a.inv_tm = 1.0 / h->par.tm; a.F_RT = h->par.F / (h->par.R * h->par.T);
   a.inv_gj_len = 1.0 / h->gj_len; a.gj_block = h->par.gj_block;
   a.inv_vol_env_M = 1.0 / (h->par.vol_env * (double)h->M);
-  a.cell_ptr = h->d_cell_ptr; a.nn = h->d_nn; a.nn_cell = h->d_nn_cell; a.bflag = h->d_bflag;
+  a.cell_ptr = h->d_cell_ptr; a.m2c = h->d_m2c; a.nn = h->d_nn; a.nn_cell = h->d_nn_cell; a.bflag = h->d_bflag;
   a.mem_sa = h->d_mem_sa; a.cell_vol = h->d_cell_vol; a.gj_w = h->d_gj_w;
   a.gjo = h->vgj ? h->d_gjo : nullptr;
   a.vm = h->d_vm[vm_parity];
   a.tab = n->d_tab; a.gamma = n->d_gamma; a.g_over_r = n->d_Rr; a.gmod = n->d_gmod; a.gmask = n->d_gmask;
   a.c_cells = n->d_cc; a.cmem = n->d_cm; a.c_mid = n->d_cmid; a.cmem_mid = n->d_cmmid; a.env = n->d_env;
   a.env_part = n->d_part; a.f_mem = n->d_fmem; a.f_gj = n->d_fgj; a.rates = n->d_rates; a.neg = n->d_neg;
-  a.nblk = n->nblk;
+  a.ntile = n->ntile; a.tile_cells = n->tile_cells; a.tile_mems = n->tile_mems;
   return a;
 }
 
 cudaError_t net_enqueue(bx_network* n, int vm_parity, bool out, cudaStream_t s) {
   const bx::NetArgs a = net_args(n, vm_parity);
+  const size_t sc = 8 * bx::net_smem_cell(n->S, n->R, n->tile_mems), sg = 8 * bx::net_smem_gj(n->S, n->tile_mems);
   if (out) {
-    bx::k_net_cell<true><<<n->nblk, bx::kNetTPB, 0, s>>>(a);
-    bx::k_net_gj<true><<<n->nblk, bx::kNetTPB, 0, s>>>(a);
+    bx::k_net_cell<true><<<n->ntile, bx::kNetTPB, sc, s>>>(a);
+    bx::k_net_gj<true><<<n->ntile, bx::kNetTPB, sg, s>>>(a);
   } else {
-    bx::k_net_cell<false><<<n->nblk, bx::kNetTPB, 0, s>>>(a);
-    bx::k_net_gj<false><<<n->nblk, bx::kNetTPB, 0, s>>>(a);
+    bx::k_net_cell<false><<<n->ntile, bx::kNetTPB, sc, s>>>(a);
+    bx::k_net_gj<false><<<n->ntile, bx::kNetTPB, sg, s>>>(a);
   }
   n->h->launches += 2;
   return cudaGetLastError();
@@ -3001,14 +3005,27 @@ int bx_network_create(bx_handle h, const bx_net_spec* sp, bx_network_handle* out
     ~Guard() { if (*p) net_free(p->get()); }
   } guard{&n};
   n->h = h; n->S = S; n->R = R; n->any_ui = any_ui;
-  n->nblk = (C + bx::kNetTPB - 1) / bx::kNetTPB;
+  // tiles of 32 cells; fewer where cells with very many membranes and many
+  // substances would not leave room for two CTAs an SM
+  for (n->tile_cells = bx::kNetCells;; n->tile_cells /= 2) {
+    n->ntile = (C + n->tile_cells - 1) / n->tile_cells;
+    n->tile_mems = 0;
+    for (int b = 0; b < n->ntile; ++b) {
+      const int c0 = b * n->tile_cells, c1 = std::min(C, c0 + n->tile_cells);
+      n->tile_mems = std::max(n->tile_mems, h->h_cell_ptr[c1] - h->h_cell_ptr[c0]);
+    }
+    if (n->tile_cells == 1 || 8 * bx::net_smem_cell(S, R, n->tile_mems) <= kNetSmemMax) break;
+  }
   if (dalloc(&n->d_tab, 1) != cudaSuccess || dalloc(&n->d_cc, (size_t)S * C) != cudaSuccess ||
       dalloc(&n->d_cm, (size_t)S * M) != cudaSuccess || dalloc(&n->d_cmid, (size_t)S * C) != cudaSuccess ||
       dalloc(&n->d_cmmid, (size_t)S * M) != cudaSuccess || dalloc(&n->d_env, (size_t)S) != cudaSuccess ||
-      dalloc(&n->d_part, (size_t)n->nblk * S) != cudaSuccess || dalloc(&n->d_fmem, (size_t)S * M) != cudaSuccess ||
+      dalloc(&n->d_part, (size_t)n->ntile * S) != cudaSuccess || dalloc(&n->d_fmem, (size_t)S * M) != cudaSuccess ||
       dalloc(&n->d_fgj, (size_t)S * M) != cudaSuccess || dalloc(&n->d_neg, 1) != cudaSuccess ||
       dalloc(&n->d_rates, (size_t)std::max(R, 1) * C) != cudaSuccess)
     return fail(BX_ENOMEM, "network allocation");
+  for (const void* k : {(const void*)bx::k_net_cell<false>, (const void*)bx::k_net_cell<true>,
+                        (const void*)bx::k_net_gj<false>, (const void*)bx::k_net_gj<true>})
+    BX_CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kNetSmemMax));
   BX_CU(cudaMemcpy(n->d_tab, tb.get(), sizeof(bx::NetTables), cudaMemcpyHostToDevice));
   BX_CU(cudaMemset(n->d_neg, 0, sizeof(unsigned long long)));
   BX_CU(cudaMemset(n->d_fmem, 0, (size_t)S * M * sizeof(double)));

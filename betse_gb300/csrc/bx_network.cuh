@@ -2,7 +2,7 @@
 //
 // MasterOfNetworks.run_loop (chemistry/networks.py:2805-2983) for the
 // substances of one network on a plain FP64 cluster without extracellular
-// spaces, as two kernels per time step, one thread per cell:
+// spaces, as two kernels per time step, one CTA per tile of up to 32 cells:
 //
 //   k_net_cell  per cell: Molecule.update_intra of every substance
 //               (networks.py:5714-5807); growth/decay and cell-zone reaction
@@ -19,6 +19,15 @@
 //               checks (sim_toolbox.py:1125-1151).  CTA 0 also reduces the
 //               environment partials in a fixed order.
 //
+// Each kernel runs in phases over its tile, so that every phase has a lane for
+// each independent value: a lane per (cell, substance or reaction) for the
+// rates (a warp works on one table entry), a lane per membrane for the fluxes
+// (coalesced loads), a lane per (cell, substance) for the sums over a cell's
+// membranes, in membrane order.  A flux that is the same at all membranes of a
+// cell is formed once.  Bound by the FP64 pipe and, before, by latency: with a
+// thread per cell (4 warps an SM at 20k cells, strided membrane loads, the
+// concentrations in local memory) 20,432 cells took 58 + 41 us, as written 36 + 26.
+//
 // The split into two launches is the one place the step needs every cell:
 // the gap-junction flux reads the partner cell after its membrane step.
 //
@@ -26,7 +35,7 @@
 // their "mid" copies, the last step's fluxes f_mem/f_gj [S][M] and reaction
 // rates [R][C], growth
 // modulation [S][C] and target masks [S][C] only for the substances that have
-// them, env [S], env partials [nblk][S]; the tables (substances, terms,
+// them, env [S], env partials [ntile][S]; the tables (substances, terms,
 // reactions, stoichiometry) are one small block in global memory that every
 // warp reads uniformly.  Geometry and Vmem are the cluster handle's own arrays.
 #pragma once
@@ -42,7 +51,8 @@ constexpr int kNetMaxSub = 16;
 constexpr int kNetMaxReact = 32;
 constexpr int kNetMaxTerms = 256;
 constexpr int kNetStoich = 4;
-constexpr int kNetTPB = 128;
+constexpr int kNetTPB = 256;
+constexpr int kNetCells = 32;           // most cells of a tile: a warp's lanes
 
 enum NetTermKind { NT_ACT = 0, NT_ACT_INDEP = 1, NT_INH = 2, NT_DIRECT_POS = 3, NT_DIRECT_NEG = 4 };
 
@@ -77,6 +87,7 @@ struct NetArgs {
   double dt, inv_tm, F_RT, inv_gj_len, gj_block, inv_vol_env_M;
   // cluster geometry and state (the handle's arrays)
   const int* cell_ptr;
+  const int* m2c;
   const int* nn;
   const int* nn_cell;
   const uint8_t* bflag;
@@ -96,12 +107,13 @@ struct NetArgs {
   double* c_mid;             // [S][C]
   double* cmem_mid;          // [S][M]
   double* env;               // [S]
-  double* env_part;          // [nblk][S]
+  double* env_part;          // [ntile][S]
   double* f_mem;             // [S][M] (OUT)
   double* f_gj;              // [S][M] (OUT)
   double* rates;             // [R][C] (OUT) cell-zone reaction rates (MasterOfNetworks.reaction_rates)
   unsigned long long* neg;   // negative concentrations seen
-  int nblk;
+  int ntile, tile_cells;     // tiles of tile_cells cells (at most kNetCells)
+  int tile_mems;             // most membranes of a tile
 };
 
 // sim_toolbox.electroflux (sim_toolbox.py:18-69) for a general charge, FP64,
@@ -142,8 +154,9 @@ __device__ __forceinline__ double net_pow(double x, double n) {
   return pow(x, n);
 }
 
+// cs: the cell's concentrations, kNetCells apart
 __device__ __forceinline__ double net_conc(const NetTermD& t, const double* cs, const double* env) {
-  return t.env ? env[t.sub] : cs[t.sub];
+  return t.env ? env[t.sub] : cs[t.sub * kNetCells];
 }
 
 // One influencer factor (get_influencers, networks.py:5084-5600).  The host
@@ -190,112 +203,133 @@ __device__ double net_factor(const NetTables& tb, int t0, int nt, const double* 
   return any_direct ? a * dsum : a;
 }
 
-// Sums v over the CTA in a fixed order (warp tree, then warps in order) and
-// writes the total from thread 0.
-__device__ __forceinline__ double net_block_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) red[w] = v;
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += red[i];
-  __syncthreads();
-  return s;
+// growth and decay of substance k (write_growth_and_decay)
+__device__ __forceinline__ double net_growth(const NetArgs& a, const NetTables& tb, int k, int c, const double* cs,
+                                             const double* env) {
+  const NetSubD& sb = tb.sub[k];
+  if (!sb.growth || !(sb.mask_row < 0 || a.gmask[(size_t)sb.mask_row * a.C + c])) return 0.0;
+  const double mod = sb.mod_row < 0 ? 1.0 : a.gmod[(size_t)sb.mod_row * a.C + c];
+  const double cc = cs[k * kNetCells] * sb.inv_gsf;
+  const double ga = net_factor(tb, sb.gt0, sb.gnt, cs, env);
+  const double da = net_factor(tb, sb.dt0, sb.dnt, cs, env);
+  return mod * (sb.r_prod * sb.tdf) * ga - (sb.r_decay * sb.tdf) * cc - (sb.decay_max * sb.tdf) * da * cc;
 }
+
+// rate of reaction j (write_reactions)
+__device__ __forceinline__ double net_rate(const NetTables& tb, int j, const double* cs, const double* env) {
+  const NetReactD& rx = tb.react[j];
+  const double al = net_factor(tb, rx.t0, rx.nt, cs, env);
+  if (rx.inv_keq == 0.0) {
+    double fwd = 1.0;
+    for (int q = 0; q < rx.nr; ++q) {
+      const double x = net_pow(cs[rx.r[q] * kNetCells] * rx.inv_rkm[q], rx.rc[q]);
+      fwd = q == 0 ? x / (1.0 + x) : fwd * (x / (1.0 + x));
+    }
+    return rx.vmax * al * fwd;
+  }
+  // BETSE's quotient applies the power before the 1e-3 (networks.py:1364-1396)
+  double num = 1.0, den = 1.0;
+  for (int q = 0; q < rx.np; ++q) {
+    const double t = 1.0e-3 * net_pow(cs[rx.p[q] * kNetCells], rx.pc[q]);
+    num = q == 0 ? t : num * t;
+  }
+  for (int q = 0; q < rx.nr; ++q) {
+    const double t = 1.0e-3 * net_pow(cs[rx.r[q] * kNetCells], rx.rc[q]);
+    den = q == 0 ? t : den * t;
+  }
+  return rx.vmax * al * (1.0 - (num / den) * rx.inv_keq);
+}
+
+// dynamic shared memory of both kernels, in doubles
+__host__ __device__ constexpr int net_smem_cell(int S, int R, int nm) { return (3 * S + R) * kNetCells + S * nm; }
+__host__ __device__ constexpr int net_smem_gj(int S, int nm) { return S * kNetCells + S * nm; }
 
 template <bool OUT>
 __global__ void __launch_bounds__(kNetTPB) k_net_cell(NetArgs a) {
   // the tables are read in place: every lane of a warp reads the same entry,
   // one broadcast load from L1
   const NetTables& tb = *a.tab;
-  __shared__ double red[kNetTPB / 32];
-  const int S = tb.S, R = tb.R;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = c < a.C;
-  double cs[kNetMaxSub], env[kNetMaxSub], fsum[kNetMaxSub];
-  for (int k = 0; k < S; ++k) {
-    cs[k] = live ? a.c_cells[(size_t)k * a.C + c] : 0.0;
-    env[k] = a.env[k];
-    fsum[k] = 0.0;
+  extern __shared__ double ns[];
+  __shared__ double env[kNetMaxSub], siv[kNetCells], sv[kNetCells];
+  const int S = tb.S, R = tb.R, t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  double* cs = ns;                               // [S][32] concentrations
+  double* sr = cs + S * kNetCells;               // [S + R][32] growth, reaction rates
+  double* sf0 = sr + (S + R) * kNetCells;        // [S][32] membrane flux at the cell's Vmem
+  double* sfa = sf0 + S * kNetCells;             // [S][tile_mems] flux times area
+  const int c0 = blockIdx.x * a.tile_cells, nc = min(a.tile_cells, a.C - c0);
+  const int m0 = a.cell_ptr[c0], nm = a.cell_ptr[c0 + nc] - m0;
+  for (int q = t; q < S * kNetCells; q += kNetTPB) {
+    const int k = q / kNetCells, lc = q - k * kNetCells;
+    cs[q] = lc < nc ? a.c_cells[(size_t)k * a.C + c0 + lc] : 0.0;
   }
+  if (t < S) env[t] = a.env[t];
+  if (warp == kNetTPB / 32 - 1 && lane < nc) {
+    siv[lane] = 1.0 / a.cell_vol[c0 + lane];
+    sv[lane] = a.vm[min(a.cell_ptr[c0 + lane], a.M - 1)];
+  }
+  __syncthreads();
+  // rates on the concentrations at the start of the step; the membrane flux of
+  // a substance whose membrane-side value is the cell's
+  for (int j = warp; j < 2 * S + R; j += kNetTPB / 32) {
+    if (lane >= nc) continue;
+    const double* cl = cs + lane;
+    if (j < S) {
+      sr[j * kNetCells + lane] = net_growth(a, tb, j, c0 + lane, cl, env);
+    } else if (j < S + R) {
+      const double rate = net_rate(tb, j - S, cl, env);
+      sr[j * kNetCells + lane] = rate;
+      if (OUT) a.rates[(size_t)(j - S) * a.C + c0 + lane] = rate;
+    } else {
+      const int k = j - S - R;
+      const NetSubD& sb = tb.sub[k];
+      const double zF = (sb.z + kNonce) * a.F_RT;
+      if (sb.Dm != 0.0 && !sb.ui)
+        sf0[k * kNetCells + lane] = net_ghk(env[k], cl[k * kNetCells], sb.Dm * a.inv_tm, zF, net_neutral(zF), sv[lane]);
+    }
+  }
+  __syncthreads();
   int neg = 0;
-  if (live) {
-    const int m0 = a.cell_ptr[c], m1 = a.cell_ptr[c + 1];
-    // rates (write_growth_and_decay / write_reactions) on the concentrations
-    // at the start of the step
-    double delta[kNetMaxSub];
+  for (int ml = t; ml < nm; ml += kNetTPB) {
+    const int m = m0 + ml, lc = a.m2c[m] - c0;
+    const double sa = a.mem_sa[m], v = a.vm[m];
     for (int k = 0; k < S; ++k) {
       const NetSubD& sb = tb.sub[k];
-      double r = 0.0;
-      const bool target = sb.mask_row < 0 || a.gmask[(size_t)sb.mask_row * a.C + c];
-      if (sb.growth && target) {
-        const double mod = sb.mod_row < 0 ? 1.0 : a.gmod[(size_t)sb.mod_row * a.C + c];
-        const double cc = cs[k] * sb.inv_gsf;
-        const double ga = net_factor(tb, sb.gt0, sb.gnt, cs, env);
-        const double da = net_factor(tb, sb.dt0, sb.dnt, cs, env);
-        r = mod * (sb.r_prod * sb.tdf) * ga - (sb.r_decay * sb.tdf) * cc - (sb.decay_max * sb.tdf) * da * cc;
+      if (sb.Dm == 0.0 && !sb.ui) {
+        if (OUT) a.f_mem[(size_t)k * a.M + m] = 0.0;
+        continue;
       }
-      delta[k] = r;
-    }
-    for (int j = 0; j < R; ++j) {
-      const NetReactD& rx = tb.react[j];
-      const double al = net_factor(tb, rx.t0, rx.nt, cs, env);
-      double rate;
-      if (rx.inv_keq == 0.0) {
-        double fwd = 1.0;
-        for (int q = 0; q < rx.nr; ++q) {
-          const double x = net_pow(cs[rx.r[q]] * rx.inv_rkm[q], rx.rc[q]);
-          fwd = q == 0 ? x / (1.0 + x) : fwd * (x / (1.0 + x));
-        }
-        rate = rx.vmax * al * fwd;
-      } else {
-        // BETSE's quotient applies the power before the 1e-3 (networks.py:1364-1396)
-        double num = 1.0, den = 1.0;
-        for (int q = 0; q < rx.np; ++q) {
-          const double t = 1.0e-3 * net_pow(cs[rx.p[q]], rx.pc[q]);
-          num = q == 0 ? t : num * t;
-        }
-        for (int q = 0; q < rx.nr; ++q) {
-          const double t = 1.0e-3 * net_pow(cs[rx.r[q]], rx.rc[q]);
-          den = q == 0 ? t : den * t;
-        }
-        rate = rx.vmax * al * (1.0 - (num / den) * rx.inv_keq);
-      }
-      if (OUT) a.rates[(size_t)j * a.C + c] = rate;
-      for (int k = 0; k < S; ++k) delta[k] += tb.rm[k][j] * rate;
-    }
-    const double inv_vol = 1.0 / a.cell_vol[c];
-    for (int k = 0; k < S; ++k) {
-      const NetSubD& sb = tb.sub[k];
-      const double c1 = cs[k] + delta[k] * a.dt;
       const double zF = (sb.z + kNonce) * a.F_RT, Dk = sb.Dm * a.inv_tm;
-      const bool neutral = net_neutral(zF);
-      double s = 0.0;
-      for (int m = m0; m < m1; ++m) {
-        double cm;
-        if (sb.ui) {
-          // Molecule.update_intra, implicit Euler toward the cell centre
-          // (neutral substance: no field term); kq = gamma Do dt' / R_rads
-          const double kq = a.g_over_r[m] * (sb.Do * (a.dt * sb.tdf));
-          cm = (kq * cs[k] + a.cmem[(size_t)k * a.M + m]) / (1.0 + kq);
-          neg += cm < 0.0;
-        } else {
-          cm = cs[k];
-        }
-        const double f = sb.Dm != 0.0 ? net_ghk(env[k], cm, Dk, zF, neutral, a.vm[m]) : 0.0;
-        const double fa = f * a.mem_sa[m];
-        s += fa;
-        if (sb.ui) a.cmem_mid[(size_t)k * a.M + m] = cm + f * a.gamma[m] * a.dt;
-        if (OUT) a.f_mem[(size_t)k * a.M + m] = f;
+      double cm = cs[k * kNetCells + lc], f = 0.0;
+      if (sb.ui) {
+        // Molecule.update_intra, implicit Euler toward the cell centre
+        // (neutral substance: no field term); kq = gamma Do dt' / R_rads
+        const double kq = a.g_over_r[m] * (sb.Do * (a.dt * sb.tdf));
+        cm = (kq * cm + a.cmem[(size_t)k * a.M + m]) / (1.0 + kq);
+        neg += cm < 0.0;
       }
-      fsum[k] = s;
-      a.c_mid[(size_t)k * a.C + c] = c1 + (s * inv_vol) * a.dt;
+      if (sb.Dm != 0.0)
+        f = !sb.ui && v == sv[lc] ? sf0[k * kNetCells + lc] : net_ghk(env[k], cm, Dk, zF, net_neutral(zF), v);
+      sfa[k * a.tile_mems + ml] = f * sa;
+      if (sb.ui) a.cmem_mid[(size_t)k * a.M + m] = cm + f * a.gamma[m] * a.dt;
+      if (OUT) a.f_mem[(size_t)k * a.M + m] = f;
     }
   }
-  for (int k = 0; k < S; ++k) {
-    const double t = net_block_sum(fsum[k], red);
-    if (threadIdx.x == 0) a.env_part[(size_t)blockIdx.x * S + k] = t;
+  __syncthreads();
+  for (int k = warp; k < S; k += kNetTPB / 32) {
+    const NetSubD& sb = tb.sub[k];
+    double s = 0.0;
+    if (lane < nc) {
+      const int c = c0 + lane;
+      if (sb.Dm != 0.0)
+        for (int ml = a.cell_ptr[c] - m0; ml < a.cell_ptr[c + 1] - m0; ++ml) s += sfa[k * a.tile_mems + ml];
+      double delta = sr[k * kNetCells + lane];
+      for (int j = 0; j < R; ++j) delta += tb.rm[k][j] * sr[(S + j) * kNetCells + lane];
+      const double c1 = cs[k * kNetCells + lane] + delta * a.dt;
+      a.c_mid[(size_t)k * a.C + c] = c1 + (s * siv[lane]) * a.dt;
+    }
+    if (sb.Dm != 0.0)
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) a.env_part[(size_t)blockIdx.x * S + k] = s;
   }
   if (neg) atomicAdd(a.neg, (unsigned long long)neg);
 }
@@ -303,58 +337,68 @@ __global__ void __launch_bounds__(kNetTPB) k_net_cell(NetArgs a) {
 template <bool OUT>
 __global__ void __launch_bounds__(kNetTPB) k_net_gj(NetArgs a) {
   const NetTables& tb = *a.tab;
-  const int S = tb.S;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  extern __shared__ double ns[];
+  const int S = tb.S, t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  double* sc = ns;                               // [S][32] concentrations, mid then final
+  double* sfa = sc + S * kNetCells;              // [S][tile_mems] -flux times area
+  const int c0 = blockIdx.x * a.tile_cells, nc = min(a.tile_cells, a.C - c0);
+  const int m0 = a.cell_ptr[c0], nm = a.cell_ptr[c0 + nc] - m0;
+  for (int q = t; q < S * kNetCells; q += kNetTPB) {
+    const int k = q / kNetCells, lc = q - k * kNetCells;
+    sc[q] = lc < nc ? a.c_mid[(size_t)k * a.C + c0 + lc] : 0.0;
+  }
+  __syncthreads();
   int neg = 0;
-  if (c < a.C) {
-    const int m0 = a.cell_ptr[c], m1 = a.cell_ptr[c + 1];
-    const double inv_vol = 1.0 / a.cell_vol[c];
+  for (int ml = t; ml < nm; ml += kNetTPB) {
+    const int m = m0 + ml, lc = a.m2c[m] - c0, n = a.nn[m], cn = a.nn_cell[m];
+    const bool open = !a.bflag[m];
+    const double sa = a.mem_sa[m], dv = a.vm[n] - a.vm[m];
+    const double go = a.gjo ? a.gjo[m] : a.gj_block * a.gj_w[m];
     for (int k = 0; k < S; ++k) {
       const NetSubD& sb = tb.sub[k];
-      const double c2 = a.c_mid[(size_t)k * a.C + c];
-      double c3 = c2;
-      if (!sb.gj_imp) {
+      const size_t km = (size_t)k * a.M + m;
+      const double cA = sb.ui ? a.cmem_mid[km] : sc[k * kNetCells + lc];
+      double f = 0.0;
+      if (!sb.gj_imp && open) {
+        const double cB = sb.ui ? a.cmem_mid[(size_t)k * a.M + n] : a.c_mid[(size_t)k * a.C + cn];
         const double zF = (sb.z + kNonce) * a.F_RT, Dk = sb.Dgj * a.gj_block * a.inv_gj_len;
-        const bool neutral = net_neutral(zF);
-        double s = 0.0;
-        for (int m = m0; m < m1; ++m) {
-          const int n = a.nn[m];
-          const double cA = sb.ui ? a.cmem_mid[(size_t)k * a.M + m] : c2;
-          const double cB = sb.ui ? a.cmem_mid[(size_t)k * a.M + n] : a.c_mid[(size_t)k * a.C + a.nn_cell[m]];
-          const double go = a.gjo ? a.gjo[m] : a.gj_block * a.gj_w[m];
-          double f = 0.0;
-          if (!a.bflag[m]) f = net_ghk(cA, cB, Dk * go, zF, neutral, a.vm[n] - a.vm[m]);
-          s += -f * a.mem_sa[m];
-          if (sb.ui) {
-            const double cm = cA + (-f) * a.gamma[m] * sb.tdf * a.dt;
-            a.cmem[(size_t)k * a.M + m] = cm;
-            neg += cm < 0.0;
-          }
-          if (OUT) a.f_gj[(size_t)k * a.M + m] = f;
-        }
-        c3 = c2 + a.dt * (s * inv_vol) * sb.tdf;
-      } else {
-        for (int m = m0; m < m1; ++m) {
-          if (sb.ui) {
-            const double cm = a.cmem_mid[(size_t)k * a.M + m];
-            a.cmem[(size_t)k * a.M + m] = cm;
-            neg += cm < 0.0;
-          }
-          if (OUT) a.f_gj[(size_t)k * a.M + m] = 0.0;
-        }
+        f = net_ghk(cA, cB, Dk * go, zF, net_neutral(zF), dv);
       }
-      if (!sb.ui)
-        for (int m = m0; m < m1; ++m) a.cmem[(size_t)k * a.M + m] = c3;
-      a.c_cells[(size_t)k * a.C + c] = c3;
-      neg += c3 < 0.0;
+      sfa[k * a.tile_mems + ml] = -f * sa;
+      if (sb.ui) {
+        const double cm = sb.gj_imp ? cA : cA + (-f) * a.gamma[m] * sb.tdf * a.dt;
+        a.cmem[km] = cm;
+        neg += cm < 0.0;
+      }
+      if (OUT) a.f_gj[km] = f;
     }
+  }
+  __syncthreads();
+  for (int k = warp; k < S; k += kNetTPB / 32) {
+    if (lane >= nc) continue;
+    const NetSubD& sb = tb.sub[k];
+    const int c = c0 + lane;
+    double c3 = sc[k * kNetCells + lane];
+    if (!sb.gj_imp) {
+      double s = 0.0;
+      for (int ml = a.cell_ptr[c] - m0; ml < a.cell_ptr[c + 1] - m0; ++ml) s += sfa[k * a.tile_mems + ml];
+      c3 = c3 + a.dt * (s * (1.0 / a.cell_vol[c])) * sb.tdf;
+      sc[k * kNetCells + lane] = c3;
+    }
+    a.c_cells[(size_t)k * a.C + c] = c3;
+    neg += c3 < 0.0;
+  }
+  __syncthreads();
+  for (int ml = t; ml < nm; ml += kNetTPB) {
+    const int m = m0 + ml, lc = a.m2c[m] - c0;
+    for (int k = 0; k < S; ++k)
+      if (!tb.sub[k].ui) a.cmem[(size_t)k * a.M + m] = sc[k * kNetCells + lc];
   }
   if (blockIdx.x == 0) {
     // the auto-mixed environment: mean over membranes of env - f sa dt / vol_env
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int k = w; k < S; k += (int)(blockDim.x >> 5)) {
+    for (int k = warp; k < S; k += kNetTPB / 32) {
       double s = 0.0;
-      for (int b = lane; b < a.nblk; b += 32) s += a.env_part[(size_t)b * S + k];
+      for (int b = lane; b < a.ntile; b += 32) s += a.env_part[(size_t)b * S + k];
       for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
       if (lane == 0) {
         const double e = a.env[k] - (s * a.dt) * a.inv_vol_env_M;
