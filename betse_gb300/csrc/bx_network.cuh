@@ -26,7 +26,7 @@
 // membranes, in membrane order.  A flux that is the same at all membranes of a
 // cell is formed once.  Bound by the FP64 pipe and, before, by latency: with a
 // thread per cell (4 warps an SM at 20k cells, strided membrane loads, the
-// concentrations in local memory) 20,432 cells took 58 + 41 us, as written 36 + 26.
+// concentrations in local memory) 20,432 cells took 58 + 41 us, as written 31 + 20.
 //
 // The split into two launches is the one place the step needs every cell:
 // the gap-junction flux reads the partner cell after its membrane step.
@@ -128,13 +128,28 @@ struct NetArgs {
 //   to the fifth power, whose remainder a^6/720 is below 2e-21 |a|.
 __device__ __forceinline__ bool net_neutral(double zF) { return fabs(zF) < 1.0e-20; }
 
+// |x| against a power of ten through the exponent and upper mantissa bits (the
+// FP64 compare costs a pipe slot): hi is the bound's upper word, and the
+// formulas on both sides of each bound agree there.
+__device__ __forceinline__ int net_abs_hi(double x) { return __double2hiint(x) & 0x7fffffff; }
+constexpr int kHi1e17 = 0x3c670ef5;      // upper word of 1e-17
+constexpr int kHi1e3 = 0x3f50624d;       // upper word of 1e-3
+// x < 0, the compare itself only where the sign bit is set
+__device__ __forceinline__ int net_is_neg(double x) { return __double2hiint(x) < 0 && x < 0.0 ? 1 : 0; }
+
+// What a substance's fluxes need, formed once per CTA.
+struct NetFlux {
+  double zF, Dk, kq;                     // (z + 1e-25) F / (R T); D / d; membrane step: Do dt', junctions: dt'
+  int on, neutral, ui, pad;              // on: the substance crosses
+};
+
 __device__ __forceinline__ double net_ghk(double cA, double cB, double Dk, double zF, bool neutral, double v) {
   if (neutral) return -Dk * (cB - cA);
   const double a = zF * (v + kNonce);
-  const double aa = fabs(a);
-  if (aa < 1.0e-17) return -Dk * (cB - cA);
+  const int aa = net_abs_hi(a);
+  if (aa < kHi1e17) return -Dk * (cB - cA);
   double ea, den;
-  if (aa > 1.0e-3) {
+  if (aa > kHi1e3) {
     ea = exp(-a);
     den = 1.0 - ea;
   } else {
@@ -251,6 +266,7 @@ __global__ void __launch_bounds__(kNetTPB) k_net_cell(NetArgs a) {
   const NetTables& tb = *a.tab;
   extern __shared__ double ns[];
   __shared__ double env[kNetMaxSub], siv[kNetCells], sv[kNetCells];
+  __shared__ NetFlux fx[kNetMaxSub];
   const int S = tb.S, R = tb.R, t = threadIdx.x, warp = t >> 5, lane = t & 31;
   double* cs = ns;                               // [S][32] concentrations
   double* sr = cs + S * kNetCells;               // [S + R][32] growth, reaction rates
@@ -262,7 +278,12 @@ __global__ void __launch_bounds__(kNetTPB) k_net_cell(NetArgs a) {
     const int k = q / kNetCells, lc = q - k * kNetCells;
     cs[q] = lc < nc ? a.c_cells[(size_t)k * a.C + c0 + lc] : 0.0;
   }
-  if (t < S) env[t] = a.env[t];
+  if (t < S) {
+    const NetSubD& sb = tb.sub[t];
+    env[t] = a.env[t];
+    const double zF = (sb.z + kNonce) * a.F_RT;
+    fx[t] = NetFlux{zF, sb.Dm * a.inv_tm, sb.Do * (a.dt * sb.tdf), sb.Dm != 0.0, net_neutral(zF), sb.ui, 0};
+  }
   if (warp == kNetTPB / 32 - 1 && lane < nc) {
     siv[lane] = 1.0 / a.cell_vol[c0 + lane];
     sv[lane] = a.vm[min(a.cell_ptr[c0 + lane], a.M - 1)];
@@ -281,10 +302,8 @@ __global__ void __launch_bounds__(kNetTPB) k_net_cell(NetArgs a) {
       if (OUT) a.rates[(size_t)(j - S) * a.C + c0 + lane] = rate;
     } else {
       const int k = j - S - R;
-      const NetSubD& sb = tb.sub[k];
-      const double zF = (sb.z + kNonce) * a.F_RT;
-      if (sb.Dm != 0.0 && !sb.ui)
-        sf0[k * kNetCells + lane] = net_ghk(env[k], cl[k * kNetCells], sb.Dm * a.inv_tm, zF, net_neutral(zF), sv[lane]);
+      if (fx[k].on && !fx[k].ui)
+        sf0[k * kNetCells + lane] = net_ghk(env[k], cl[k * kNetCells], fx[k].Dk, fx[k].zF, fx[k].neutral, sv[lane]);
     }
   }
   __syncthreads();
@@ -292,42 +311,45 @@ __global__ void __launch_bounds__(kNetTPB) k_net_cell(NetArgs a) {
   for (int ml = t; ml < nm; ml += kNetTPB) {
     const int m = m0 + ml, lc = a.m2c[m] - c0;
     const double sa = a.mem_sa[m], v = a.vm[m];
+    const bool same = __double_as_longlong(v) == __double_as_longlong(sv[lc]);
     for (int k = 0; k < S; ++k) {
-      const NetSubD& sb = tb.sub[k];
-      if (sb.Dm == 0.0 && !sb.ui) {
-        if (OUT) a.f_mem[(size_t)k * a.M + m] = 0.0;
-        continue;
-      }
-      const double zF = (sb.z + kNonce) * a.F_RT, Dk = sb.Dm * a.inv_tm;
-      double cm = cs[k * kNetCells + lc], f = 0.0;
-      if (sb.ui) {
+      const NetFlux& x = fx[k];
+      const size_t km = (size_t)k * a.M + m;
+      double f = 0.0;
+      if (x.ui) {
         // Molecule.update_intra, implicit Euler toward the cell centre
         // (neutral substance: no field term); kq = gamma Do dt' / R_rads
-        const double kq = a.g_over_r[m] * (sb.Do * (a.dt * sb.tdf));
-        cm = (kq * cm + a.cmem[(size_t)k * a.M + m]) / (1.0 + kq);
-        neg += cm < 0.0;
+        const double kq = a.g_over_r[m] * x.kq;
+        double cm = (kq * cs[k * kNetCells + lc] + a.cmem[km]) / (1.0 + kq);
+        neg += net_is_neg(cm);
+        if (x.on) {
+          f = net_ghk(env[k], cm, x.Dk, x.zF, x.neutral, v);
+          sfa[k * a.tile_mems + ml] = f * sa;
+          cm = cm + f * a.gamma[m] * a.dt;
+        }
+        a.cmem_mid[km] = cm;
+      } else if (x.on) {
+        f = same ? sf0[k * kNetCells + lc]
+                 : net_ghk(env[k], cs[k * kNetCells + lc], x.Dk, x.zF, x.neutral, v);
+        sfa[k * a.tile_mems + ml] = f * sa;
       }
-      if (sb.Dm != 0.0)
-        f = !sb.ui && v == sv[lc] ? sf0[k * kNetCells + lc] : net_ghk(env[k], cm, Dk, zF, net_neutral(zF), v);
-      sfa[k * a.tile_mems + ml] = f * sa;
-      if (sb.ui) a.cmem_mid[(size_t)k * a.M + m] = cm + f * a.gamma[m] * a.dt;
-      if (OUT) a.f_mem[(size_t)k * a.M + m] = f;
+      if (OUT) a.f_mem[km] = f;
     }
   }
   __syncthreads();
   for (int k = warp; k < S; k += kNetTPB / 32) {
-    const NetSubD& sb = tb.sub[k];
+    const bool on = fx[k].on;
     double s = 0.0;
     if (lane < nc) {
       const int c = c0 + lane;
-      if (sb.Dm != 0.0)
+      if (on)
         for (int ml = a.cell_ptr[c] - m0; ml < a.cell_ptr[c + 1] - m0; ++ml) s += sfa[k * a.tile_mems + ml];
       double delta = sr[k * kNetCells + lane];
       for (int j = 0; j < R; ++j) delta += tb.rm[k][j] * sr[(S + j) * kNetCells + lane];
       const double c1 = cs[k * kNetCells + lane] + delta * a.dt;
-      a.c_mid[(size_t)k * a.C + c] = c1 + (s * siv[lane]) * a.dt;
+      a.c_mid[(size_t)k * a.C + c] = on ? c1 + (s * siv[lane]) * a.dt : c1;
     }
-    if (sb.Dm != 0.0)
+    if (on)
       for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (lane == 0) a.env_part[(size_t)blockIdx.x * S + k] = s;
   }
@@ -339,6 +361,8 @@ __global__ void __launch_bounds__(kNetTPB) k_net_gj(NetArgs a) {
   const NetTables& tb = *a.tab;
   extern __shared__ double ns[];
   const int S = tb.S, t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  __shared__ double siv[kNetCells];
+  __shared__ NetFlux fx[kNetMaxSub];
   double* sc = ns;                               // [S][32] concentrations, mid then final
   double* sfa = sc + S * kNetCells;              // [S][tile_mems] -flux times area
   const int c0 = blockIdx.x * a.tile_cells, nc = min(a.tile_cells, a.C - c0);
@@ -347,6 +371,12 @@ __global__ void __launch_bounds__(kNetTPB) k_net_gj(NetArgs a) {
     const int k = q / kNetCells, lc = q - k * kNetCells;
     sc[q] = lc < nc ? a.c_mid[(size_t)k * a.C + c0 + lc] : 0.0;
   }
+  if (t < S) {
+    const NetSubD& sb = tb.sub[t];
+    const double zF = (sb.z + kNonce) * a.F_RT;
+    fx[t] = NetFlux{zF, sb.Dgj * a.gj_block * a.inv_gj_len, a.dt * sb.tdf, !sb.gj_imp, net_neutral(zF), sb.ui, 0};
+  }
+  if (warp == kNetTPB / 32 - 1 && lane < nc) siv[lane] = 1.0 / a.cell_vol[c0 + lane];
   __syncthreads();
   int neg = 0;
   for (int ml = t; ml < nm; ml += kNetTPB) {
@@ -355,20 +385,20 @@ __global__ void __launch_bounds__(kNetTPB) k_net_gj(NetArgs a) {
     const double sa = a.mem_sa[m], dv = a.vm[n] - a.vm[m];
     const double go = a.gjo ? a.gjo[m] : a.gj_block * a.gj_w[m];
     for (int k = 0; k < S; ++k) {
-      const NetSubD& sb = tb.sub[k];
+      const NetFlux& x = fx[k];
       const size_t km = (size_t)k * a.M + m;
-      const double cA = sb.ui ? a.cmem_mid[km] : sc[k * kNetCells + lc];
       double f = 0.0;
-      if (!sb.gj_imp && open) {
-        const double cB = sb.ui ? a.cmem_mid[(size_t)k * a.M + n] : a.c_mid[(size_t)k * a.C + cn];
-        const double zF = (sb.z + kNonce) * a.F_RT, Dk = sb.Dgj * a.gj_block * a.inv_gj_len;
-        f = net_ghk(cA, cB, Dk * go, zF, net_neutral(zF), dv);
+      if (x.on && open) {
+        const double cA = x.ui ? a.cmem_mid[km] : sc[k * kNetCells + lc];
+        const double cB = x.ui ? a.cmem_mid[(size_t)k * a.M + n] : a.c_mid[(size_t)k * a.C + cn];
+        f = net_ghk(cA, cB, x.Dk * go, x.zF, x.neutral, dv);
       }
-      sfa[k * a.tile_mems + ml] = -f * sa;
-      if (sb.ui) {
-        const double cm = sb.gj_imp ? cA : cA + (-f) * a.gamma[m] * sb.tdf * a.dt;
+      if (x.on) sfa[k * a.tile_mems + ml] = -f * sa;
+      if (x.ui) {
+        double cm = a.cmem_mid[km];
+        if (x.on) cm = cm + (-f) * a.gamma[m] * x.kq;
         a.cmem[km] = cm;
-        neg += cm < 0.0;
+        neg += net_is_neg(cm);
       }
       if (OUT) a.f_gj[km] = f;
     }
@@ -376,23 +406,22 @@ __global__ void __launch_bounds__(kNetTPB) k_net_gj(NetArgs a) {
   __syncthreads();
   for (int k = warp; k < S; k += kNetTPB / 32) {
     if (lane >= nc) continue;
-    const NetSubD& sb = tb.sub[k];
     const int c = c0 + lane;
     double c3 = sc[k * kNetCells + lane];
-    if (!sb.gj_imp) {
+    if (fx[k].on) {
       double s = 0.0;
       for (int ml = a.cell_ptr[c] - m0; ml < a.cell_ptr[c + 1] - m0; ++ml) s += sfa[k * a.tile_mems + ml];
-      c3 = c3 + a.dt * (s * (1.0 / a.cell_vol[c])) * sb.tdf;
+      c3 = c3 + (s * siv[lane]) * fx[k].kq;
       sc[k * kNetCells + lane] = c3;
     }
     a.c_cells[(size_t)k * a.C + c] = c3;
-    neg += c3 < 0.0;
+    neg += net_is_neg(c3);
   }
   __syncthreads();
   for (int ml = t; ml < nm; ml += kNetTPB) {
     const int m = m0 + ml, lc = a.m2c[m] - c0;
     for (int k = 0; k < S; ++k)
-      if (!tb.sub[k].ui) a.cmem[(size_t)k * a.M + m] = sc[k * kNetCells + lc];
+      if (!fx[k].ui) a.cmem[(size_t)k * a.M + m] = sc[k * kNetCells + lc];
   }
   if (blockIdx.x == 0) {
     // the auto-mixed environment: mean over membranes of env - f sa dt / vol_env
