@@ -15,9 +15,10 @@
 //     K-adjacent cores 128 B apart, 8-row groups 1024 B apart), so each tile is
 //     one contiguous 16 KB block;
 //   * the right-hand sides X are split and packed the same way per call;
-//   * one CTA per 128 x 128 output tile: a producer thread streams the four
-//     tiles of each 64-wide K block with cp.async.bulk (TMA engine) into a
-//     3-stage ring guarded by mbarriers; one thread issues
+//   * one CTA per output tile of 128 rows and 16 to 128 columns (tile_width): a
+//     producer thread streams the four operand tiles of each 64-wide K block
+//     with cp.async.bulk (TMA engine) into a ring of 3 to 6 stages guarded by
+//     mbarriers; one thread issues
 //     tcgen05.mma.kind::f16 (BF16 x BF16 -> FP32 in TMEM) for
 //     A_hi.X_hi + A_hi.X_lo + A_lo.X_hi and commits each stage back to the
 //     producer; four epilogue warps read the accumulator with tcgen05.ld and
@@ -46,22 +47,25 @@ namespace bxg {
 
 using namespace bxtc;
 
-constexpr int BM = 128, BN = 128, BK = 64, STAGES = 3;
+constexpr int BM = 128, BN = 128, BK = 64;           // BN: columns of a packed tile of X^T
 constexpr int TILE = BM * BK;                        // elements per 128x64 tile
 constexpr int TILE_BYTES = TILE * 2;                 // 16 KB of BF16
-constexpr int STAGE_BYTES = 4 * TILE_BYTES;          // A_hi, A_lo, B_hi, B_lo
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;
 constexpr int kThreads = 192;                        // producer, MMA, 4 epilogue warps
-constexpr uint32_t kTmemCols = BN;                   // FP32 accumulator: 128 lanes x BN columns
 constexpr unsigned int kErrTimeout = 1u;
 
-// kind::f16 instruction descriptor: FP32 accumulator, BF16 A and B, both K-major
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                            ((uint32_t)(BM >> 4) << 24);
-
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t accum) {
-  mma_f16(d_tmem, a, b, kIdesc, accum);
-}
+// An output tile NW columns wide reads NW rows of a packed X^T tile, which are
+// contiguous there (8-row groups).
+template <int NW>
+struct Shape {
+  static constexpr int b_bytes = NW * BK * 2;
+  static constexpr int stage_bytes = 2 * (TILE_BYTES + b_bytes);       // A_hi, A_lo, B_hi, B_lo
+  static constexpr int stages = NW == 128 ? 3 : NW == 64 ? 4 : NW == 32 ? 5 : 6;
+  static constexpr int smem = stages * stage_bytes + 1024;
+  static constexpr uint32_t tmem_cols = NW < 32 ? 32 : NW;             // FP32 accumulator: 128 lanes x NW columns
+  // kind::f16 instruction descriptor: FP32 accumulator, BF16 A and B, both K-major
+  static constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NW >> 3) << 17) |
+                                    ((uint32_t)(BM >> 4) << 24);
+};
 
 struct GemmArgs {
   const __nv_bfloat16* a_hi;  // [Mt][Kt] tiles
@@ -73,17 +77,26 @@ struct GemmArgs {
   double* Y;                  // row-major [m][ldy]
   int ldy;
   int accumulate;             // Y += A X instead of Y = A X
-  unsigned int* err;
+  unsigned int* err;          // mapped host memory
 };
 
+// Bound by the chain of dependent MMAs on one accumulator: 12 a K block, some
+// 95 cycles each even at 16 columns (64 would fill the tensor core at 128), so
+// a K block takes 0.6 us at every width and what counts is how many SMs run
+// one.  3001 x 3001 on 96 columns: 24 CTAs of 128 columns 40.8 us, 144 of 16
+// columns 27.8 (a launch among others).
+template <int NW>
 __global__ void __launch_bounds__(kThreads, 1) k_gemm_bf16x3(GemmArgs g) {
+  using SH = Shape<NW>;
+  constexpr int STAGES = SH::stages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], accum_full;
   __shared__ uint32_t tmem_base;
   __shared__ int failed;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nt = blockIdx.x, mt = blockIdx.y, Kt = g.Kt;  // N-tiles of one row block run together (A shared in L2)
+  const int mt = blockIdx.y, Kt = g.Kt;         // N-tiles of one row block run together (A shared in L2)
+  const int col0 = blockIdx.x * NW, nt = col0 / BN;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -97,7 +110,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_bf16x3(GemmArgs g) {
   __syncwarp();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                 "r"(kTmemCols));
+                 "r"(SH::tmem_cols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -119,13 +132,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_bf16x3(GemmArgs g) {
         break;
       }
       const uint32_t fb = smem_u32(&full[s]);
-      const uint32_t dst = smem_u32(smem + (size_t)s * STAGE_BYTES);
-      const size_t ao = ((size_t)mt * Kt + kb) * TILE, bo = ((size_t)nt * Kt + kb) * TILE;
-      mbar_expect_tx(fb, STAGE_BYTES);
+      const uint32_t dst = smem_u32(smem + (size_t)s * SH::stage_bytes);
+      const size_t ao = ((size_t)mt * Kt + kb) * TILE, bo = ((size_t)nt * Kt + kb) * TILE + (size_t)(col0 % BN) * BK;
+      mbar_expect_tx(fb, SH::stage_bytes);
       bulk_g2s(dst, g.a_hi + ao, TILE_BYTES, fb);
       bulk_g2s(dst + TILE_BYTES, g.a_lo + ao, TILE_BYTES, fb);
-      bulk_g2s_hint(dst + 2 * TILE_BYTES, g.b_hi + bo, TILE_BYTES, fb, keep);
-      bulk_g2s_hint(dst + 3 * TILE_BYTES, g.b_lo + bo, TILE_BYTES, fb, keep);
+#if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 900)
+      if (kb == 0) cudaGridDependencySynchronize();   // X is packed from here on
+#endif
+      bulk_g2s_hint(dst + 2 * TILE_BYTES, g.b_hi + bo, SH::b_bytes, fb, keep);
+      bulk_g2s_hint(dst + 2 * TILE_BYTES + SH::b_bytes, g.b_lo + bo, SH::b_bytes, fb, keep);
       issued = kb + 1;
     }
     // drain: the last copies of each stage have landed before the CTA can exit
@@ -141,17 +157,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_bf16x3(GemmArgs g) {
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t base = smem_u32(smem + (size_t)s * STAGE_BYTES);
+      const uint32_t base = smem_u32(smem + (size_t)s * SH::stage_bytes);
 #pragma unroll
       for (int kk = 0; kk < BK / 16; ++kk) {
         const uint32_t o = (uint32_t)kk * 256u;  // two K-adjacent core matrices per MMA (K = 16)
         const uint64_t ah = smem_desc(base + o, 128, 1024);
         const uint64_t al = smem_desc(base + TILE_BYTES + o, 128, 1024);
         const uint64_t bh = smem_desc(base + 2 * TILE_BYTES + o, 128, 1024);
-        const uint64_t bl = smem_desc(base + 3 * TILE_BYTES + o, 128, 1024);
-        mma_bf16(tmem, ah, bh, (kb > 0 || kk > 0) ? 1u : 0u);
-        mma_bf16(tmem, ah, bl, 1u);
-        mma_bf16(tmem, al, bh, 1u);
+        const uint64_t bl = smem_desc(base + 2 * TILE_BYTES + SH::b_bytes + o, 128, 1024);
+        mma_f16(tmem, ah, bh, SH::idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+        mma_f16(tmem, ah, bl, SH::idesc, 1u);
+        mma_f16(tmem, al, bh, SH::idesc, 1u);
       }
       mma_commit(smem_u32(&empty[s]));  // stage free once these MMAs have read it
     }
@@ -166,14 +182,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_bf16x3(GemmArgs g) {
       failed = 1;
     } else {
       const int row = mt * BM + q * 32 + lane;
-      for (int c0 = 0; c0 < BN; c0 += 16) {
+      for (int c0 = 0; c0 < NW; c0 += 16) {
         float v[16];
         tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
         if (row < g.m) {
           double* yr = g.Y + (size_t)row * g.ldy;
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const int col = nt * BN + c0 + i;
+            const int col = col0 + c0 + i;
             if (col < g.ncols) yr[col] = g.accumulate ? yr[col] + (double)v[i] : (double)v[i];
           }
         }
@@ -185,26 +201,83 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_bf16x3(GemmArgs g) {
   if (warp == 0) {
     __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(SH::tmem_cols));
   }
-  if (threadIdx.x == 0 && failed) atomicOr(g.err, kErrTimeout);
+  if (threadIdx.x == 0 && failed) {
+    *(volatile unsigned int*)g.err = kErrTimeout;
+    __threadfence_system();
+  }
+}
+
+// Columns of an output tile: the fewest waves of one CTA an SM, and of those
+// widths the narrowest.  A wave lasts as long as its chain of MMAs at every
+// width and only slightly longer at a wider one (n = 3001, us: 16 columns in
+// tiles of 16 / 32 / 64 / 128 28.8 / 28.8 / 30.9 / 34.9); a second wave doubles
+// it (128 columns 55 / 30.8 / 32.9 / 37.5, 250 columns 81 / 57 / 32.9 / 37.0).
+// The same sums in the same order at every width.
+inline int tile_width(int Mt, int nrhs, int sms) {
+  int best = 128;
+  long long fewest = 0;
+  for (int w = 128; w >= 16; w /= 2) {
+    const long long waves = ((long long)Mt * ((nrhs + w - 1) / w) + sms - 1) / sms;
+    if (w == 128 || waves <= fewest) {
+      best = w;
+      fewest = waves;
+    }
+  }
+  return best;
+}
+
+template <int NW>
+cudaError_t launch_gemm_w(const GemmArgs& g, int Mt, cudaStream_t s) {
+  using SH = Shape<NW>;
+  cudaError_t e = cudaFuncSetAttribute(k_gemm_bf16x3<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SH::smem);
+  if (e != cudaSuccess) return e;
+  // programmatic dependent launch: the set-up and the first A tiles overlap the
+  // end of the kernel that packs X
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((g.ncols + NW - 1) / NW), (unsigned)Mt);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = SH::smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_gemm_bf16x3<NW>, g);
+}
+
+inline cudaError_t launch_gemm(const GemmArgs& g, int Mt, int sms, cudaStream_t s) {
+  switch (tile_width(Mt, g.ncols, sms)) {
+    case 16: return launch_gemm_w<16>(g, Mt, s);
+    case 32: return launch_gemm_w<32>(g, Mt, s);
+    case 64: return launch_gemm_w<64>(g, Mt, s);
+    default: return launch_gemm_w<128>(g, Mt, s);
+  }
 }
 
 // Split src (FP64, element (r, k) at src[r*ld_r + k*ld_k]) into packed BF16
-// hi/lo tiles [rows/128][cols/64], zero outside [0,rows) x [0,cols).
+// hi/lo tiles [rows/128][cols/64], zero outside [0,rows) x [0,cols).  A thread
+// holds eight consecutive k of one row, a 16-byte piece of a core matrix;
+// neighbouring threads hold neighbouring rows, which X^T has contiguous.
 __global__ void k_pack_split(const double* __restrict__ src, int rows, int cols, long long ld_r, long long ld_k,
                              int Kt, long long n_el, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n_el;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long tile = e / TILE;
-    const int w = (int)(e - tile * TILE);
-    const int core = w >> 6, in = w & 63;
-    const int r = ((core >> 3) << 3) + (in >> 3), k = ((core & 7) << 3) + (in & 7);
-    const int row = (int)(tile / Kt) * BM + r, col = (int)(tile % Kt) * BK + k;
-    const double a = (row < rows && col < cols) ? src[(long long)row * ld_r + (long long)col * ld_k] : 0.0;
-    const __nv_bfloat16 h = __double2bfloat16(a);
-    hi[e] = h;
-    lo[e] = __double2bfloat16(a - (double)__bfloat162float(h));
+  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n_el / 8;
+       p += (long long)gridDim.x * blockDim.x) {
+    const long long tile = p / (TILE / 8);
+    const int w = (int)(p - tile * (TILE / 8)), r = w & (BM - 1), k8 = w / BM;
+    const int row = (int)(tile / Kt) * BM + r, col = (int)(tile % Kt) * BK + 8 * k8;
+    __align__(16) __nv_bfloat16 h[8], l[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const double a = (row < rows && col + q < cols) ? src[(long long)row * ld_r + (long long)(col + q) * ld_k] : 0.0;
+      h[q] = __double2bfloat16(a);
+      l[q] = __double2bfloat16(a - (double)__bfloat162float(h[q]));
+    }
+    const long long d = tile * TILE + (((r >> 3) << 3) + k8) * 64 + (r & 7) * 8;
+    *reinterpret_cast<uint4*>(hi + d) = *reinterpret_cast<const uint4*>(h);
+    *reinterpret_cast<uint4*>(lo + d) = *reinterpret_cast<const uint4*>(l);
   }
 }
 
@@ -257,7 +330,8 @@ struct bx_dense_op {
   int cap_rhs = 0;                          // packed-X and residual capacity (columns)
   __nv_bfloat16 *b_hi = nullptr, *b_lo = nullptr;
   double* resid = nullptr;
-  unsigned int* err = nullptr;
+  unsigned int* err = nullptr;              // mapped host memory: read after a synchronisation
+  int sms = 152;
 };
 
 namespace {
@@ -297,16 +371,24 @@ unsigned grid_for(long long n_el) {
 
 // Y (=|+=) A X on stream s, X and Y [n][nrhs] row-major on the device
 int gemm(bx_dense_op* op, const double* X, double* Y, int nrhs, bool accumulate, cudaStream_t s) {
-  const int Nt = (nrhs + bxg::BN - 1) / bxg::BN;
-  const long long n_el = (long long)Nt * op->Kt * bxg::TILE;
+  const long long n_el = (long long)((nrhs + bxg::BN - 1) / bxg::BN) * op->Kt * bxg::TILE;
   // B operand is X^T: element (j, k) = X[k][j]
-  bxg::k_pack_split<<<grid_for(n_el), 256, 0, s>>>(X, nrhs, op->n, 1, nrhs, op->Kt, n_el, op->b_hi, op->b_lo);
+  bxg::k_pack_split<<<grid_for(n_el / 8), 256, 0, s>>>(X, nrhs, op->n, 1, nrhs, op->Kt, n_el, op->b_hi, op->b_lo);
   GX(cudaGetLastError());
-  bxg::GemmArgs a{op->a_hi, op->a_lo, op->b_hi, op->b_lo, op->Kt, op->n, nrhs, Y, nrhs, accumulate ? 1 : 0,
-                  op->err};
-  bxg::k_gemm_bf16x3<<<dim3((unsigned)Nt, (unsigned)op->Mt), bxg::kThreads, bxg::SMEM_BYTES, s>>>(a);
-  GX(cudaGetLastError());
+  GX(bxg::launch_gemm(bxg::GemmArgs{op->a_hi, op->a_lo, op->b_hi, op->b_lo, op->Kt, op->n, nrhs, Y, nrhs,
+                                    accumulate ? 1 : 0, op->err},
+                      op->Mt, op->sms, s));
   return BX_OK;
+}
+
+// the error word, in mapped host memory, and the device's size
+cudaError_t alloc_err(bx_dense_op* op) {
+  cudaError_t e = cudaHostAlloc(&op->err, sizeof(unsigned int), cudaHostAllocMapped);
+  if (e != cudaSuccess) return e;
+  *op->err = 0u;
+  int dev = 0;
+  e = cudaGetDevice(&dev);
+  return e != cudaSuccess ? e : cudaDeviceGetAttribute(&op->sms, cudaDevAttrMultiProcessorCount, dev);
 }
 
 }  // namespace
@@ -316,7 +398,6 @@ extern "C" {
 int bx_dense_op_create(const double* A, int n, bx_dense_op_handle* out) {
   if (!A || !out || n <= 0) return gfail(BX_EINVAL, "bx_dense_op_create: bad arguments");
   *out = nullptr;
-  GX(cudaFuncSetAttribute(bxg::k_gemm_bf16x3, cudaFuncAttributeMaxDynamicSharedMemorySize, bxg::SMEM_BYTES));
   bx_dense_op* op = new bx_dense_op();
   op->n = n;
   op->Mt = (n + bxg::BM - 1) / bxg::BM;
@@ -326,13 +407,11 @@ int bx_dense_op_create(const double* A, int n, bx_dense_op_handle* out) {
   const size_t rows_per = std::max<size_t>(bxg::BM, ((size_t)256 << 20) / ((size_t)n * sizeof(double)) / bxg::BM * bxg::BM);
   int rc = BX_OK;
   if (cudaMalloc(&op->a_hi, el * 2) != cudaSuccess || cudaMalloc(&op->a_lo, el * 2) != cudaSuccess ||
-      cudaMalloc(&op->err, sizeof(unsigned int)) != cudaSuccess ||
+      alloc_err(op) != cudaSuccess ||
       cudaMalloc(&stage, std::min<size_t>(rows_per, (size_t)n) * n * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     rc = gfail(BX_ENOMEM, "cudaMalloc dense operator");
   }
-  if (rc == BX_OK && cudaMemset(op->err, 0, sizeof(unsigned int)) != cudaSuccess)
-    rc = gfail(BX_ECUDA, "cudaMemset");
   // split row blocks (whole 128-row tile rows) through a bounded staging buffer
   for (size_t r0 = 0; rc == BX_OK && r0 < (size_t)n; r0 += rows_per) {
     const size_t nr = std::min(rows_per, (size_t)n - r0);
@@ -343,7 +422,7 @@ int bx_dense_op_create(const double* A, int n, bx_dense_op_handle* out) {
     const int mt0 = (int)(r0 / bxg::BM), mtn = (int)((nr + bxg::BM - 1) / bxg::BM);
     const long long n_el = (long long)mtn * op->Kt * bxg::TILE;
     const size_t off = (size_t)mt0 * op->Kt * bxg::TILE;
-    bxg::k_pack_split<<<grid_for(n_el), 256>>>(stage, (int)nr, n, n, 1, op->Kt, n_el, op->a_hi + off,
+    bxg::k_pack_split<<<grid_for(n_el / 8), 256>>>(stage, (int)nr, n, n, 1, op->Kt, n_el, op->a_hi + off,
                                                op->a_lo + off);
     if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
       rc = gfail(BX_ECUDA, "dense operator split");
@@ -360,20 +439,18 @@ int bx_dense_op_create(const double* A, int n, bx_dense_op_handle* out) {
 int bx_dense_op_create_empty(int n, bx_dense_op_handle* out) {
   if (!out || n <= 0) return gfail(BX_EINVAL, "bx_dense_op_create_empty: bad arguments");
   *out = nullptr;
-  GX(cudaFuncSetAttribute(bxg::k_gemm_bf16x3, cudaFuncAttributeMaxDynamicSharedMemorySize, bxg::SMEM_BYTES));
   bx_dense_op* op = new bx_dense_op();
   op->n = n;
   op->Mt = (n + bxg::BM - 1) / bxg::BM;
   op->Kt = (n + bxg::BK - 1) / bxg::BK;
   const size_t el = (size_t)op->Mt * op->Kt * bxg::TILE;
   if (cudaMalloc(&op->a_hi, el * 2) != cudaSuccess || cudaMalloc(&op->a_lo, el * 2) != cudaSuccess ||
-      cudaMalloc(&op->err, sizeof(unsigned int)) != cudaSuccess) {
+      alloc_err(op) != cudaSuccess) {
     cudaGetLastError();
     bx_dense_op_destroy(op);
     return gfail(BX_ENOMEM, "cudaMalloc dense operator");
   }
-  if (cudaMemset(op->a_hi, 0, el * 2) != cudaSuccess || cudaMemset(op->a_lo, 0, el * 2) != cudaSuccess ||
-      cudaMemset(op->err, 0, sizeof(unsigned int)) != cudaSuccess) {
+  if (cudaMemset(op->a_hi, 0, el * 2) != cudaSuccess || cudaMemset(op->a_lo, 0, el * 2) != cudaSuccess) {
     bx_dense_op_destroy(op);
     return gfail(BX_ECUDA, "cudaMemset dense operator");
   }
@@ -447,10 +524,8 @@ int bx_dense_op_apply(bx_dense_op_handle op, const double* X, double* Y, int nrh
 
 int bx_dense_op_status(bx_dense_op_handle op, int* timed_out) {
   if (!op || !timed_out) return gfail(BX_EINVAL, "null argument");
-  unsigned int e = 0;
   GX(cudaDeviceSynchronize());
-  GX(cudaMemcpy(&e, op->err, sizeof(e), cudaMemcpyDeviceToHost));
-  *timed_out = (e & bxg::kErrTimeout) ? 1 : 0;
+  *timed_out = (*(volatile unsigned int*)op->err & bxg::kErrTimeout) ? 1 : 0;
   return BX_OK;
 }
 
@@ -460,15 +535,12 @@ int bx_dense_op_time(bx_dense_op_handle op, const double* X, double* Y, int nrhs
   if (rc != BX_OK) return rc;
   rc = gemm(op, X, Y, nrhs, false, nullptr);  // warm-up (also packs X)
   if (rc != BX_OK) return rc;
-  const int Nt = (nrhs + bxg::BN - 1) / bxg::BN;
   bxg::GemmArgs a{op->a_hi, op->a_lo, op->b_hi, op->b_lo, op->Kt, op->n, nrhs, Y, nrhs, 0, op->err};
   cudaEvent_t e0, e1;
   GX(cudaEventCreate(&e0));
   GX(cudaEventCreate(&e1));
   GX(cudaEventRecord(e0, nullptr));
-  for (int i = 0; i < n_iter; ++i)
-    bxg::k_gemm_bf16x3<<<dim3((unsigned)Nt, (unsigned)op->Mt), bxg::kThreads, bxg::SMEM_BYTES>>>(a);
-  GX(cudaGetLastError());
+  for (int i = 0; i < n_iter; ++i) GX(bxg::launch_gemm(a, op->Mt, op->sms, nullptr));
   GX(cudaEventRecord(e1, nullptr));
   GX(cudaEventSynchronize(e1));
   float t = 0.f;
@@ -489,7 +561,7 @@ int bx_dense_op_destroy(bx_dense_op_handle op) {
   cudaFree(op->b_hi);
   cudaFree(op->b_lo);
   cudaFree(op->resid);
-  cudaFree(op->err);
+  cudaFreeHost(op->err);
   delete op;
   return BX_OK;
 }
