@@ -899,6 +899,47 @@ cudaError_t enqueue_env(bx_cluster* h, bool out, bool flux_done, cudaStream_t s)
   return cudaGetLastError();
 }
 
+// Copies of one call, gathered: arrays that both lie on this device go by one
+// k_copy_list launch, the others (host memory, another device) by a copy each.
+class Copies {
+ public:
+  explicit Copies(cudaStream_t s) : s_(s) { cudaGetDevice(&dev_); }
+  cudaError_t add(double* dst, const double* src, size_t n) {
+    if (!dst || !src || n == 0) return cudaSuccess;
+    if (!here(dst) || !here(src) || n > (size_t)1 << 30)
+      return cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDefault, s_);
+    if (l_.count == bx::kCopyMax) {
+      const cudaError_t e = run();
+      if (e != cudaSuccess) return e;
+    }
+    l_.dst[l_.count] = dst;
+    l_.src[l_.count] = src;
+    l_.n[l_.count] = (long long)n;
+    l_.first[l_.count + 1] = l_.first[l_.count] + (int)((n + bx::kCopyBlock - 1) / bx::kCopyBlock);
+    ++l_.count;
+    return cudaSuccess;
+  }
+  cudaError_t run() {
+    if (l_.count == 0) return cudaSuccess;
+    bx::k_copy_list<<<(unsigned)l_.first[l_.count], 256, 0, s_>>>(l_);
+    l_.count = 0;
+    return cudaGetLastError();
+  }
+
+ private:
+  bool here(const void* p) const {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == dev_ && ((uintptr_t)p & 7) == 0;
+  }
+  cudaStream_t s_;
+  int dev_ = 0;
+  bx::CopyList l_{};
+};
+
 // Enqueue one time step (reads parity, writes parity^1).
 cudaError_t enqueue_step(bx_cluster* h, int parity, bool out, cudaStream_t s) {
   cudaError_t e;
@@ -1805,13 +1846,24 @@ int bx_state_upload(bx_handle h, const bx_state* s) {
   h->have_state = false;
   double* vm_dst = split ? h->st_vm : h->d_vm[0];
   double* cc_dst = split ? h->st_cc : h->d_cc;
-  BX_CU(cudaMemcpyAsync(vm_dst, s->vm, (size_t)M * sizeof(double), cudaMemcpyDefault, st));
-  BX_CU(cudaMemcpyAsync(cc_dst, s->cc_cells, (size_t)I * C * sizeof(double), cudaMemcpyDefault, st));
-  BX_CU(cudaMemcpyAsync(h->st_cam, s->cc_at_mem, (size_t)I * M * sizeof(double), cudaMemcpyDefault, st));
+  Copies cp(st);
+  BX_CU(cp.add(vm_dst, s->vm, M));
+  BX_CU(cp.add(cc_dst, s->cc_cells, (size_t)I * C));
+  BX_CU(cp.add(h->st_cam, s->cc_at_mem, (size_t)I * M));
+  BX_CU(cp.add(h->d_cenv, s->cc_env, nenv));
+  if (h->vgj) BX_CU(cp.add(split ? h->st_go : h->d_gjo, s->gjopen ? s->gjopen : h->d_gj_w, M));
+  if (h->ecm) {
+    BX_CU(cp.add(h->d_Ex, s->E_env_x, h->G));
+    BX_CU(cp.add(h->d_Ey, s->E_env_y, h->G));
+  }
+  BX_CU(cp.run());
   BX_CU(cudaMemsetAsync(h->d_flag, 0, 2 * sizeof(int), st));
   const int tb = 256;
-  bx::k_state_check<<<(M + tb - 1) / tb, tb, 0, st>>>(io, vm_dst, h->st_cam, split ? 1 : 2, h->d_flag);
+  bx::k_state_check<<<(M + tb - 1) / tb, tb, 0, st>>>(io, vm_dst, h->st_cam, split ? 1 : 2, h->d_flag,
+                                                      split ? nullptr : h->d_ccm[0]);
   BX_CU(cudaGetLastError());
+  for (unsigned* c : {h->r_ctl, h->pl_ctl})
+    if (c) BX_CU(cudaMemsetAsync(c, 0, 2 * sizeof(unsigned), st));   // a fresh state: no timeout
   int flag[2] = {0, 0};
   BX_CU(cudaMemcpyAsync(flag, h->d_flag, sizeof(flag), cudaMemcpyDeviceToHost, st));
   BX_CU(cudaStreamSynchronize(st));
@@ -1828,40 +1880,16 @@ int bx_state_upload(bx_handle h, const bx_state* s) {
                                                             h->s_cc2);
     BX_CU(cudaGetLastError());
     if (h->vgj) {
-      if (s->gjopen)
-        BX_CU(cudaMemcpyAsync(h->st_go, s->gjopen, (size_t)M * sizeof(double), cudaMemcpyDefault, st));
-      else
-        BX_CU(cudaMemcpyAsync(h->st_go, h->d_gj_w, (size_t)M * sizeof(double), cudaMemcpyDeviceToDevice, st));
       BX_CU(cudaMemsetAsync(h->t_gjo, 0, (size_t)h->Q * sizeof(float), st));
       bx::k_state_pack_gjo<<<(M + tb - 1) / tb, tb, 0, st>>>(io, h->st_go, h->t_gjo);
       BX_CU(cudaGetLastError());
     }
-    BX_CU(cudaMemcpyAsync(h->d_cenv, s->cc_env, nenv * sizeof(double), cudaMemcpyDefault, st));
-    if (h->ecm) {
-      BX_CU(cudaMemcpyAsync(h->d_Ex, s->E_env_x, (size_t)h->G * sizeof(double), cudaMemcpyDefault, st));
-      BX_CU(cudaMemcpyAsync(h->d_Ey, s->E_env_y, (size_t)h->G * sizeof(double), cudaMemcpyDefault, st));
-    } else {
+    if (!h->ecm) {
       k_round_to_float<<<(unsigned)((nenv + 255) / 256), 256, 0, st>>>(h->d_cenv, h->s_cenv_f, (int)nenv);
       BX_CU(cudaGetLastError());
     }
-  } else {
-    bx::k_state_pack_ccm<<<(C + tb - 1) / tb, tb, 0, st>>>(io, h->st_cam, h->d_ccm[0]);
-    BX_CU(cudaGetLastError());
-    BX_CU(cudaMemcpyAsync(h->d_cenv, s->cc_env, nenv * sizeof(double), cudaMemcpyDefault, st));
-    if (h->vgj) {
-      if (s->gjopen)
-        BX_CU(cudaMemcpyAsync(h->d_gjo, s->gjopen, (size_t)M * sizeof(double), cudaMemcpyDefault, st));
-      else
-        BX_CU(cudaMemcpyAsync(h->d_gjo, h->d_gj_w, (size_t)M * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    }
-    if (h->ecm) {
-      BX_CU(cudaMemcpyAsync(h->d_Ex, s->E_env_x, (size_t)h->G * sizeof(double), cudaMemcpyDefault, st));
-      BX_CU(cudaMemcpyAsync(h->d_Ey, s->E_env_y, (size_t)h->G * sizeof(double), cudaMemcpyDefault, st));
-    }
+    BX_CU(cudaStreamSynchronize(st));
   }
-  for (unsigned* c : {h->r_ctl, h->pl_ctl})
-    if (c) BX_CU(cudaMemsetAsync(c, 0, 2 * sizeof(unsigned), st));   // a fresh state: no timeout
-  BX_CU(cudaStreamSynchronize(st));
   h->have_state = true;
   h->have_outputs = false;
   h->last_step_outputs = false;
@@ -1879,9 +1907,7 @@ int bx_state_download(bx_handle h, bx_state* s) {
   const bx::StateIO io = state_io(h);
   const size_t nenv = h->ecm ? (size_t)I * h->G : (size_t)h->ncl * I;
   const int tb = 256;
-  auto d2h = [&](double* dst, const double* src, size_t n) {
-    return dst ? cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDefault, st) : cudaSuccess;
-  };
+  Copies cp(st);
   if (h->mode == MODE_SPLIT) {
     const int n = std::max(M, C);
     const bool go = h->vgj && s->gjopen;
@@ -1889,22 +1915,23 @@ int bx_state_download(bx_handle h, bx_state* s) {
                                                               go ? h->t_gjo : nullptr, h->st_vm, h->st_cam,
                                                               h->st_cc, h->st_go);
     BX_CU(cudaGetLastError());
-    BX_CU(d2h(s->vm, h->st_vm, M));
-    BX_CU(d2h(s->cc_cells, h->st_cc, (size_t)I * C));
-    if (go) BX_CU(d2h(s->gjopen, h->st_go, M));
+    BX_CU(cp.add(s->vm, h->st_vm, M));
+    BX_CU(cp.add(s->cc_cells, h->st_cc, (size_t)I * C));
+    if (go) BX_CU(cp.add(s->gjopen, h->st_go, M));
   } else {
     bx::k_state_unpack_cam<<<(M + tb - 1) / tb, tb, 0, st>>>(io, h->d_ccm[h->parity], h->st_cam);
     BX_CU(cudaGetLastError());
-    BX_CU(d2h(s->vm, h->d_vm[h->parity], M));
-    BX_CU(d2h(s->cc_cells, h->d_cc, (size_t)I * C));
-    if (h->vgj) BX_CU(d2h(s->gjopen, h->d_gjo, M));
+    BX_CU(cp.add(s->vm, h->d_vm[h->parity], M));
+    BX_CU(cp.add(s->cc_cells, h->d_cc, (size_t)I * C));
+    if (h->vgj) BX_CU(cp.add(s->gjopen, h->d_gjo, M));
   }
-  BX_CU(d2h(s->cc_at_mem, h->st_cam, (size_t)I * M));
+  BX_CU(cp.add(s->cc_at_mem, h->st_cam, (size_t)I * M));
   if (h->ecm) {
-    BX_CU(d2h(s->E_env_x, h->d_Ex, h->G));
-    BX_CU(d2h(s->E_env_y, h->d_Ey, h->G));
+    BX_CU(cp.add(s->E_env_x, h->d_Ex, h->G));
+    BX_CU(cp.add(s->E_env_y, h->d_Ey, h->G));
   }
-  BX_CU(d2h(s->cc_env, h->d_cenv, nenv));
+  BX_CU(cp.add(s->cc_env, h->d_cenv, nenv));
+  BX_CU(cp.run());
   BX_CU(cudaStreamSynchronize(st));
   return BX_OK;
 }
@@ -2023,20 +2050,20 @@ int bx_step(bx_handle h, int n_steps, int want_outputs, void* stream) {
 int bx_status(bx_handle h, bx_step_status* st) {
   if (!h || !st) return fail(BX_EINVAL, "null argument");
   unsigned long long v[4];
+  unsigned ctl[2] = {0u, 0u};
+  unsigned* rc = h->mode == MODE_SPLIT ? h->r_ctl : h->pl_res ? h->pl_ctl : nullptr;
+  BX_CU(cudaMemcpyAsync(v, h->d_status, sizeof(v), cudaMemcpyDeviceToHost, h->stream));
+  if (rc) BX_CU(cudaMemcpyAsync(ctl, rc, sizeof(ctl), cudaMemcpyDeviceToHost, h->stream));
   BX_CU(cudaStreamSynchronize(h->stream));
-  BX_CU(cudaMemcpy(v, h->d_status, sizeof(v), cudaMemcpyDeviceToHost));
   st->steps_done = h->steps_done;
   st->nan_vm = (int32_t)std::min<unsigned long long>(v[0], 0x7fffffff);
   st->nan_conc = (int32_t)std::min<unsigned long long>(v[1], 0x7fffffff);
   st->neg_clamped = (int64_t)v[2];
   st->unstable = (v[0] || v[1]) ? 1 : 0;
   st->precision = h->precision;
-  unsigned* rc = h->mode == MODE_SPLIT ? h->r_ctl : h->pl_res ? h->pl_ctl : nullptr;
   if (rc) {
     // the resident kernel's grid barrier gave up (its wait is bounded): the
     // state of that run is incomplete
-    unsigned ctl[2] = {0u, 0u};
-    BX_CU(cudaMemcpy(ctl, rc, sizeof(ctl), cudaMemcpyDeviceToHost));
     if (ctl[1]) {
       h->have_state = false;
       BX_CU(cudaMemset(rc, 0, sizeof(ctl)));
@@ -2068,8 +2095,10 @@ int bx_outputs_download(bx_handle h, bx_outputs* o) {
       {o->rho_env, h->ecm ? h->d_rho_env : nullptr, G},
       {o->v_env, h->ecm ? h->d_venv : nullptr, G},
   };
-  for (const Pair& p : pairs)
-    if (p.dst && p.src) BX_CU(cudaMemcpy(p.dst, p.src, p.n * sizeof(double), cudaMemcpyDefault));
+  Copies cp(h->stream);
+  for (const Pair& p : pairs) BX_CU(cp.add(p.dst, p.src, p.n));
+  BX_CU(cp.run());
+  BX_CU(cudaStreamSynchronize(h->stream));
   return BX_OK;
 }
 
@@ -2757,10 +2786,9 @@ int bx_env_fields(bx_handle h, const double* D_env_weight, double* v_env, double
   if (rc != BX_OK) return rc;
   const size_t G = (size_t)h->G;
   double* dst[6] = {v_env, E_env_x, E_env_y, J_env_x, J_env_y, B_field};
-  for (int q = 0; q < 6; ++q)
-    if (dst[q])
-      BX_CU(cudaMemcpyAsync(dst[q], h->f_buf + (size_t)q * G, G * sizeof(double), cudaMemcpyDefault,
-                            h->stream));
+  Copies cp(h->stream);
+  for (int q = 0; q < 6; ++q) BX_CU(cp.add(dst[q], h->f_buf + (size_t)q * G, G));
+  BX_CU(cp.run());
   BX_CU(cudaStreamSynchronize(h->stream));
   return BX_OK;
 }

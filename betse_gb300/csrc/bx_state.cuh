@@ -28,16 +28,52 @@ __device__ __forceinline__ double state_phib(const StateIO& io, int m) {
   return io.phib_on ? io.phib[io.map_env[m]] : 0.0;
 }
 
+// Several arrays copied by one launch: a block takes 1024 doubles of one of
+// them.  (A copy engine takes a call and some 5 us for each array.)
+constexpr int kCopyMax = 24, kCopyBlock = 1024;
+struct CopyList {
+  double* dst[kCopyMax];
+  const double* src[kCopyMax];
+  long long n[kCopyMax];
+  int first[kCopyMax + 1];          // first block of each array
+  int count;
+};
+__global__ void __launch_bounds__(256) k_copy_list(CopyList l) {
+  int a = 0;
+  while (a + 1 < l.count && (int)blockIdx.x >= l.first[a + 1]) ++a;
+  const long long o = (long long)((int)blockIdx.x - l.first[a]) * kCopyBlock;
+  const double* s = l.src[a] + o;
+  double* d = l.dst[a] + o;
+  const int n = (int)(l.n[a] - o < kCopyBlock ? l.n[a] - o : kCopyBlock);
+  double v[kCopyBlock / 256];
+#pragma unroll
+  for (int q = 0; q < kCopyBlock / 256; ++q) {
+    const int t = threadIdx.x + 256 * q;
+    if (t < n) v[q] = s[t];
+  }
+#pragma unroll
+  for (int q = 0; q < kCopyBlock / 256; ++q) {
+    const int t = threadIdx.x + 256 * q;
+    if (t < n) d[t] = v[q];
+  }
+}
+
 // The checks of bx_state_upload, one thread per membrane: flag[0] when
 // cc_at_mem differs from its cell's first membrane (a NaN differs too), flag[1]
 // when vm + Phi_b is not uniform over the cell (check_vm 1, the split form: to
 // rounding; 2, the plain form: bit for bit, which its factored step needs).
+// Plain form (ccm): the first membrane's thread also lays down the cell's
+// membrane-side concentrations.
 __global__ void k_state_check(StateIO io, const double* __restrict__ vm, const double* __restrict__ cam,
-                              int check_vm, int* flag) {
+                              int check_vm, int* flag, double* ccm) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= io.M) return;
-  const int f = io.cell_ptr[io.m2c[m]];
-  if (m == f) return;
+  const int c = io.m2c[m], f = io.cell_ptr[c];
+  if (m == f) {
+    if (ccm)
+      for (int i = 0; i < io.I; ++i) ccm[(size_t)i * io.C + c] = cam[(size_t)i * io.M + f];
+    return;
+  }
   for (int i = 0; i < io.I; ++i)
     if (cam[(size_t)i * io.M + m] != cam[(size_t)i * io.M + f]) { atomicOr(&flag[0], 1); break; }
   if (check_vm) {
@@ -46,14 +82,6 @@ __global__ void k_state_check(StateIO io, const double* __restrict__ vm, const d
     if (check_vm == 2 ? !(v == v0) : fabs(v - v0) > 1e-12 * fabs(v0) + 1e-18)
       if (!*(volatile int*)&flag[1]) atomicOr(&flag[1], 1);
   }
-}
-
-// plain form: the membrane-side concentration of each cell
-__global__ void k_state_pack_ccm(StateIO io, const double* __restrict__ cam, double* ccm) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= io.C) return;
-  const int f = io.cell_ptr[c];
-  for (int i = 0; i < io.I; ++i) ccm[(size_t)i * io.C + c] = cam[(size_t)i * io.M + f];
 }
 
 // split form, one thread per cell: record (membrane-side concentrations, Vmem)
