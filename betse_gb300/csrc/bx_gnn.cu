@@ -55,17 +55,18 @@ __device__ __forceinline__ float2 ld_bf2(const bf16* row, int lane) {
   return __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(row)[lane]);
 }
 
-// x (FP32 [rows][n_in]) -> BF16 [rows][W], zero-padded
-__global__ void k_pack_x(int rows, int n_in, const float* __restrict__ x, bf16* __restrict__ X) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)rows * W) return;
-  const int i = (int)(t / W), f = (int)(t % W);
-  X[t] = __float2bfloat16_rn(f < n_in ? x[(size_t)i * n_in + f] : 0.0f);
+// Programmatic dependent launch: every kernel of a pass waits for the one
+// before it here, after it has fetched what no kernel of the pass writes (the
+// weights, the graph), and lets the next one start as it ends.
+__device__ __forceinline__ void grid_wait() {
+#if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 900)
+  cudaGridDependencySynchronize();
+#endif
 }
 
 // ---- forward layers on the tensor cores
 constexpr int kTcRows = 128;                         // nodes per CTA (the MMA's M)
-constexpr int kTcThreads = 128;                      // four warps: TMEM lanes 32 w .. 32 w + 31
+constexpr int kTcThreads = 256;                      // warp w: TMEM lanes 32 (w % 4) ..., half of the columns
 constexpr int kActTile = kTcRows * W * 2;            // 16 KB of BF16
 constexpr int kWTile = W * W * 2;                    // 8 KB
 constexpr int kTcSmem = 2 * (kActTile + kWTile) + 1024;   // two inputs (MODE 1)
@@ -75,7 +76,7 @@ constexpr uint32_t kIdescFwd = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(
                                ((uint32_t)(kTcRows >> 4) << 24);
 
 // A tile of ROWS rows of a row-major [*][64] BF16 array is ROWS * 8 pieces of
-// 16 bytes; thread t holds pieces t, t + 128, ...  All of a thread's loads
+// 16 bytes; thread t holds pieces t, t + 256, ...  All of a thread's loads
 // are issued before any store, so a tile costs one memory round trip.
 template <int ROWS>
 __device__ __forceinline__ void load_rows(uint4 (&v)[ROWS * 8 / kTcThreads], const bf16* __restrict__ src,
@@ -100,17 +101,52 @@ __device__ __forceinline__ void store_rows(uint8_t* tile, const uint4 (&v)[ROWS 
   }
 }
 
-// MODE 0: encoder  H = relu(in1 W1^T + b)
-// MODE 1: message  R = relu(in1 W1^T + in2 W2^T + b), H = in1 + R
+// eight FP32 values to 16 bytes of BF16
+__device__ __forceinline__ uint4 pack_bf8(const float (&v)[8]) {
+  uint4 u;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) h[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+  return u;
+}
+
+struct FwdArgs {
+  int n;
+  const bf16* in1;                 // [n][W]; MODE 0 writes it (the padded inputs)
+  bf16* in2;                       // MODE 1: the neighbour means, written here
+  const bf16* wb;
+  int off_w1, off_w2;
+  const float* master;
+  int off_b;
+  bf16 *outR, *outH;
+  float* outY;
+  int n_out;
+  unsigned* err;
+  const float* x;                  // MODE 0: [n][n_in]
+  int n_in;
+  const int *ptr, *nbr;            // MODE 1: adjacency
+  int lo;
+};
+
+// MODE 0: encoder  H = relu(x W1^T + b), x zero-padded to W columns in BF16
+// MODE 1: message  R = relu(in1 W1^T + A W2^T + b), H = in1 + R, A the mean of
+//                  in1 over the neighbours: gathered eight lanes a node
+//                  (16 bytes each), four rows in flight, summed in list order
 // MODE 2: decoder  Y = in1 W1^T + b (FP32, first n_out columns)
+// Bound by latency (gather, tile, MMA, read-back in sequence): with the inputs
+// packed and the means formed by kernels of their own a forward pass of 30,858
+// nodes took 92 us, 85 now (and four launches fewer).
 // A wait that runs out (about two seconds) raises *err and leaves the rows
 // unwritten; the TMEM is freed either way.
 template <int MODE>
-__global__ void __launch_bounds__(kTcThreads) k_fwd_tc(int n, const bf16* __restrict__ in1, const bf16* __restrict__ in2,
-                                                       const bf16* __restrict__ wb, int off_w1, int off_w2,
-                                                       const float* __restrict__ master, int off_b,
-                                                       bf16* __restrict__ outR, bf16* __restrict__ outH,
-                                                       float* __restrict__ outY, int n_out, unsigned* err) {
+__global__ void __launch_bounds__(kTcThreads) k_fwd_tc(FwdArgs a) {
+  const int n = a.n, n_out = a.n_out;
+  const bf16 *in1 = a.in1, *wb = a.wb;
+  const float* master = a.master;
+  const int off_w1 = a.off_w1, off_w2 = a.off_w2, off_b = a.off_b;
+  bf16 *outR = a.outR, *outH = a.outH;
+  float* outY = a.outY;
+  unsigned* err = a.err;
   using namespace bxtc;
   extern __shared__ uint8_t tc_smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~uintptr_t(1023));
@@ -124,24 +160,85 @@ __global__ void __launch_bounds__(kTcThreads) k_fwd_tc(int n, const bf16* __rest
   const int r0 = blockIdx.x * kTcRows;
   const int valid = min(kTcRows, n - r0);
 
-  if (MODE == 1) {
-    // both activation tiles in one round trip, then both weight tiles (L2-resident)
-    uint4 va[kTcRows * 8 / kTcThreads], vb[kTcRows * 8 / kTcThreads];
-    load_rows<kTcRows>(va, in1 + (size_t)r0 * W, valid);
-    load_rows<kTcRows>(vb, in2 + (size_t)r0 * W, valid);
-    store_rows<kTcRows>(a1, va);
-    store_rows<kTcRows>(a2, vb);
+  {
     uint4 w1[W * 8 / kTcThreads], w2[W * 8 / kTcThreads];
     load_rows<W>(w1, wb + off_w1, W);
-    load_rows<W>(w2, wb + off_w2, W);
+    if (MODE == 1) load_rows<W>(w2, wb + off_w2, W);
     store_rows<W>(b1, w1);
-    store_rows<W>(b2, w2);
-  } else {
-    uint4 va[kTcRows * 8 / kTcThreads], w1[W * 8 / kTcThreads];
+    if (MODE == 1) store_rows<W>(b2, w2);
+  }
+  if (MODE == 0) {
+    grid_wait();
+    for (int e = (int)threadIdx.x; e < kTcRows * 8; e += kTcThreads) {
+      const int r = e >> 3, c = e & 7;
+      float v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        v[q] = r < valid && 8 * c + q < a.n_in ? a.x[(size_t)(r0 + r) * a.n_in + 8 * c + q] : 0.f;
+      const uint4 u = pack_bf8(v);
+      if (r < valid) reinterpret_cast<uint4*>(const_cast<bf16*>(in1) + (size_t)(r0 + r) * W)[c] = u;
+      *reinterpret_cast<uint4*>(a1 + ((r >> 3) * 8 + c) * 128 + (r & 7) * 16) = u;
+    }
+  } else if (MODE == 1) {
+    constexpr int NP8 = kTcThreads / 8, NIT = kTcRows / NP8;      // nodes a pass, passes
+    const int g8 = (int)threadIdx.x >> 3, c = (int)threadIdx.x & 7;
+    int pa[NIT], pb[NIT], nb[NIT];
+#pragma unroll
+    for (int it = 0; it < NIT; ++it) {
+      const int r = g8 + it * NP8;
+      pa[it] = r < valid ? a.ptr[a.lo + r0 + r] : 0;
+      pb[it] = r < valid ? a.ptr[a.lo + r0 + r + 1] : 0;
+    }
+#pragma unroll
+    for (int it = 0; it < NIT; ++it) nb[it] = pa[it] + c < pb[it] ? a.nbr[pa[it] + c] : -1;
+    grid_wait();
+    uint4 va[kTcRows * 8 / kTcThreads];
     load_rows<kTcRows>(va, in1 + (size_t)r0 * W, valid);
-    load_rows<W>(w1, wb + off_w1, W);
+#pragma unroll
+    for (int it = 0; it < NIT; ++it) {
+      const int r = g8 + it * NP8, deg = pb[it] - pa[it];
+      int most = deg;
+#pragma unroll
+      for (int o = 8; o < 32; o <<= 1) most = max(most, __shfl_xor_sync(FULL, most, o));
+      float s[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) s[q] = 0.f;
+      for (int p0 = 0; p0 < most; p0 += 8) {
+        if (p0 > 0) nb[it] = pa[it] + p0 + c < pb[it] ? a.nbr[pa[it] + p0 + c] : -1;
+#pragma unroll
+        for (int k0 = 0; k0 < 8; k0 += 4) {
+          if (p0 + k0 >= most) break;
+          uint4 h[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int j = __shfl_sync(FULL, nb[it], k0 + u, 8);
+            h[u] = j >= 0 ? reinterpret_cast<const uint4*>(in1 + (size_t)(j - a.lo) * W)[c] : make_uint4(0u, 0u, 0u, 0u);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const __nv_bfloat162* b2v = reinterpret_cast<const __nv_bfloat162*>(&h[u]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const float2 f = __bfloat1622float2(b2v[q]);
+              s[2 * q] += f.x;
+              s[2 * q + 1] += f.y;
+            }
+          }
+        }
+      }
+      if (deg > 0)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s[q] /= (float)deg;
+      const uint4 u = pack_bf8(s);
+      if (r < valid) reinterpret_cast<uint4*>(a.in2 + (size_t)(r0 + r) * W)[c] = u;
+      *reinterpret_cast<uint4*>(a2 + ((r >> 3) * 8 + c) * 128 + (r & 7) * 16) = u;
+    }
     store_rows<kTcRows>(a1, va);
-    store_rows<W>(b1, w1);
+  } else {
+    grid_wait();
+    uint4 va[kTcRows * 8 / kTcThreads];
+    load_rows<kTcRows>(va, in1 + (size_t)r0 * W, valid);
+    store_rows<kTcRows>(a1, va);
   }
   // the tensor core reads shared memory through the async proxy
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -179,23 +276,26 @@ __global__ void __launch_bounds__(kTcThreads) k_fwd_tc(int n, const bf16* __rest
   const bool ok = __all_sync(FULL, mbar_wait(smem_u32(&done), 0u));
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (ok) {
-    float v[W];
+    constexpr int HC = W / 2;                        // this warp's columns
+    const int f0 = (warp >> 2) * HC, r = r0 + (warp & 3) * 32 + lane;
+    float v[HC];
 #pragma unroll
-    for (int c0 = 0; c0 < W; c0 += 16) tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v + c0);
-    const int r = r0 + warp * 32 + lane;
+    for (int c0 = 0; c0 < HC; c0 += 16)
+      tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(f0 + c0), v + c0);
     if (r < n) {
-      const size_t o = (size_t)r * W;
+      const size_t o = (size_t)r * W + f0;
 #pragma unroll
-      for (int f = 0; f < W; ++f) v[f] += master[off_b + f];
+      for (int f = 0; f < HC; ++f) v[f] += master[off_b + f0 + f];
       if (MODE == 2) {
 #pragma unroll
-        for (int f = 0; f < W; ++f)           // constant indices keep v in registers
-          if (f < n_out) outY[(size_t)r * n_out + f] = v[f];
+        for (int f = 0; f < HC; ++f)          // constant indices keep v in registers
+          if (f0 + f < n_out) outY[(size_t)r * n_out + f0 + f] = v[f];
       } else {
 #pragma unroll
-        for (int f8 = 0; f8 < W; f8 += 8) {
+        for (int f8 = 0; f8 < HC; f8 += 8) {
           __align__(16) bf16 rr[8], hh[8];
-          const uint4 x = reinterpret_cast<const uint4*>(in1 + o)[f8 / 8];
+          uint4 x = make_uint4(0u, 0u, 0u, 0u);
+          if (MODE == 1) x = reinterpret_cast<const uint4*>(in1 + o)[f8 / 8];
           const bf16* xb = reinterpret_cast<const bf16*>(&x);
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
@@ -219,27 +319,6 @@ __global__ void __launch_bounds__(kTcThreads) k_fwd_tc(int n, const bf16* __rest
   }
 }
 
-// A_i = mean_{j in nbr(i)} H_j for local nodes i in [0, n) of a range starting at lo
-__global__ void k_agg(int n, int lo, const int* __restrict__ ptr, const int* __restrict__ nbr,
-                      const bf16* __restrict__ H, bf16* __restrict__ A) {
-  const int lane = threadIdx.x & 31;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  for (int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n; i += nw) {
-    const int a = ptr[lo + i], b = ptr[lo + i + 1];
-    float sx = 0.f, sy = 0.f;
-    for (int p = a; p < b; ++p) {
-      const float2 h = ld_bf2(H + (size_t)(nbr[p] - lo) * W, lane);
-      sx += h.x;
-      sy += h.y;
-    }
-    if (b > a) {
-      sx /= (float)(b - a);
-      sy /= (float)(b - a);
-    }
-    reinterpret_cast<__nv_bfloat162*>(A + (size_t)i * W)[lane] = __floats2bfloat162_rn(sx, sy);
-  }
-}
-
 // ---- backward: one kernel per layer
 // A layer's backward is two FP32 products with the same left factor dZ: the
 // input gradients dZ [W1 | W2] (over the layer's outputs) and the weight
@@ -250,7 +329,7 @@ __global__ void k_agg(int n, int lo, const int* __restrict__ ptr, const int* __r
 // the transposed neighbour mean of the layer above's G.  Bound by the FMA pipe
 // (the gradients are FP32); with a warp per node, operands by shuffle and the
 // weight gradients in their own passes a training step of 30,858 nodes took
-// 653 us, 289 now (a middle layer 109 us before, 38 to 46 now).
+// 653 us, 251 now (a middle layer 109 us before, 37 to 46 now).
 constexpr int kBwdT = 256, kBwdRows = 64, kBwdPerSM = 2;
 
 struct BwdArgs {
@@ -324,6 +403,7 @@ __global__ void __launch_bounds__(kBwdT, kBwdPerSM) k_bwd(BwdArgs a) {
       }
     }
   }
+  grid_wait();
   const int F = MODE == BWD_TOP ? a.n_out : W;                   // rows of dZ^T that are not zero
   const float scale = MODE == BWD_TOP ? 2.0f / ((float)a.n * (float)a.n_out) : 0.f;
   float acc[8][CPT], bacc = 0.f, loss = 0.f;
@@ -336,6 +416,7 @@ __global__ void __launch_bounds__(kBwdT, kBwdPerSM) k_bwd(BwdArgs a) {
     const int rows = min(chunk, row1 - i0);
     __syncthreads();                                             // the tile of the chunk before is done with
     // ---- the layer's inputs
+#pragma unroll 4
     for (int q = t; q < rows * (NCOL / 8); q += kBwdT) {
       const int r = q / (NCOL / 8), c8 = q - r * (NCOL / 8);
       const bf16* src = (MODE == BWD_MID && c8 >= W / 8 ? a.in2 : a.in1) + (size_t)(i0 + r) * W + (c8 & 7) * 8;
@@ -349,16 +430,16 @@ __global__ void __launch_bounds__(kBwdT, kBwdPerSM) k_bwd(BwdArgs a) {
     }
     // ---- dZ
     if (MODE == BWD_TOP) {
-      for (int q = t; q < rows * W; q += kBwdT) {
-        const int r = q / W, f = q - r * W;
-        float d = 0.f;
-        if (f < a.n_out) {
-          const size_t o = (size_t)(i0 + r) * a.n_out + f;
-          const float e = a.yhat[o] - a.y[o];
-          loss += e * e;
-          d = scale * e;
-        }
-        sZ[r * W + f] = d;
+      for (int q = t; q < rows * (W / 4); q += kBwdT)
+        reinterpret_cast<float4*>(sZ)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      __syncthreads();
+#pragma unroll 4
+      for (int q = t; q < rows * a.n_out; q += kBwdT) {
+        const int r = q / a.n_out, f = q - r * a.n_out;
+        const size_t o = (size_t)i0 * a.n_out + q;
+        const float e = a.yhat[o] - a.y[o];
+        loss += e * e;
+        sZ[r * W + f] = scale * e;
       }
     } else {
       // half a warp per node, four features a lane
@@ -602,10 +683,6 @@ int nfail(int code, const std::string& msg) {
     if (e_ != cudaSuccess) return nfail(BX_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-unsigned node_grid(int n) {
-  return (unsigned)std::max(1, std::min((n + 7) / 8, 152 * 8));
-}
-
 int ensure_cap(bx_gnn* h, int rows) {
   if (rows <= h->cap) return BX_OK;
   void* ptrs[] = {h->act, h->yhat, h->dHa, h->dHb, h->Ga, h->Gb};
@@ -651,25 +728,41 @@ int check_range(bx_gnn* h, int lo, int hi) {
   return ensure_cap(h, hi - lo);
 }
 
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                       Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 int forward(bx_gnn* h, int lo, int hi, const float* x, int n_in, int n_out) {
   using namespace bxn;
   const int n = hi - lo;
   cudaStream_t s = h->stream;
-  const long long tot = (long long)n * W;
-  k_pack_x<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(n, n_in, x, plane(h, P_X));
-  const unsigned g = node_grid(n);
-  const unsigned gt = (unsigned)((n + kTcRows - 1) / kTcRows);
-  k_fwd_tc<0><<<gt, kTcThreads, kTcSmem1, s>>>(n, plane(h, P_X), nullptr, h->wb, OFF_W0, 0, h->master, OFF_B0,
-                                              nullptr, plane(h, P_H0), nullptr, 0, h->err);
+  const unsigned g = (unsigned)((n + kTcRows - 1) / kTcRows);
+  FwdArgs a{};
+  a.n = n; a.wb = h->wb; a.master = h->master; a.err = h->err;
+  a.x = x; a.n_in = n_in; a.ptr = h->ptr; a.nbr = h->nbr; a.lo = lo;
+  a.in1 = plane(h, P_X); a.outH = plane(h, P_H0); a.off_w1 = OFF_W0; a.off_b = OFF_B0;
+  // (an ordinary launch: the weights may come from the kernel before it)
+  k_fwd_tc<0><<<g, kTcThreads, kTcSmem1, s>>>(a);
   for (int l = 0; l < NMP; ++l) {
     const int o = OFF_MP + l * MP_STRIDE;
-    k_agg<<<g, kThreads, 0, s>>>(n, lo, h->ptr, h->nbr, plane(h, P_H0 + l), plane(h, P_A1 + l));
-    k_fwd_tc<1><<<gt, kTcThreads, kTcSmem, s>>>(n, plane(h, P_H0 + l), plane(h, P_A1 + l), h->wb, o, o + W * W,
-                                                h->master, o + 2 * W * W, plane(h, P_R1 + l), plane(h, P_H1 + l),
-                                                nullptr, 0, h->err);
+    a.in1 = plane(h, P_H0 + l); a.in2 = plane(h, P_A1 + l); a.outR = plane(h, P_R1 + l); a.outH = plane(h, P_H1 + l);
+    a.off_w1 = o; a.off_w2 = o + W * W; a.off_b = o + 2 * W * W;
+    NX(launch_pdl(k_fwd_tc<1>, g, kTcThreads, kTcSmem, s, a));
   }
-  k_fwd_tc<2><<<gt, kTcThreads, kTcSmem1, s>>>(n, plane(h, P_H3), nullptr, h->wb, OFF_WD, 0, h->master, OFF_BD,
-                                              nullptr, nullptr, h->yhat, n_out, h->err);
+  a.in1 = plane(h, P_H3); a.outY = h->yhat; a.n_out = n_out; a.off_w1 = OFF_WD; a.off_b = OFF_BD;
+  NX(launch_pdl(k_fwd_tc<2>, g, kTcThreads, kTcSmem1, s, a));
   NX(cudaGetLastError());
   return BX_OK;
 }
@@ -696,20 +789,20 @@ int backward(bx_gnn* h, int lo, int hi, const float* y, int n_out, int* nb) {
   a.part = h->part; a.loss_part = h->loss_part;
   a.yhat = h->yhat; a.y = y; a.n_out = n_out;
   a.in1 = plane(h, P_H3); a.off_w1 = OFF_WD; a.off_part = OFF_WD; a.outH = h->dHa;
-  k_bwd<BWD_TOP><<<g, kBwdT, BwdShape<BWD_TOP>::smem, s>>>(a);
+  NX(launch_pdl(k_bwd<BWD_TOP>, g, kBwdT, BwdShape<BWD_TOP>::smem, s, a));
   float *dH = h->dHa, *dHn = h->dHb, *Gn = h->Ga, *Go = h->Gb;
   for (int l = NMP - 1; l >= 0; --l) {
     const int o = OFF_MP + l * MP_STRIDE;
     a.dH = dH; a.outH = dHn; a.outG = Gn;
     a.mask = plane(h, P_R1 + l); a.in1 = plane(h, P_H0 + l); a.in2 = plane(h, P_A1 + l);
     a.off_w1 = o; a.off_w2 = o + W * W; a.off_part = o;
-    k_bwd<BWD_MID><<<g, kBwdT, BwdShape<BWD_MID>::smem, s>>>(a);
+    NX(launch_pdl(k_bwd<BWD_MID>, g, kBwdT, BwdShape<BWD_MID>::smem, s, a));
     a.G = Gn;
     std::swap(dH, dHn);
     std::swap(Gn, Go);
   }
   a.dH = dH; a.mask = plane(h, P_H0); a.in1 = plane(h, P_X); a.off_part = OFF_W0;
-  k_bwd<BWD_ENC><<<g, kBwdT, BwdShape<BWD_ENC>::smem, s>>>(a);
+  NX(launch_pdl(k_bwd<BWD_ENC>, g, kBwdT, BwdShape<BWD_ENC>::smem, s, a));
   NX(cudaGetLastError());
   return BX_OK;
 }
