@@ -1276,11 +1276,12 @@ cudaError_t plain_dsa(bx_cluster* h) {
 //   else      64, halved while fewer than two tiles an SM would be left.
 // Halved further while a tile's shared memory would exceed kPlainSmemMax (cells with very
 // many membranes).
-// Measured us per step, cells per tile 8 / 16 / 32 / 64 (r: resident):
-// 2,878 cells 15.1 / 16.6 / 10.9r / 13.7r, 6,069 cells 25.6 / 17.2 / 20.9 /
-// 13.6r, 9,918 cells 37.5 / 28.3 / 21.2 / 30.7 (so at 64 the resident rule
-// stops where the tiles exceed the SMs), 20,432 cells 67.6 / 42.6 / 37.3 /
-// 33.0, 100,043 cells 293 / 176 / 121 / 108.
+// Measured us per step, cells per tile 32 / 64 (r: resident): 2,878 cells 10.3r
+// / 12.8r, 6,069 cells 16.2 / 12.8r, 9,918 cells 18.6 / 22.3 (so at 64 the
+// resident rule stops where the tiles exceed the SMs), 20,432 cells 31.7 /
+// 31.2, 100,043 cells 107 / 91.5; 8 / 16 cells (with expm1 instead of the
+// kernel's own, which the others are 5 to 10 % faster for): 15.1 / 16.6, 25.6 /
+// 17.2, 37.5 / 28.3, 67.6 / 42.6, 293 / 176.
 constexpr size_t kPlainSmemMax = 100 * 1024;
 int build_plain_layout(bx_cluster* h) {
   const int C = h->C, M = h->M, I = h->I, ncl = h->ncl;

@@ -16,8 +16,8 @@
 // about 400 FP64 thread instructions a cell against 1900.  Everything stays
 // FP64; only the order of the sums differs (one rounding per term).
 // Measured per step (k_cell_step with k_env_mix before): 100k cells 403 ->
-// 100 us, 20k cells 85 -> 33 us, 2900 cells 41 -> 11.1 us, 185 cells
-// 40 -> 10.3 us (12.5 with the one-lane-per-ion kernel that this one replaced).
+// 91 us, 20k cells 85 -> 31 us, 2900 cells 41 -> 10.3 us, 185 cells
+// 40 -> 9.7 us (12.5 with the one-lane-per-ion kernel that this one replaced).
 //
 // One CTA advances one tile: NC consecutive cells of one cluster, in phases
 // separated by bar.sync:
@@ -46,7 +46,7 @@
 //   pump, and phase C forms each membrane's flux from two factors per cell and
 //   ion, f sa = Dm sa (P - Q c_env): five FP64 instructions a membrane and ion.
 //   The last blocks of the launch compute the grid's Nernst-Planck flux.
-//   20,400 cells on 200 x 200: step 126 -> 58.8 us; 4975 on 100 x 100: 44 -> 28)
+//   20,400 cells on 200 x 200: step 126 -> 57 us; 4975 on 100 x 100: 44 -> 27)
 //   resident    many steps per cooperative launch, one tile per CTA, all of
 //               them co-resident: the state stays in shared memory, tiles
 //               exchange Vmem and concentrations through L2 and meet once a
@@ -137,6 +137,98 @@ template <> struct PlainIons<1> {
   __device__ static constexpr int n(const StepConst&) { return 6; }
   __device__ static constexpr int zc(const StepConst&, int i) { return i < 2 ? 1 : i == 3 ? 2 : -1; }
   static constexpr int NI = 6;
+};
+
+// expm1 and exp by table (P. T. P. Tang, "Table-driven implementation of the
+// exponential function in IEEE floating-point arithmetic", ACM TOMS 15, 1989;
+// "... of the expm1 function ...", ACM TOMS 18, 1992): x = (64 m + j) ln2 / 64
+// + r, |r| <= ln2 / 128, exp(x) = 2^m 2^(j/64) (1 + p), p = expm1(r) by its
+// Taylor series to r^6 (the next term is below 2^-57 of p).  A table entry is
+// 2^(j/64) rounded and the rest relative to it, so that
+// expm1(x) = T (p + rest) + (T - 1).  Fourteen FP64 instructions, where the pipe
+// spends 21.5 on expm1 and 16.8 on exp; outside |x| < 690 (and for NaN) those
+// are called.  Against 113-bit values over 2 M points of |x| < 690, 10, 0.7,
+// 0.02 and down to 1e-30: at most 1.12 ulp (expm1 1.14; below 0.02 alone 1.12
+// and 0.51) and 0.51 ulp (exp 0.87).  A step of 100,043 cells 100.1 -> 91.4 us,
+// of 185 cells 10.3 -> 9.7, voltage-gated 2,878 cells 18.2 -> 16.3.
+constexpr double kLn2Hi = 0x1.62e42fefa0000p-7, kLn2Lo = 0x1.cf79abc9e3b3ap-46;   // ln2 / 64: 36 bits (times 17-bit integers exact) and the rest
+constexpr double kInvLn2 = 0x1.71547652b82fep+6;                            // 64 / ln2
+__device__ const double2 kExpTab[64] = {
+    {0x1.0000000000000p+0, 0x0.0p+0}, {0x1.02c9a3e778061p+0, -0x1.160139cd8dc5dp-56},
+    {0x1.059b0d3158574p+0, 0x1.cd2523567f613p-55}, {0x1.0874518759bc8p+0, 0x1.0f74e61e6c861p-57},
+    {0x1.0b5586cf9890fp+0, 0x1.79aa65d837b6dp-54}, {0x1.0e3ec32d3d1a2p+0, 0x1.ebe3d702f9cd1p-60},
+    {0x1.11301d0125b51p+0, -0x1.556522a2fbd0ep-54}, {0x1.1429aaea92de0p+0, -0x1.1c923b9d5f416p-54},
+    {0x1.172b83c7d517bp+0, -0x1.01b15eaa59348p-55}, {0x1.1a35beb6fcb75p+0, 0x1.b898c3f1353bfp-55},
+    {0x1.1d4873168b9aap+0, 0x1.aecf73e3a2f60p-54}, {0x1.2063b88628cd6p+0, 0x1.a6f4144a6c38dp-55},
+    {0x1.2387a6e756238p+0, 0x1.68efde3a8a894p-54}, {0x1.26b4565e27cddp+0, 0x1.0472b981fe7f2p-55},
+    {0x1.29e9df51fdee1p+0, 0x1.2f7e16d09ab31p-55}, {0x1.2d285a6e4030bp+0, 0x1.b3782720c0ab4p-55},
+    {0x1.306fe0a31b715p+0, 0x1.34d754db0abb6p-55}, {0x1.33c08b26416ffp+0, 0x1.fdd395dd3f84ap-55},
+    {0x1.371a7373aa9cbp+0, -0x1.24aedcc4b5068p-54}, {0x1.3a7db34e59ff7p+0, -0x1.1d1e83e9436d2p-56},
+    {0x1.3dea64c123422p+0, 0x1.59f48a72a4c6dp-55}, {0x1.4160a21f72e2ap+0, -0x1.8a78f4817895bp-58},
+    {0x1.44e086061892dp+0, 0x1.363ed60c2ac11p-59}, {0x1.486a2b5c13cd0p+0, 0x1.ecce1daa10379p-57},
+    {0x1.4bfdad5362a27p+0, 0x1.690cebb7aafb0p-56}, {0x1.4f9b2769d2ca7p+0, -0x1.f94340071a38ep-55},
+    {0x1.5342b569d4f82p+0, -0x1.8dec6bd0f385fp-56}, {0x1.56f4736b527dap+0, 0x1.3350518fdd78ep-54},
+    {0x1.5ab07dd485429p+0, 0x1.063e1e21c5409p-54}, {0x1.5e76f15ad2148p+0, 0x1.432e62b64c035p-54},
+    {0x1.6247eb03a5585p+0, -0x1.c33c53bef4da8p-55}, {0x1.6623882552225p+0, -0x1.3cedd78565858p-54},
+    {0x1.6a09e667f3bcdp+0, -0x1.3b3efbf5e2228p-54}, {0x1.6dfb23c651a2fp+0, -0x1.367efb86da9eep-57},
+    {0x1.71f75e8ec5f74p+0, -0x1.81f647e5a3ecfp-56}, {0x1.75feb564267c9p+0, -0x1.619321e55e68ap-55},
+    {0x1.7a11473eb0187p+0, -0x1.b32dcb94da51dp-56}, {0x1.7e2f336cf4e62p+0, 0x1.5ebe1abd66c55p-57},
+    {0x1.82589994cce13p+0, -0x1.369b6f13b3734p-54}, {0x1.868d99b4492edp+0, -0x1.4d450d872576ep-54},
+    {0x1.8ace5422aa0dbp+0, 0x1.db72fc1f0eab4p-55}, {0x1.8f1ae99157736p+0, 0x1.bf68359f35f44p-56},
+    {0x1.93737b0cdc5e5p+0, -0x1.da9b88b6c1e29p-58}, {0x1.97d829fde4e50p+0, -0x1.2434322f4f9aap-54},
+    {0x1.9c49182a3f090p+0, 0x1.1affc2b91ce27p-56}, {0x1.a0c667b5de565p+0, -0x1.7c50422622263p-55},
+    {0x1.a5503b23e255dp+0, -0x1.1bbd1d3bcbb15p-54}, {0x1.a9e6b5579fdbfp+0, 0x1.469846e735ab3p-55},
+    {0x1.ae89f995ad3adp+0, 0x1.c1a7792cb3387p-55}, {0x1.b33a2b84f15fbp+0, -0x1.5c3d956dcaebap-58},
+    {0x1.b7f76f2fb5e47p+0, -0x1.8d6f438ad9334p-57}, {0x1.bcc1e904bc1d2p+0, 0x1.4ffd70a5fddcdp-56},
+    {0x1.c199bdd85529cp+0, 0x1.36eae30af0cb3p-56}, {0x1.c67f12e57d14bp+0, 0x1.4e08fd10959acp-55},
+    {0x1.cb720dcef9069p+0, 0x1.76b2c6c921968p-57}, {0x1.d072d4a07897cp+0, -0x1.fad5d3ffffa6fp-55},
+    {0x1.d5818dcfba487p+0, 0x1.4a385a63d07a7p-56}, {0x1.da9e603db3285p+0, 0x1.e5a50d5c192acp-55},
+    {0x1.dfc97337b9b5fp+0, -0x1.2d52107b43e1fp-55}, {0x1.e502ee78b3ff6p+0, 0x1.4b604603a88d3p-56},
+    {0x1.ea4afa2a490dap+0, -0x1.ff7128fd391f0p-55}, {0x1.efa1bee615a27p+0, 0x1.ec3bc41aa2008p-55},
+    {0x1.f50765b6e4540p+0, 0x1.a64a931d185eep-55}, {0x1.fa7c1819e90d8p+0, 0x1.7893b4d91cd9dp-56}};
+
+struct PlainExp {
+  double T, q;             // exp(x) = T (1 + q)
+};
+__device__ __forceinline__ bool plain_exp_ok(double x) { return (__double2hiint(x) & 0x7fffffff) < 0x40859000; }
+__device__ __forceinline__ PlainExp plain_exp_parts(const double2* tab, double x) {
+  const double t = fma(x, kInvLn2, 0x1.8p52);            // the integer 64 m + j in the low word
+  const int k = __double2loint(t);
+  const double n = t - 0x1.8p52;
+  const double2 e = tab[k & 63];
+  const double h = fma(n, -kLn2Hi, x);                   // r without its rounded part
+  const double r = fma(n, -kLn2Lo, h);
+  double c = fma(r, 1.0 / 720.0, 1.0 / 120.0);
+  c = fma(r, c, 1.0 / 24.0);
+  c = fma(r, c, 1.0 / 6.0);
+  c = fma(r, c, 0.5);
+  return PlainExp{__hiloint2double(__double2hiint(e.x) + ((k >> 6) << 20), __double2loint(e.x)),
+                  h + fma(r * r, c, fma(n, -kLn2Lo, e.y))};
+}
+__device__ __forceinline__ double plain_expm1(const double2* tab, double x) {
+  if (!plain_exp_ok(x)) return expm1(x);
+  const PlainExp p = plain_exp_parts(tab, x);
+  return fma(p.T, p.q, p.T - 1.0);
+}
+__device__ __forceinline__ double plain_exp(const double2* tab, double x) {
+  if (!plain_exp_ok(x)) return exp(x);
+  const PlainExp p = plain_exp_parts(tab, x);
+  return fma(p.T, p.q, p.T);
+}
+
+// What the fluxes through one membrane share (GhkShared with its quotients
+// over one reciprocal): e1 = exp(-a1), e2 = e1^2, kr = (a1 / d) / expm1(-a1),
+// kr2 = 2 kr / (2 + expm1(-a1)).
+struct PlainShared {
+  double e1, e2, kr, kr2;
+  __device__ __forceinline__ PlainShared(const double2* tab, double v_nonce, double F_RT, double inv_d) {
+    const double a1 = v_nonce * F_RT, em1 = plain_expm1(tab, -a1), u = 2.0 + em1;
+    const double g = a1 * inv_d * (1.0 / (em1 * u));
+    e1 = 1.0 + em1;
+    e2 = e1 * e1;
+    kr = g * u;
+    kr2 = g + g;
+  }
 };
 
 // The flux factor of charge code zc for a side A -> B: ghk_flux without Dc,
@@ -236,12 +328,14 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r, EnvNp en) {
   constexpr int T = kPlainT, NI = IS::NI;
   extern __shared__ double sm[];
   __shared__ int s_flag;
+  __shared__ double2 stab[64];            // kExpTab
   const int I = IS::n(k);
   const PlainSmem L(r.nc_max, r.ne_max, r.nm_max, I, GATED, ECM);
   double *sQ = sm + L.q, *sv = sm + L.v, *scm = sm + L.cm, *scc = sm + L.cc, *sx = sm + L.x, *s1 = sm + L.s1,
          *sk = sm + L.k, *senv = sm + L.env, *slvl = sm + L.lvl, *sga = sm + L.ga, *sgg = sm + L.gg, *sen = sm + L.en, *spm = sm + L.pm;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, b = blockIdx.x;
 
+  if (t < 64) stab[t] = kExpTab[t];
   // A streaming launch releases the next one as its CTAs exit: released at its
   // start, the next step's CTAs take whatever room the SMs have and the load
   // ends up uneven (20,400 cells 33.2 -> 41.5 us).
@@ -281,20 +375,18 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r, EnvNp en) {
       if (i < I) cB[i] = halo ? __ldcg(cin + (size_t)i * g.C + en.y) : scm[en.y * I + i];
     const double vgj = (vn + kNonce) - v1;        // update_gj, sim.py:2166
     const double vg1 = vgj + kNonce;
-    GhkShared<double> s;
-    s.init(vg1, k.F_RT);
-    const double kr = s.a1 * k.inv_gj_len * s.r, kr2 = 2.0 * kr * s.q2, e2 = s.e1 * s.e1;
+    const PlainShared s(stab, vg1, k.F_RT, k.inv_gj_len);
 #pragma unroll
     for (int i = 0; i < NI; ++i)
       if (i < I)
-        sQ[e * I + i] = plain_ghk(IS::zc(k, i), k.z[i], vg1, k.F_RT, k.inv_gj_len, kr, kr2, s.e1, e2,
+        sQ[e * I + i] = plain_ghk(IS::zc(k, i), k.z[i], vg1, k.F_RT, k.inv_gj_len, s.kr, s.kr2, s.e1, s.e2,
                                   scm[en.x * I + i], cB[i]);
     if (GATED) {
       // Gap_Junction.run (channels/gap_junction.py:52-81): one implicit Euler
       // update per ion with these two coefficients (phase G)
       const double V1 = 1.0e3 * fabs(vgj);
-      const double al = kGjLambda * exp(-kGjA1 * (V1 - k.gj_vth));
-      double be = kGjLambda * exp(kGjA2 * (V1 - k.gj_vth));
+      const double al = kGjLambda * plain_exp(stab, -kGjA1 * (V1 - k.gj_vth));
+      double be = kGjLambda * plain_exp(stab, kGjA2 * (V1 - k.gj_vth));
       be = be / (1.0 + 50.0 * be);
       sga[2 * e] = k.gj_dt_ms * (al + be * k.gj_min);
       sga[2 * e + 1] = 1.0 / (1.0 + al * k.gj_dt_ms + be * k.gj_dt_ms);
@@ -302,14 +394,12 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r, EnvNp en) {
   };
   // cell lc: the shared exponentials of its Vmem
   auto cell_exp = [&](int lc) {
-    GhkShared<double> s;
-    s.init(sv[lc] + kNonce, k.F_RT);
-    const double kr = s.a1 * k.inv_tm * s.r;
+    const PlainShared s(stab, sv[lc] + kNonce, k.F_RT, k.inv_tm);
     double* o = sk + lc * kPlainCell;
-    o[PK_K1] = kr;
+    o[PK_K1] = s.kr;
     o[PK_E1] = s.e1;
-    o[PK_K2] = 2.0 * kr * s.q2;
-    o[PK_E2] = s.e1 * s.e1;
+    o[PK_K2] = s.kr2;
+    o[PK_E2] = s.e2;
     o[PK_DTV] = k.dt * g.ivol[c0 + lc];
   };
   // cell lc: its pumps, times the cell's membrane area
