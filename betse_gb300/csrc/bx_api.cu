@@ -141,6 +141,7 @@ struct bx_cluster {
   // ---- environment
   double *d_cenv = nullptr, *d_phib = nullptr, *d_env_part = nullptr, *d_mem_flux_sa = nullptr,
          *d_pump = nullptr, *d_env_scale = nullptr;
+  float *d_Denv_f = nullptr, *d_Ex_f = nullptr, *d_Ey_f = nullptr, *d_fx_f = nullptr, *d_fy_f = nullptr;   // split form
   double *d_Denv = nullptr, *d_Ex = nullptr, *d_Ey = nullptr, *d_fx = nullptr, *d_fy = nullptr,
          *d_tmp = nullptr, *d_tmp2 = nullptr, *d_venv = nullptr, *d_rho_env = nullptr, *d_vsrc = nullptr;
   unsigned long long* d_status = nullptr;
@@ -231,6 +232,7 @@ void free_all(bx_cluster* h) {
       h->t_gw, h->t_dtv, h->t_dvc, h->t_rng,
       h->s_cenv_f, h->s_pump, h->s_part, h->s_phib, h->d_cenv, h->d_phib, h->d_env_part,
       h->d_mem_flux_sa, h->d_pump, h->d_env_scale, h->d_Denv, h->d_Ex, h->d_Ey, h->d_fx, h->d_fy,
+      h->d_Denv_f, h->d_Ex_f, h->d_Ey_f, h->d_fx_f, h->d_fy_f,
       h->d_tmp, h->d_tmp2, h->d_venv, h->d_rho_env, h->d_vsrc, h->d_status, h->o_fmem, h->o_fgj, h->o_rate,
       h->o_rho, h->o_Jn, h->o_Imem, h->o_Jcx, h->o_Jcy, h->o_Jc, h->o_vmave, h->o_dvm, h->o_Ecx,
       h->o_Ecy, h->o_Emc, h->o_Egjx, h->o_Egjy, h->o_gjopen, h->o_sigma, h->o_vmc, h->o_vm_mem,
@@ -378,6 +380,11 @@ bx::EnvConst make_env_const(const bx_cluster* h) {
     s += w[q + 4];
   }
   for (int q = 0; q < 9; ++q) e.gw[q] = w[q] / s;
+  e.inv_delta_f = (float)e.inv_delta;
+  e.inv_2delta_f = (float)e.inv_2delta;
+  e.dt_f = (float)e.dt;
+  for (int i = 0; i < h->I; ++i) e.np_alpha_f[i] = (float)e.np_alpha[i];
+  for (int q = 0; q < 9; ++q) e.gw_f[q] = (float)e.gw[q];
   return e;
 }
 
@@ -534,10 +541,12 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), unsigned grid, unsigned block, cu
 // The grid's Nernst-Planck flux in nthreads-wide blocks of the cell kernel's
 // launch (with the Ca-ATPase it has run before, and with sharpness < 1 the
 // split form's stencil is FP64: a launch of its own)
-bx::EnvNp env_np(const bx_cluster* h, int nthreads) {
+bx::EnvNp env_np(const bx_cluster* h, int nthreads, bool want_flux = true) {
   bx::EnvNp n{};
   if (!h->ecm) return n;
-  n.cenv = h->d_cenv; n.Denv = h->d_Denv; n.Ex = h->d_Ex; n.Ey = h->d_Ey; n.fx = h->d_fx; n.fy = h->d_fy;
+  n.cenv = h->d_cenv; n.Denv = h->d_Denv; n.Ex = h->d_Ex; n.Ey = h->d_Ey;
+  n.Denv_f = h->d_Denv_f; n.Ex_f = h->d_Ex_f; n.Ey_f = h->d_Ey_f; n.fx_f = h->d_fx_f; n.fy_f = h->d_fy_f;
+  if (want_flux) { n.fx = h->d_fx; n.fy = h->d_fy; }
   n.e = make_env_const(h);
   if (nthreads) n.nblk = (h->G * h->I + nthreads - 1) / nthreads;
   return n;
@@ -549,7 +558,7 @@ bool env_flux_in_cell_launch(const bx_cluster* h, bool out) {
 
 template <int TPB, bool OUT, bool PHIB, bool ECM>
 cudaError_t launch_split_t(bx_cluster* h, int parity, cudaStream_t s) {
-  const bx::EnvNp en = env_np(h, ECM && env_flux_in_cell_launch(h, OUT) ? TPB : 0);
+  const bx::EnvNp en = env_np(h, ECM && env_flux_in_cell_launch(h, OUT) ? TPB : 0, OUT);
   const unsigned grid = (unsigned)(h->nblk + en.nblk);
   if (is_betse_six_ions(h))
     return launch_pdl(bx::k_split_step<TPB, kRec, 1, OUT, PHIB, ECM>, grid, TPB, s, split_geom(h),
@@ -879,14 +888,17 @@ cudaError_t enqueue_env(bx_cluster* h, bool out, bool flux_done, cudaStream_t s)
                    nty = (unsigned)((h->ny + bx::kEnvTY - 1) / bx::kEnvTY);
     const double* phib = h->phib_nonzero ? h->d_phib : nullptr;
     double* rho = out ? h->d_rho_env : nullptr;
-    auto update = split ? bx::k_env_update_charge<float> : bx::k_env_update_charge<double>;
     auto fields = split ? bx::k_env_fields_tile<float> : bx::k_env_fields_tile<double>;
-    cudaError_t e = launch_pdl(update, gc, bx::kEnvUpT, s, h->d_cenv, (const double*)h->d_fx, (const double*)h->d_fy,
-                               (const int*)h->d_env_ptr, (const double*)h->d_mem_flux_sa,
-                               (const uint8_t*)h->d_touched, h->d_vsrc, rho, ec);
+    cudaError_t e =
+        split ? launch_pdl(bx::k_env_update_charge<float>, gc, bx::kEnvUpT, s, h->d_cenv, (const float*)h->d_fx_f,
+                           (const float*)h->d_fy_f, (const int*)h->d_env_ptr, (const double*)h->d_mem_flux_sa,
+                           (const uint8_t*)h->d_touched, h->d_vsrc, rho, ec)
+              : launch_pdl(bx::k_env_update_charge<double>, gc, bx::kEnvUpT, s, h->d_cenv, (const double*)h->d_fx,
+                           (const double*)h->d_fy, (const int*)h->d_env_ptr, (const double*)h->d_mem_flux_sa,
+                           (const uint8_t*)h->d_touched, h->d_vsrc, rho, ec);
     if (e != cudaSuccess) return e;
     e = launch_pdl(fields, ntx * nty, bx::kEnvTX * bx::kEnvTY, s, (const double*)h->d_vsrc, phib, h->d_venv, ec.screen,
-                   h->d_Ex, h->d_Ey, ec, (int)ntx);
+                   h->d_Ex, h->d_Ey, h->d_Ex_f, h->d_Ey_f, ec, (int)ntx);
     h->launches += 2;
     return e;
   }
@@ -894,7 +906,7 @@ cudaError_t enqueue_env(bx_cluster* h, bool out, bool flux_done, cudaStream_t s)
   h->launches += 1;
   bx::k_env_gauss_y<<<gg, kEnvTPB, 0, s>>>(h->d_vsrc, h->d_tmp, ec);
   bx::k_env_gauss_x<<<gg, kEnvTPB, 0, s>>>(h->d_tmp, h->phib_nonzero ? h->d_phib : nullptr, h->d_venv, ec);
-  bx::k_env_neg_grad<<<gg, kEnvTPB, 0, s>>>(h->d_venv, ec.screen, h->d_Ex, h->d_Ey, ec);
+  bx::k_env_neg_grad<<<gg, kEnvTPB, 0, s>>>(h->d_venv, ec.screen, h->d_Ex, h->d_Ey, h->d_Ex_f, h->d_Ey_f, ec);
   h->launches += 3;
   return cudaGetLastError();
 }
@@ -1646,6 +1658,11 @@ int create_impl(const bx_geom* gs, const bx_params* ps, int ncl, int precision, 
     ALLOC(h->d_Denv, (size_t)I * G);
     ALLOC(h->d_Ex, G); ALLOC(h->d_Ey, G);
     ALLOC(h->d_fx, (size_t)I * G); ALLOC(h->d_fy, (size_t)I * G);
+    if (h->mode == MODE_SPLIT) {
+      ALLOC(h->d_Denv_f, (size_t)I * G);
+      ALLOC(h->d_Ex_f, G); ALLOC(h->d_Ey_f, G);
+      ALLOC(h->d_fx_f, (size_t)I * G); ALLOC(h->d_fy_f, (size_t)I * G);
+    }
     ALLOC(h->d_tmp, G); ALLOC(h->d_tmp2, (size_t)I * G);
     ALLOC(h->d_venv, G); ALLOC(h->d_rho_env, G); ALLOC(h->d_vsrc, G);
     if (h->ca) ALLOC(h->d_cnew, (size_t)I * G);
@@ -1762,19 +1779,25 @@ int bx_set_membrane_diffusivity(bx_handle h, const double* Dm) {
   return BX_OK;
 }
 
+// FP32 copy of an FP64 array, rounded to nearest
+__global__ void k_round_to_float(const double* __restrict__ a, float* __restrict__ b, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) b[i] = __double2float_rn(a[i]);
+}
+
 int bx_set_env_diffusivity(bx_handle h, const double* D_env) {
   if (!h || !D_env) return fail(BX_EINVAL, "null argument");
   if (!h->ecm) return fail(BX_EINVAL, "environment diffusivity needs is_ecm");
   BX_CU(cudaStreamSynchronize(h->stream));
-  BX_CU(cudaMemcpy(h->d_Denv, D_env, (size_t)h->I * h->G * sizeof(double), cudaMemcpyHostToDevice));
+  BX_CU(cudaMemcpyAsync(h->d_Denv, D_env, (size_t)h->I * h->G * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  if (h->d_Denv_f) {
+    const int n = h->I * h->G;
+    k_round_to_float<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(h->d_Denv, h->d_Denv_f, n);
+    BX_CU(cudaGetLastError());
+  }
+  BX_CU(cudaStreamSynchronize(h->stream));
   h->have_denv = true;
   return BX_OK;
-}
-
-// FP32 copy of the well-mixed environment, rounded to nearest on the device
-__global__ void k_round_to_float(const double* __restrict__ a, float* __restrict__ b, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = __double2float_rn(a[i]);
 }
 
 // Device staging for state transfers: the caller's arrays in BETSE's layouts
@@ -1887,8 +1910,11 @@ int bx_state_upload(bx_handle h, const bx_state* s) {
     }
     if (!h->ecm) {
       k_round_to_float<<<(unsigned)((nenv + 255) / 256), 256, 0, st>>>(h->d_cenv, h->s_cenv_f, (int)nenv);
-      BX_CU(cudaGetLastError());
+    } else {
+      k_round_to_float<<<(unsigned)((h->G + 255) / 256), 256, 0, st>>>(h->d_Ex, h->d_Ex_f, h->G);
+      k_round_to_float<<<(unsigned)((h->G + 255) / 256), 256, 0, st>>>(h->d_Ey, h->d_Ey_f, h->G);
     }
+    BX_CU(cudaGetLastError());
     BX_CU(cudaStreamSynchronize(st));
   }
   h->have_state = true;

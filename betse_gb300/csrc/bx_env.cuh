@@ -17,22 +17,22 @@ __global__ void k_env_np_flux(EnvNp a) {
 
 // fd.diff with the reference's flipped one-sided edge signs (finitediff.py:1268-1303)
 template <typename R = double>
-__device__ __forceinline__ R ddx_neg(const double* f, const EnvConst& e, int i, int j) {
+__device__ __forceinline__ R ddx_neg(const R* f, const EnvConst& e, int i, int j) {
   // diff(-f, axis=0)
-  const double* r = f + i * e.nx;
-  const R inv_d = (R)e.inv_delta, inv_2d = (R)e.inv_2delta;
-  if (j == 0) return ((-(R)r[0]) - (-(R)r[1])) * inv_d;
-  if (j == e.nx - 1) return ((-(R)r[j - 1]) - (-(R)r[j])) * inv_d;
-  return -((-(R)r[j - 1]) - (-(R)r[j + 1])) * inv_2d;
+  const R* r = f + i * e.nx;
+  const R inv_d = env_inv_d<R>(e), inv_2d = env_inv_2d<R>(e);
+  if (j == 0) return ((-r[0]) - (-r[1])) * inv_d;
+  if (j == e.nx - 1) return ((-r[j - 1]) - (-r[j])) * inv_d;
+  return -((-r[j - 1]) - (-r[j + 1])) * inv_2d;
 }
 template <typename R = double>
-__device__ __forceinline__ R ddy_neg(const double* f, const EnvConst& e, int i, int j) {
+__device__ __forceinline__ R ddy_neg(const R* f, const EnvConst& e, int i, int j) {
   // diff(-f, axis=1)
   const int nx = e.nx;
-  const R inv_d = (R)e.inv_delta, inv_2d = (R)e.inv_2delta;
-  if (i == 0) return -((-(R)f[nx + j]) - (-(R)f[j])) * inv_d;
-  if (i == e.ny - 1) return -((-(R)f[i * nx + j]) - (-(R)f[(i - 1) * nx + j])) * inv_d;
-  return -((-(R)f[(i - 1) * nx + j]) - (-(R)f[(i + 1) * nx + j])) * inv_2d;
+  const R inv_d = env_inv_d<R>(e), inv_2d = env_inv_2d<R>(e);
+  if (i == 0) return -((-f[nx + j]) - (-f[j])) * inv_d;
+  if (i == e.ny - 1) return -((-f[i * nx + j]) - (-f[(i - 1) * nx + j])) * inv_d;
+  return -((-f[(i - 1) * nx + j]) - (-f[(i + 1) * nx + j])) * inv_2d;
 }
 
 // Environment charge of grid cell k from its new concentrations, for
@@ -167,8 +167,9 @@ __global__ void k_env_gauss_x(const double* __restrict__ tmp, const double* __re
 }
 
 // E = -gradient(scale * F)  (fd.gradient, finitediff.py:1236-1266)
-__global__ void k_env_neg_grad(const double* __restrict__ F, double scale, double* Ex, double* Ey,
-                               EnvConst e) {
+// (and its FP32 copy in the split form)
+__global__ void k_env_neg_grad(const double* __restrict__ F, double scale, double* Ex, double* Ey, float* Ex_f,
+                               float* Ey_f, EnvConst e) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= e.G) return;
   const int i = k / e.nx, j = k - i * e.nx;
@@ -183,6 +184,10 @@ __global__ void k_env_neg_grad(const double* __restrict__ F, double scale, doubl
   else gy = -(f(i - 1, j) - f(i + 1, j)) * e.inv_2delta;
   Ex[k] = -gx;
   Ey[k] = -gy;
+  if (Ex_f) {
+    Ex_f[k] = (float)-gx;
+    Ey_f[k] = (float)-gy;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -201,11 +206,12 @@ __global__ void k_env_neg_grad(const double* __restrict__ F, double scale, doubl
 // Bound by the FP64 pipe in both forms, so what counts is full lanes: with
 // eight lanes a cell and the charge summed by shuffles in all of them, 20 FP64
 // warp instructions per four cells took 24 us (split) and 22 us (FP64) on
-// 200 x 200 cells; as written 15.0 and 12.8 us (a launch by itself).
+// 200 x 200 cells; as written 11.5 and 13 us (a launch by itself; split with the
+// fluxes and constants converted from FP64 by every thread 15.0).
 constexpr int kEnvUpT = 192, kEnvUpCells = 32;
 template <typename R>
-__global__ void __launch_bounds__(kEnvUpT) k_env_update_charge(double* cenv, const double* __restrict__ fx,
-                                                               const double* __restrict__ fy,
+__global__ void __launch_bounds__(kEnvUpT) k_env_update_charge(double* cenv, const R* __restrict__ fx,
+                                                               const R* __restrict__ fy,
                                                                const int* __restrict__ env_ptr,
                                                                const double* __restrict__ mem_flux_sa,
                                                                const uint8_t* __restrict__ touched, double* vsrc,
@@ -216,10 +222,10 @@ __global__ void __launch_bounds__(kEnvUpT) k_env_update_charge(double* cenv, con
   for (int q = threadIdx.x; q < nk * e.I; q += kEnvUpT) {
     const int lk = q / e.I, ion = q - lk * e.I, k = k0 + lk;
     const int i = k / e.nx, j = k - i * e.nx;
-    const double* fxi = fx + (size_t)ion * e.G;
-    const double* fyi = fy + (size_t)ion * e.G;
+    const R* fxi = fx + (size_t)ion * e.G;
+    const R* fyi = fy + (size_t)ion * e.G;
     const R div = ddx_neg<R>(fxi, e, i, j) + ddy_neg<R>(fyi, e, i, j);
-    double c = cb_at(cenv, e, ion, i, j) + (double)(div * (R)e.dt);
+    double c = cb_at(cenv, e, ion, i, j) + (double)(div * env_dt<R>(e));
     // the membrane exchange, four rows at a time (their loads are
     // independent), added in list order; a cell's lanes read a row together
     double s = 0.0;
@@ -257,7 +263,8 @@ template <typename R>
 __global__ void __launch_bounds__(kEnvTX * kEnvTY) k_env_fields_tile(const double* __restrict__ vsrc,
                                                                      const double* __restrict__ phib,
                                                                      double* venv, double scale, double* Ex,
-                                                                     double* Ey, EnvConst e, int ntx) {
+                                                                     double* Ey, float* Ex_f, float* Ey_f, EnvConst e,
+                                                                     int ntx) {
   __shared__ R src[kEnvSY][kEnvSX];
   __shared__ R gy[kEnvVY][kEnvSX];
   __shared__ R v[kEnvVY][kEnvVX];
@@ -278,7 +285,7 @@ __global__ void __launch_bounds__(kEnvTX * kEnvTY) k_env_fields_tile(const doubl
     for (int w = -4; w <= 4; ++w) {
       const int ii = i + w;
       if (ii < 0 || ii >= e.ny) continue;
-      acc += (R)e.gw[w + 4] * src[a + 4 + w][b];
+      acc += env_gw<R>(e, w + 4) * src[a + 4 + w][b];
     }
     gy[a][b] = acc;
   }
@@ -290,7 +297,7 @@ __global__ void __launch_bounds__(kEnvTX * kEnvTY) k_env_fields_tile(const doubl
     for (int w = -4; w <= 4; ++w) {
       const int jj = j + w;
       if (jj < 0 || jj >= e.nx) continue;
-      acc += (R)e.gw[w + 4] * gy[a][b + 4 + w];
+      acc += env_gw<R>(e, w + 4) * gy[a][b + 4 + w];
     }
     const bool in = i >= 0 && i < e.ny && j >= 0 && j < e.nx;
     v[a][b] = in ? acc + (phib ? (R)phib[i * e.nx + j] : (R)0) : (R)0;
@@ -302,7 +309,7 @@ __global__ void __launch_bounds__(kEnvTX * kEnvTY) k_env_fields_tile(const doubl
   if (i >= e.ny || j >= e.nx) return;   // (an exited thread has released)
   const int k = i * e.nx + j;
   venv[k] = (double)v[a][b];
-  const R sc = (R)scale, inv_d = (R)e.inv_delta, inv_2d = (R)e.inv_2delta;
+  const R sc = (R)scale, inv_d = env_inv_d<R>(e), inv_2d = env_inv_2d<R>(e);
   auto f = [&](int da, int db) { return sc * v[a + da][b + db]; };
   R gx, gyy;
   if (j == 0) gx = (f(0, 1) - f(0, 0)) * inv_d;
@@ -313,6 +320,10 @@ __global__ void __launch_bounds__(kEnvTX * kEnvTY) k_env_fields_tile(const doubl
   else gyy = -(f(-1, 0) - f(1, 0)) * inv_2d;
   Ex[k] = (double)(-gx);
   Ey[k] = (double)(-gyy);
+  if (sizeof(R) == 4) {
+    Ex_f[k] = (float)-gx;
+    Ey_f[k] = (float)-gyy;
+  }
   grid_release();
 }
 
