@@ -196,8 +196,8 @@ __device__ __forceinline__ float warp_sum_down(float v) {
 // read before the dependency wait.  This kernel lets k_split_env start when it
 // ends, not while it runs: k_split_env in turn lets the next step's CTAs in,
 // and those would be placed among this step's, unevenly over the SMs (64
-// clusters of 200 to 5000 cells: 12.4 us a step then, 9.3 now; 8 clusters 8.5
-// and 7.4; 100,043 cells 13.7 and 12.0).
+// clusters of 200 to 5000 cells: 12.4 us a step, released at the end 9.3; 8
+// clusters 8.5 and 7.4; 100,043 cells 13.7 and 12.0).
 // ---------------------------------------------------------------------------
 // PF > 0: the first PF gap-junction entries of each cell (static data) are
 // loaded before the grid dependency wait, so after it each round of U
