@@ -16,7 +16,7 @@
 // about 400 FP64 thread instructions a cell against 1900.  Everything stays
 // FP64; only the order of the sums differs (one rounding per term).
 // Measured per step (k_cell_step with k_env_mix before): 100k cells 403 ->
-// 91 us, 20k cells 85 -> 31 us, 2900 cells 41 -> 10.3 us, 185 cells
+// 91 us, 20k cells 85 -> 30.4 us, 2900 cells 41 -> 10.1 us, 185 cells
 // 40 -> 9.7 us (12.5 with the one-lane-per-ion kernel that this one replaced).
 //
 // One CTA advances one tile: NC consecutive cells of one cluster, in phases
@@ -402,8 +402,8 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r, EnvNp en) {
     o[PK_E2] = s.e2;
     o[PK_DTV] = k.dt * g.ivol[c0 + lc];
   };
-  // cell lc: its pumps, times the cell's membrane area
-  auto cell_pump = [&](int lc) {
+  // cell lc: its pumps (bit 0 Na/K, bit 1 Ca), times the cell's membrane area
+  auto cell_pump = [&](int lc, int which) {
     double* o = sk + lc * kPlainCell;
     const double e1 = o[PK_E1];
     const double* cm = scm + lc * I;
@@ -418,11 +418,13 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r, EnvNp en) {
       return;
     }
     const double sa = g.sa[c0 + lc];
-    double fna = 0.0;
-    if (pcoef != 0.0)                             // Na/K-ATPase (sim.py:1196-1234)
-      fna = pump_fna<double>(k, pcoef, e1, cm[k.iNa], senv[k.iNa], cm[k.iK], senv[k.iK]);
-    o[PK_FNA] = fna * sa;
-    if (k.iCa >= 0)                               // ca_handler (sim.py:2126-2155)
+    if (which & 1) {
+      double fna = 0.0;
+      if (pcoef != 0.0)                           // Na/K-ATPase (sim.py:1196-1234)
+        fna = pump_fna<double>(k, pcoef, e1, cm[k.iNa], senv[k.iNa], cm[k.iK], senv[k.iK]);
+      o[PK_FNA] = fna * sa;
+    }
+    if ((which & 2) && k.iCa >= 0)                // ca_handler (sim.py:2126-2155)
       o[PK_FCA] = pump_fca<double>(k, e1, scc[lc * I + k.iCa], senv[k.iCa]) * sa;
   };
 
@@ -437,7 +439,7 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r, EnvNp en) {
         if (q < nl) entry(q, false);
       } else {
         cell_exp(q - nlp);
-        if (!RES || step == 0) cell_pump(q - nlp);
+        if (!RES || step == 0) cell_pump(q - nlp, 3);
       }
     }
     if (RES && step > 0) {
@@ -457,7 +459,17 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r, EnvNp en) {
         senv[t] = senv[t] - (a + c) * r.env_scale[cl];
       }
       __syncthreads();
-      for (int q = t; q < nc; q += T) cell_pump(q);
+      // (on the step's critical path: the two pumps in different warps; with
+      // both in one, a gated step of 2,878 cells took 16.3 us, 15.3 now)
+      if (k.iCa < 0) {
+        for (int q = t; q < nc; q += T) cell_pump(q, 1);
+      } else {
+        const int ncp = (nc + 31) & ~31;
+        for (int q = t; q < 2 * ncp; q += T) {
+          const int lc = q < ncp ? q : q - ncp;
+          if (lc < nc) cell_pump(lc, q < ncp ? 1 : 2);
+        }
+      }
       __syncthreads();
     }
     // ---- M: each membrane's environment and pump
@@ -574,10 +586,7 @@ k_plain_step(PlainGeom g, StepPtrs p, StepConst k, PlainRun r, EnvNp en) {
       double* w = vout; vout = const_cast<double*>(vin); vin = w;
       w = cout; cout = const_cast<double*>(cin); cin = w;
       __syncthreads();
-      if (t == 0) {
-        __threadfence();
-        res_arrive(r.ctl);
-      }
+      if (t == 0) res_arrive(r.ctl);         // a release: the CTA's writes, ordered by the bar.sync, with it
     }
   }
   if (bad) atomicAdd(&p.status[1], (unsigned long long)bad);
