@@ -43,6 +43,7 @@
 
 #include <cstdint>
 
+#include "bx_env_np.cuh"
 #include "bx_kernels.cuh"
 
 namespace bx {
@@ -367,6 +368,7 @@ __global__ void __launch_bounds__(kNetTPB) k_net_gj(NetArgs a) {
   double* sfa = sc + S * kNetCells;              // [S][tile_mems] -flux times area
   const int c0 = blockIdx.x * a.tile_cells, nc = min(a.tile_cells, a.C - c0);
   const int m0 = a.cell_ptr[c0], nm = a.cell_ptr[c0 + nc] - m0;
+  grid_wait();
   for (int q = t; q < S * kNetCells; q += kNetTPB) {
     const int k = q / kNetCells, lc = q - k * kNetCells;
     sc[q] = lc < nc ? a.c_mid[(size_t)k * a.C + c0 + lc] : 0.0;
