@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kTcThreads) k_fwd_tc(FwdArgs a) {
 // the transposed neighbour mean of the layer above's G.  Bound by the FMA pipe
 // (the gradients are FP32); with a warp per node, operands by shuffle and the
 // weight gradients in their own passes a training step of 30,858 nodes took
-// 653 us, 251 now (a middle layer 109 us before, 37 to 46 now).
+// 653 us, 245 now (a middle layer 109 us before, 36 to 44 now).
 constexpr int kBwdT = 256, kBwdRows = 64, kBwdPerSM = 2;
 
 struct BwdArgs {
@@ -463,51 +463,67 @@ __global__ void __launch_bounds__(kBwdT, kBwdPerSM) k_bwd(BwdArgs a) {
 #pragma unroll
       for (int it = 0; it < NIT; ++it) wt[it] = nb[it] >= 0 ? a.inv_deg[nb[it]] : 0.f;
 #pragma unroll
-      for (int it = 0; it < NIT; ++it) {
-        const int r = hw + it * NH;
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f), d = s;
-        uint2 mk = make_uint2(0u, 0u);
-        if (r < rows) {
-          d = reinterpret_cast<const float4*>(a.dH + (size_t)(i0 + r) * W)[l16];
-          mk = reinterpret_cast<const uint2*>(a.mask + (size_t)(i0 + r) * W)[l16];
+      for (int it0 = 0; it0 < NIT; it0 += 2) {               // two nodes a half-warp: eight rows in flight
+        float4 s[2], d[2];
+        uint2 mk[2];
+        int most = 0;
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          const int r = hw + (it0 + v) * NH;
+          s[v] = d[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+          mk[v] = make_uint2(0u, 0u);
+          if (r < rows) {
+            d[v] = reinterpret_cast<const float4*>(a.dH + (size_t)(i0 + r) * W)[l16];
+            mk[v] = reinterpret_cast<const uint2*>(a.mask + (size_t)(i0 + r) * W)[l16];
+          }
+          most = max(most, pb[it0 + v] - pa[it0 + v]);
         }
-        const int deg = pb[it] - pa[it];
-        const int most = max(deg, __shfl_xor_sync(FULL, deg, 16));
+        most = max(most, __shfl_xor_sync(FULL, most, 16));
         for (int p0 = 0; p0 < most; p0 += 16) {
           if (p0 > 0) {
-            const int p = pa[it] + p0 + l16;
-            nb[it] = p < pb[it] ? a.nbrT[p] : -1;
-            wt[it] = nb[it] >= 0 ? a.inv_deg[nb[it]] : 0.f;
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+              const int p = pa[it0 + v] + p0 + l16;
+              nb[it0 + v] = p < pb[it0 + v] ? a.nbrT[p] : -1;
+              wt[it0 + v] = nb[it0 + v] >= 0 ? a.inv_deg[nb[it0 + v]] : 0.f;
+            }
           }
           for (int k0 = 0; k0 < min(16, most - p0); k0 += 4) {
-            float4 g[4];
-            float w[4];
+            float4 g[2][4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int i = __shfl_sync(FULL, nb[it], k0 + u, 16);
-              w[u] = __shfl_sync(FULL, wt[it], k0 + u, 16);
-              g[u] = i >= 0 ? reinterpret_cast<const float4*>(a.G + (size_t)(i - a.lo) * W)[l16]
-                            : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+            for (int v = 0; v < 2; ++v)
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              s.x = fmaf(g[u].x, w[u], s.x);
-              s.y = fmaf(g[u].y, w[u], s.y);
-              s.z = fmaf(g[u].z, w[u], s.z);
-              s.w = fmaf(g[u].w, w[u], s.w);
-            }
+              for (int u = 0; u < 4; ++u) {
+                const int i = __shfl_sync(FULL, nb[it0 + v], k0 + u, 16);
+                g[v][u] = i >= 0 ? reinterpret_cast<const float4*>(a.G + (size_t)(i - a.lo) * W)[l16]
+                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+              }
+#pragma unroll
+            for (int v = 0; v < 2; ++v)
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                const float w = __shfl_sync(FULL, wt[it0 + v], k0 + u, 16);
+                s[v].x = fmaf(g[v][u].x, w, s[v].x);
+                s[v].y = fmaf(g[v][u].y, w, s[v].y);
+                s[v].z = fmaf(g[v][u].z, w, s[v].z);
+                s[v].w = fmaf(g[v][u].w, w, s[v].w);
+              }
           }
         }
-        if (r < rows) {
-          d.x += s.x; d.y += s.y; d.z += s.z; d.w += s.w;
-          if (MODE == BWD_MID) *reinterpret_cast<float4*>(sD + r * W + 4 * l16) = d;
-          const float2 m0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mk.x));
-          const float2 m1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mk.y));
-          if (!(m0.x > 0.f)) d.x = 0.f;
-          if (!(m0.y > 0.f)) d.y = 0.f;
-          if (!(m1.x > 0.f)) d.z = 0.f;
-          if (!(m1.y > 0.f)) d.w = 0.f;
-          *reinterpret_cast<float4*>(sZ + r * W + 4 * l16) = d;
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          const int r = hw + (it0 + v) * NH;
+          if (r >= rows) continue;
+          float4 x = d[v];
+          x.x += s[v].x; x.y += s[v].y; x.z += s[v].z; x.w += s[v].w;
+          if (MODE == BWD_MID) *reinterpret_cast<float4*>(sD + r * W + 4 * l16) = x;
+          const float2 m0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mk[v].x));
+          const float2 m1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mk[v].y));
+          if (!(m0.x > 0.f)) x.x = 0.f;
+          if (!(m0.y > 0.f)) x.y = 0.f;
+          if (!(m1.x > 0.f)) x.z = 0.f;
+          if (!(m1.y > 0.f)) x.w = 0.f;
+          *reinterpret_cast<float4*>(sZ + r * W + 4 * l16) = x;
         }
       }
     }
