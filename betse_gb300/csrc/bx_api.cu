@@ -1285,7 +1285,9 @@ cudaError_t plain_dsa(bx_cluster* h) {
 //   resident  the smallest power of two from 2 to 64 whose tiles fit one a SM
 //             (one cluster): small clusters spread over every SM and keep their
 //             state there;
-//   else      64, halved while fewer than two tiles an SM would be left.
+//   else      64, halved while fewer than two tiles an SM would be left, to 32
+//             at least, with extracellular spaces 16: smaller tiles evaluate
+//             too many junctions twice.
 // Halved further while a tile's shared memory would exceed kPlainSmemMax (cells with very
 // many membranes).
 // Measured us per step, cells per tile 32 / 64 (r: resident): 2,878 cells 10.3r
@@ -1293,7 +1295,12 @@ cudaError_t plain_dsa(bx_cluster* h) {
 // resident rule stops where the tiles exceed the SMs), 20,432 cells 31.7 /
 // 31.2, 100,043 cells 107 / 91.5; 8 / 16 cells (with expm1 instead of the
 // kernel's own, which the others are 5 to 10 % faster for): 15.1 / 16.6, 25.6 /
-// 17.2, 37.5 / 28.3, 67.6 / 42.6, 293 / 176.
+// 17.2, 37.5 / 28.3, 67.6 / 42.6, 293 / 176.  Batches, 4 / 8 / 16 / 32 / 64
+// cells: 8 clusters of 250 15.0 / 12.9 / 13.0 / 12.5 / 16.1, 4 of 1000 27.7 /
+// 16.7 / 14.9 / 13.4 / 16.2, 64 of 300 82 / 50 / 31 / 23.7 / 21.8.  Extracellular
+// spaces, 4 / 8 / 16 / 32 cells: 2,333 cells 35.3 / 24.9 / 24.6 / 24.7, 4,975
+// 48.5 / 36.5 / 27.1 / 28.5; 20,432 cells, 45 / 64 / 68 / 96: 56.4 / 57.1 / 59.5
+// / 58.2.
 constexpr size_t kPlainSmemMax = 100 * 1024;
 int build_plain_layout(bx_cluster* h) {
   const int C = h->C, M = h->M, I = h->I, ncl = h->ncl;
@@ -1313,7 +1320,8 @@ int build_plain_layout(bx_cluster* h) {
     for (nc = 2; tiles_of(nc) > h->sm_count;) nc <<= 1;
   } else {
     want_res = false;
-    while (nc > 4 && tiles_of(nc) < 2 * h->sm_count) nc >>= 1;
+    const int least = h->ecm ? 16 : 32;
+    while (nc > least && tiles_of(nc) < 2 * h->sm_count) nc >>= 1;
   }
   std::vector<int2> tile;
   std::vector<int4> ent;
