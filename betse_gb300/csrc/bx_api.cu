@@ -652,7 +652,11 @@ void drop_resident(bx_cluster* h) {
 }
 
 template <int ZP>
-void* resident_kernel() { return reinterpret_cast<void*>(bx::k_split_resident<ZP>); }
+const void* resident_kernel(int ntile_max) {
+  if (ntile_max <= 22) return reinterpret_cast<const void*>(bx::k_split_resident<ZP, 1, 704>);
+  if (ntile_max <= 32) return reinterpret_cast<const void*>(bx::k_split_resident<ZP, 1, 1024>);
+  return reinterpret_cast<const void*>(bx::k_split_resident<ZP, 2, 1024>);
+}
 
 // Partition of the tiles over one CTA per SM for k_split_resident, each CTA's
 // gap-junction entries re-indexed into its record table (own cells, then
@@ -726,7 +730,7 @@ int build_resident(bx_cluster* h) {
   if (L.total > (size_t)optin)
     return refuse("the cells of one SM need " + std::to_string(L.total) + " bytes of shared memory (" +
                   std::to_string(optin) + " available)");
-  const void* kern = six ? resident_kernel<1>() : resident_kernel<0>();
+  const void* kern = six ? resident_kernel<1>(ntile_max) : resident_kernel<0>(ntile_max);
   // the device's limit, so handles of different sizes never undercut each other
   BX_CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
   const int threads = 32 * std::min(ntile_max, 32);
@@ -768,7 +772,7 @@ cudaError_t launch_resident(bx_cluster* h, int parity, int n_steps, cudaStream_t
   bx::SplitPtrs sp = split_ptrs(h, parity);
   bx::SplitConst k = make_split_const(h);
   void* args[] = {&fg, &sp, &k, &ra, &n_steps};
-  const void* kern = is_betse_six_ions(h) ? resident_kernel<1>() : resident_kernel<0>();
+  const void* kern = is_betse_six_ions(h) ? resident_kernel<1>(h->r_ntile_max) : resident_kernel<0>(h->r_ntile_max);
   return cudaLaunchCooperativeKernel(kern, dim3(h->r_grid), dim3(h->r_threads), args, h->r_smem, s);
 }
 

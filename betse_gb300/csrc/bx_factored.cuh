@@ -394,12 +394,16 @@ __device__ __forceinline__ void res_gj_range(const SplitConst& k, int I, const f
   }
 }
 
-template <int ZP>
-__global__ void __launch_bounds__(1024, 1)
+// CPT: cells per thread (their carried sums in registers), MAXT: most threads.
+// One cell a thread and 704 threads (22 tiles a CTA: clusters to 107,000 cells)
+// leave 92 registers (72 are used) and one pass; with 64 registers and a second,
+// empty pass over the cells a step took, in us, at 100,043 / 62,000 / 31,000 /
+// 9,918 cells 8.25 / 7.91 / 6.24 / 6.75, now 8.12 / 7.63 / 5.85 / 6.46.
+template <int ZP, int CPT, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
 k_split_resident(FactGeom fg, SplitPtrs p, SplitConst k, ResArrays ra, int n_steps) {
   using IS = IonSet<ZP>;
   constexpr int NI = IS::NI;
-  constexpr int CPT = 2;                                         // cells per thread kept in registers (max)
   const int I = IS::n(k);
   extern __shared__ __align__(16) unsigned char res_smem[];
   const ResSmem L(ra.ntile_max, ra.nent_max, ra.nhalo_max, NI);
