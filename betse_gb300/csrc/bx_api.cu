@@ -870,8 +870,7 @@ cudaError_t enqueue_env(bx_cluster* h, bool out, bool flux_done, cudaStream_t s)
   const int gi = env_grid(h->G * h->I);   // one thread per (ion, grid cell)
   const bool split = h->mode == MODE_SPLIT && !(h->par.sharpness < 1.0);   // FP32 stencils around FP64 state
   if (!flux_done && !h->ca) {
-    if (split) bx::k_env_np_flux<float><<<gi, kEnvTPB, 0, s>>>(env_np(h, 0));
-    else bx::k_env_np_flux<double><<<gi, kEnvTPB, 0, s>>>(env_np(h, 0));
+    bx::k_env_np_flux<double><<<gi, kEnvTPB, 0, s>>>(env_np(h, 0));   // (the split form's FP32 flux: with its cells)
     h->launches += 1;
   }
   if (h->ca) {
