@@ -3206,13 +3206,16 @@ int bx_network_step(bx_network_handle n, int n_steps, int with_ions, int want_ou
   int left = n_steps;
   const int tail = want_outputs ? 1 : 0;
   if (with_ions) {
+    // The graph starts from parity 0 and, where its ion step is the factored
+    // one, from a Vmem that is one value per cell: single steps until both hold
+    // (at most two).
+    while (left - tail >= kGraphChunk && (h->parity != 0 || (plain_factored(h, false) && !h->vm_uniform))) {
+      cudaError_t e = net_enqueue_coupled(n, h->parity, false, s);
+      if (e != cudaSuccess) return fail(BX_ECUDA, std::string("network step launch: ") + cudaGetErrorString(e));
+      h->parity ^= 1;
+      --left;
+    }
     if (left - tail >= kGraphChunk) {
-      if (h->parity != 0 || !h->vm_uniform) {
-        cudaError_t e = net_enqueue_coupled(n, h->parity, false, s);
-        if (e != cudaSuccess) return fail(BX_ECUDA, std::string("network step launch: ") + cudaGetErrorString(e));
-        h->parity ^= 1;
-        --left;
-      }
       if (!n->graph || n->graph_gen != h->layout_gen) {
         if (n->graph) cudaGraphExecDestroy(n->graph);
         n->graph = nullptr;
