@@ -146,7 +146,7 @@ struct bx_cluster {
          *d_tmp = nullptr, *d_tmp2 = nullptr, *d_venv = nullptr, *d_rho_env = nullptr, *d_vsrc = nullptr;
   unsigned long long* d_status = nullptr;
   // ---- factored plain step (bx_plain.cuh)
-  bool vm_uniform = false;         // Vmem is one value per cell (the factored step needs it)
+  bool vm_uniform = false;         // Vmem is one value per cell (read only where plain_factored holds)
   int pl_pin = 0;                  // cells per tile pinned by a launch configuration (0: by size)
   int pl_nc = 0, pl_ntile = 0, pl_ne = 0, pl_nm = 0;   // cells per tile, tiles, largest tile
   bool pl_res = false;             // the resident form fits: one tile per co-resident CTA
@@ -1859,6 +1859,7 @@ int bx_set_boundary_potential(bx_handle h, const double* Phi_b) {
   if (nz != h->phib_nonzero) {
     h->graph_valid = false;
     ++h->layout_gen;
+    h->vm_uniform = false;   // steps under a potential leave a Vmem that differs within a cell
   }
   h->phib_nonzero = nz;
   return BX_OK;

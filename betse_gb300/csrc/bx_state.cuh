@@ -60,8 +60,9 @@ __global__ void __launch_bounds__(256) k_copy_list(CopyList l) {
 
 // The checks of bx_state_upload, one thread per membrane: flag[0] when
 // cc_at_mem differs from its cell's first membrane (a NaN differs too), flag[1]
-// when vm + Phi_b is not uniform over the cell (check_vm 1, the split form: to
-// rounding; 2, the plain form: bit for bit, which its factored step needs).
+// when Vmem is not uniform over the cell (check_vm 1, the split form: vm + Phi_b,
+// to rounding; 2, the plain form: vm itself, bit for bit, which its factored step
+// needs whatever the potential is by then).
 // Plain form (ccm): the first membrane's thread also lays down the cell's
 // membrane-side concentrations.
 __global__ void k_state_check(StateIO io, const double* __restrict__ vm, const double* __restrict__ cam,
@@ -77,10 +78,15 @@ __global__ void k_state_check(StateIO io, const double* __restrict__ vm, const d
   for (int i = 0; i < io.I; ++i)
     if (cam[(size_t)i * io.M + m] != cam[(size_t)i * io.M + f]) { atomicOr(&flag[0], 1); break; }
   if (check_vm) {
-    const double v0 = vm[f] + state_phib(io, f), v = vm[m] + state_phib(io, m);
+    bool differs;
+    if (check_vm == 2) {
+      differs = !(vm[m] == vm[f]);
+    } else {
+      const double v0 = vm[f] + state_phib(io, f), v = vm[m] + state_phib(io, m);
+      differs = fabs(v - v0) > 1e-12 * fabs(v0) + 1e-18;
+    }
     // (a polarizable state differs everywhere: no more atomics once it is known)
-    if (check_vm == 2 ? !(v == v0) : fabs(v - v0) > 1e-12 * fabs(v0) + 1e-18)
-      if (!*(volatile int*)&flag[1]) atomicOr(&flag[1], 1);
+    if (differs && !*(volatile int*)&flag[1]) atomicOr(&flag[1], 1);
   }
 }
 
