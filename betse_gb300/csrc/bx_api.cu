@@ -1727,6 +1727,18 @@ void bx_destroy(bx_handle h) {
   delete h;
 }
 
+// What was laid out for the kernels of one ion set (BETSE's six ions or any
+// others), after a change to the other.  was_six: before the change.
+static int follow_ion_set(bx_cluster* h, bool was_six) {
+  if (is_betse_six_ions(h) == was_six) return BX_OK;
+  BX_CU(cudaStreamSynchronize(h->stream));
+  if (h->mode != MODE_SPLIT) return h->pl_base ? build_plain_layout(h) : BX_OK;
+  drop_resident(h);                    // laid out again by the next step that runs it
+  BX_CU(build_geo_blob(h));
+  BX_CU(cudaStreamSynchronize(h->stream));
+  return BX_OK;
+}
+
 int bx_set_params(bx_handle h, const bx_params* p) {
   if (!h || !p) return fail(BX_EINVAL, "null argument");
   if (p->n_ions != h->I || (p->is_ecm != 0) != h->ecm || (p->v_sensitive_gj != 0) != h->vgj)
@@ -1737,11 +1749,13 @@ int bx_set_params(bx_handle h, const bx_params* p) {
   if ((p->cell_polarizability != 0.0) != h->polar)
     return fail(BX_EINVAL, "cell polarizability cannot be switched on or off after create");
   if (h->ncl > 1) return fail(BX_EINVAL, "use bx_batch_set_params for a batch");
+  const bool six = is_betse_six_ions(h);
   h->par = *p;
   h->cl_par[0] = *p;
   h->graph_valid = false;
   ++h->layout_gen;
-  return upload_param_arrays(h);
+  const int rc = upload_param_arrays(h);
+  return rc != BX_OK ? rc : follow_ion_set(h, six);
 }
 
 int bx_batch_set_params(bx_handle h, const bx_params* p) {
@@ -1752,11 +1766,13 @@ int bx_batch_set_params(bx_handle h, const bx_params* p) {
   if ((p[0].v_sensitive_gj != 0) != h->vgj || ca_pump_on(p[0]) != h->ca || (h->ca && p[0].iCa != h->par.iCa) ||
       (p[0].cell_polarizability != 0.0) != h->polar)
     return fail(BX_EINVAL, "v_sensitive_gj, the Ca-ATPase and cell polarizability cannot change after create");
+  const bool six = is_betse_six_ions(h);
   h->par = p[0];
   h->cl_par.assign(p, p + h->ncl);
   h->graph_valid = false;
   ++h->layout_gen;
-  return upload_param_arrays(h);
+  const int rc = upload_param_arrays(h);
+  return rc != BX_OK ? rc : follow_ion_set(h, six);
 }
 
 int bx_set_membrane_diffusivity(bx_handle h, const double* Dm) {
