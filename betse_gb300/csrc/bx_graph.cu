@@ -850,7 +850,6 @@ extern "C" int bx_graph_create(int n_levels, const bx_graph_level* levels, const
     if ((rc = check_csr(levels[l], expect, "level operator")) != BX_OK) return rc;
   }
   if ((rc = check_csr(*weighted, n, "weighted Laplacian")) != BX_OK) return rc;
-  if (n_levels > kMaxLevels) return gfail(BX_EINVAL, "bx_graph_create: more than 16 levels");
   auto* h = new bx_graph_solver();
   h->n = n;
   h->max_rhs = max_rhs;
@@ -864,6 +863,8 @@ extern "C" int bx_graph_create(int n_levels, const bx_graph_level* levels, const
   while (h->lc[0] < n_levels - 1 && levels[h->lc[0]].n > kDense) ++h->lc[0];
   h->lc[1] = h->lc[0];
   while (h->lc[0] > 0 && h->lc[1] < n_levels - 1 && (long long)levels[h->lc[1]].n * levels[h->lc[1]].n > 2LL * n) ++h->lc[1];
+  // (a 32-bit node count is down to 512 at level 11 at the latest, and to the root
+  // of twice itself sooner: whatever levels lie above, kMaxLevels holds those used)
   // shared memory of each level's staged rows: the largest row block's
   for (int gi = 0; gi < 4; ++gi)
     for (int l = 0; l < h->lc[1]; ++l) {
