@@ -2131,8 +2131,8 @@ int bx_status(bx_handle h, bx_step_status* st) {
 int bx_outputs_download(bx_handle h, bx_outputs* o) {
   if (!h || !o) return fail(BX_EINVAL, "null argument");
   if (!h->have_outputs) return fail(BX_ESTATE, "no step with want_outputs has run");
-  BX_CU(cudaStreamSynchronize(h->stream));
-  // the handle's stream does not wait for the default one, whose work may still use the destinations
+  // the handle's stream, which the copies run on, does not wait for the default one, whose work may still
+  // use the destinations
   BX_CU(cudaStreamSynchronize(cudaStreamLegacy));
   const size_t M = h->M, C = h->C, I = h->I, G = h->G;
   struct Pair {
