@@ -331,8 +331,9 @@ int bx_dense_op_set_columns(bx_dense_op_handle op, int col0, int ncols, const do
  * is Lw, vor_sa [n] the cell areas.  max_rhs bounds nrhs (the workspace is
  * 12 n max_rhs doubles).  Right-hand sides and results are DEVICE arrays
  * [n x nrhs] row-major; a solve stops when every column's residual is below
- * tol relative to its right-hand side (checked every 4 iterations) or after
- * max_iter iterations; iters and rel_res report the worst column. */
+ * 0.4 tol (bx_lap_gj_dense: tol) relative to its right-hand side, checked every
+ * 4 iterations, or after max_iter iterations; iters and rel_res report the worst
+ * column, which is converged at rel_res <= tol. */
 typedef struct bx_graph_level {
     int32_t n, nnz;
     const int32_t* row_ptr;
