@@ -179,6 +179,7 @@ SIGNATURES = {
                                    ct.POINTER(ct.c_int), ct.POINTER(ct.c_double), ct.c_void_p]),
     'bx_lap_gj_dense': (ct.c_int, [ct.c_void_p, ct.c_double, ct.c_int, ct.POINTER(ct.c_int),
                                    ct.POINTER(ct.c_double), ct.c_void_p, ct.POINTER(ct.c_void_p)]),
+    'bx_graph_barrier_check': (ct.c_int, [ct.c_void_p, ct.POINTER(ct.c_int)]),
     'bx_graph_destroy': (ct.c_int, [ct.c_void_p]),
     'bx_gnn_create': (ct.c_int, [ct.POINTER(ct.c_void_p)]),
     'bx_gnn_n_params': (ct.c_int, []),

@@ -820,7 +820,7 @@ cudaError_t launch_cell(bx_cluster* h, int parity, bool out, cudaStream_t s) {
 // n steps of the factored plain step: one per launch, or (resident) all in
 // one cooperative launch
 cudaError_t launch_plain(bx_cluster* h, int parity, int n, bool resident, cudaStream_t s,
-                         long long timeout_ns = kResTimeoutNs) {
+                         long long timeout_ns = kResTimeoutNs, int counter = 0) {
   bx::PlainGeom g{};
   g.C = h->C; g.M = h->M; g.ntile = h->pl_ntile;
   g.tile = h->pl_tile; g.tile_cl = h->pl_tile_cl; g.cl_tile = h->pl_cl_tile; g.cl_group = h->pl_cl_group;
@@ -839,7 +839,7 @@ cudaError_t launch_plain(bx_cluster* h, int parity, int n, bool resident, cudaSt
   const bx::StepConst k = make_step_const(h);
   const bx::StepPtrs p = step_ptrs(h, parity);
   const bool six = is_betse_six_ions(h);
-  return resident ? bx::launch_plain_resident(six, h->vgj, s, g, p, k, r)
+  return resident ? bx::launch_plain_resident(six, h->vgj, s, g, p, k, r, counter)
                   : bx::launch_plain_step(six, h->vgj, h->ecm, s, g, p, k, r, env_np(h, h->ecm ? bx::kPlainT : 0));
 }
 
@@ -2320,27 +2320,32 @@ int bx_set_launch_config(bx_handle h, int tpb, int kernel) {
 }
 
 // Failure detection of the resident kernel without a fault: one launch whose
-// grid barrier waits for one CTA more than the grid has, so every CTA's wait
-// runs out after timeout_ns; the kernel then raises its timeout flag and
-// returns, leaving the state as it was (the run never writes it back).
+// grid barrier waits for one CTA more than the grid has (plain form: counts
+// from too far below), so every CTA's wait runs out after timeout_ns; the kernel
+// then raises its timeout flag and returns, leaving the state as it was (the run
+// never writes it back).
 int bx_resident_barrier_check(bx_handle h, int64_t timeout_ns, int* timed_out) {
   if (!h || !timed_out || timeout_ns <= 0 || timeout_ns > kResTimeoutNs)
     return fail(BX_EINVAL, "timeout_ns must be in (0, 2e9]");
   if (!h->have_state || !h->have_dm) return fail(BX_ESTATE, "upload state and Dm first");
-  if (!fact_eligible(h, false)) return fail(BX_EINVAL, "the resident kernel does not cover this handle");
-  if (h->r_state == 0) {
+  // (gated junctions: the first step updates the open fractions in place)
+  const bool plain = h->pl_res && !h->vgj && h->vm_uniform && plain_factored(h, false);
+  if (!plain && !fact_eligible(h, false)) return fail(BX_EINVAL, "the resident kernel does not cover this handle");
+  if (!plain && h->r_state == 0) {
     const int rc = build_resident(h);
     if (rc != BX_OK) return rc;
   }
-  if (h->r_state != 1) return fail(BX_EINVAL, h->r_why);
-  cudaError_t e = launch_resident(h, h->parity, 2, h->stream, (long long)timeout_ns, 1u);
+  if (!plain && h->r_state != 1) return fail(BX_EINVAL, h->r_why);
+  cudaError_t e = plain ? launch_plain(h, h->parity, 2, true, h->stream, (long long)timeout_ns, bx::kStuckByte)
+                        : launch_resident(h, h->parity, 2, h->stream, (long long)timeout_ns, 1u);
   if (e != cudaSuccess) return fail(BX_ECUDA, cudaGetErrorString(e));
   h->launches++;
+  if (plain) h->last_step_outputs = false;   // the Vmem before the last step, which bx_env_fields reads, is gone
   BX_CU(cudaStreamSynchronize(h->stream));
-  unsigned ctl[2] = {0u, 0u};
-  BX_CU(cudaMemcpy(ctl, h->r_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
+  unsigned ctl[2] = {0u, 0u}, *dc = plain ? h->pl_ctl : h->r_ctl;
+  BX_CU(cudaMemcpy(ctl, dc, sizeof(ctl), cudaMemcpyDeviceToHost));
   *timed_out = ctl[1] ? 1 : 0;
-  BX_CU(cudaMemset(h->r_ctl, 0, sizeof(ctl)));
+  BX_CU(cudaMemset(dc, 0, sizeof(ctl)));
   return BX_OK;
 }
 

@@ -716,7 +716,7 @@ namespace {
 // X = L+ B for K columns (B and X device [n][K], distinct from the
 // workspace): enqueued; slot s of `out` gets the iterations and the residual.
 int solve_async(bx_graph_solver* h, const double* B, double* X, int K, double tol, int max_iter, int slot,
-                cudaStream_t s) {
+                cudaStream_t s, int counter = 0) {
   CgArgs a{};
   a.K = K;
   a.lc = h->lc[K > kNarrow];
@@ -737,6 +737,7 @@ int solve_async(bx_graph_solver* h, const double* B, double* X, int K, double to
   a.part = h->part; a.scal = h->scal; a.tol = tol; a.max_iter = max_iter; a.ctl = h->ctl + 2 * slot;
   a.out = h->out + 2 * slot;
   GCK(cudaMemsetAsync(a.ctl, 0, 2 * sizeof(unsigned), s));
+  if (counter) GCK(cudaMemsetAsync(a.ctl, counter, sizeof(unsigned), s));
   void* args[] = {&a};
   GCK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_graph_cg), dim3((unsigned)grid), dim3(kCgT), args,
                                   smem, s));
@@ -1018,6 +1019,16 @@ extern "C" int bx_lap_gj_dense(bx_graph_handle h, double tol, int max_iter, int*
   if (iters) *iters = worst_it;
   if (rel_res) *rel_res = worst_res;
   *out = op;
+  return BX_OK;
+}
+
+extern "C" int bx_graph_barrier_check(bx_graph_handle h, int* timed_out) {
+  if (!h || !timed_out) return gfail(BX_EINVAL, "null argument");
+  GCK(cudaMemset(h->T1, 0, (size_t)h->n * sizeof(double)));
+  const int rc = solve_async(h, h->T1, h->T2, 1, 1e-12, 4, 0, nullptr, 0x80);   // a count no wait can reach
+  if (rc != BX_OK) return rc;
+  *timed_out = solve_result(h, 1, nullptr, nullptr, nullptr) == BX_ECUDA ? 1 : 0;
+  GCK(cudaGetLastError());
   return BX_OK;
 }
 

@@ -713,8 +713,11 @@ static __global__ void k_plain_dsam(int M, int I, const double* __restrict__ Dm,
 // launchers (bx_step_f64_small.cu); ecm: with the grid's flux in en.nblk more blocks
 cudaError_t launch_plain_step(bool six, bool gated, bool ecm, cudaStream_t s, const PlainGeom& g, const StepPtrs& p,
                               const StepConst& k, const PlainRun& r, const EnvNp& en);
+// counter: the byte the barrier's counter is filled with (0; kStuckByte: a count
+// that no wait of this launch can reach)
+constexpr int kStuckByte = 0x80;
 cudaError_t launch_plain_resident(bool six, bool gated, cudaStream_t s, const PlainGeom& g, const StepPtrs& p,
-                                  const StepConst& k, const PlainRun& r);
+                                  const StepConst& k, const PlainRun& r, int counter);
 // CTAs of the resident form that fit one SM with this much shared memory (0: none)
 cudaError_t plain_resident_per_sm(bool six, bool gated, size_t smem, int* per_sm);
 // the shared-memory limit of both forms, raised once per device

@@ -40,8 +40,8 @@ cudaError_t launch_plain_step(bool six, bool gated, bool ecm, cudaStream_t s, co
 }
 
 cudaError_t launch_plain_resident(bool six, bool gated, cudaStream_t s, const PlainGeom& g, const StepPtrs& p,
-                                  const StepConst& k, const PlainRun& r) {
-  cudaError_t e = cudaMemsetAsync(r.ctl, 0, sizeof(unsigned), s);   // the barrier counter
+                                  const StepConst& k, const PlainRun& r, int counter) {
+  cudaError_t e = cudaMemsetAsync(r.ctl, counter, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
   EnvNp en{};
   void* args[] = {const_cast<PlainGeom*>(&g), const_cast<StepPtrs*>(&p), const_cast<StepConst*>(&k),

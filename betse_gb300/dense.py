@@ -287,6 +287,13 @@ class LapGJ:
     def apply(self, X, tol=1e-12, max_iter=1000, stream=None):
         return self._run(self.lib.bx_lap_gj_apply, X, tol, max_iter, stream)
 
+    def barrier_check(self):
+        """Run a solve with a grid barrier that cannot complete; True if its
+        bounded wait (two seconds) ran out and was reported."""
+        t = ct.c_int()
+        _lib.check(self.lib.bx_graph_barrier_check(self.h, ct.byref(t)), 'bx_graph_barrier_check')
+        return bool(t.value)
+
     def dense(self, tol=1e-10, max_iter=1000, stream=None):
         import torch
         st = torch.cuda.current_stream().cuda_stream if stream is None else int(stream)

@@ -246,7 +246,8 @@ class ClusterEngine:
         return tpb.value, kind.value
 
     def resident_barrier_check(self, timeout_s=0.05):
-        """Run the resident kernel once with a grid barrier that cannot
+        """Run the resident kernel (the split form's, or the plain form's
+        without voltage-gated junctions) once with a grid barrier that cannot
         complete; True if its bounded wait ran out and was reported (the
         state is unchanged)."""
         t = ct.c_int()

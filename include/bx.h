@@ -356,6 +356,10 @@ int bx_lap_gj_apply(bx_graph_handle h, const double* X, double* Y, int nrhs, dou
  * matrix is formed */
 int bx_lap_gj_dense(bx_graph_handle h, double tol, int max_iter, int* iters, double* rel_res,
                     void* stream, bx_dense_op_handle* out);
+/* Failure detection of the solver, tested without a fault: a solve whose grid
+ * barrier can never complete, so that its bounded wait (two seconds) runs out.
+ * *timed_out = 1 if that was reported; the handle solves on afterwards. */
+int bx_graph_barrier_check(bx_graph_handle h, int* timed_out);
 int bx_graph_destroy(bx_graph_handle h);
 
 /* Warm-start graph network (no reference counterpart: BETSE's init phase
@@ -462,10 +466,11 @@ int bx_get_launch_config(bx_handle h, int* tpb, int* kernel);
 /* Whether the resident kernel fits this handle (*fits), and its grid, CTA
  * size and shared memory per CTA.  BX_EINVAL (with the reason) if not. */
 int bx_resident_info(bx_handle h, int* fits, int* grid, int* threads, int64_t* smem_bytes);
-/* Failure detection of the resident kernel, tested without a fault: one
- * launch whose grid barrier can never complete, so every CTA's bounded wait
- * runs out after timeout_ns (at most 2e9).  *timed_out = 1 if the kernel
- * reported the timeout; the state is left as it was. */
+/* Failure detection of the resident kernels (the split form's, and the plain
+ * form's without voltage-gated junctions), tested without a fault: one launch
+ * whose grid barrier can never complete, so every CTA's bounded wait runs out
+ * after timeout_ns (at most 2e9).  *timed_out = 1 if the kernel reported the
+ * timeout; the state is left as it was. */
 int bx_resident_barrier_check(bx_handle h, int64_t timeout_ns, int* timed_out);
 
 /* Autotuner: times n_steps steps (run as bx_step runs them) for each
