@@ -268,7 +268,7 @@ struct CgCta {
     __syncthreads();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, q = w >> 2;
     if (q < nq) {
-      const int u = threadIdx.x & 127;           // 128 threads a quantity, 8 values each
+      const int u = threadIdx.x & 127;           // 128 threads a quantity, kCgT / 128 values each
       double s = 0.0;
 #pragma unroll
       for (int j = 0; j < kCgT / 128; ++j) s += red[q * kCgT + j * 128 + u];
@@ -788,6 +788,18 @@ int lap_gj(bx_graph_solver* h, const double* X, double* Y, int K, double tol, in
   return solve_result(h, 2, iters, rel_res, s);
 }
 
+// One k_graph_pinv and its result; counter: the byte that the barrier's count starts from
+int run_pinv(PinvArgs a, int grid, int counter = 0) {
+  unsigned timed_out = 0;
+  void* args[] = {&a};
+  GCK(cudaMemset(a.ctl, 0, 2 * sizeof(unsigned)));
+  if (counter) GCK(cudaMemset(a.ctl, counter, sizeof(unsigned)));
+  GCK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_graph_pinv), dim3((unsigned)std::min(a.n, grid)),
+                                  dim3(512), args, 0, nullptr));
+  GCK(cudaMemcpy(&timed_out, a.ctl + 1, sizeof(unsigned), cudaMemcpyDeviceToHost));
+  return timed_out ? gfail(BX_ECUDA, "dense level: the grid barrier timed out") : BX_OK;
+}
+
 // The dense pseudo-inverse of a level's graph Laplacian, on the GPU.
 int build_pinv(bx_graph_solver* h, Level& L, const bx_graph_level& src) {
   const int n = src.n;
@@ -814,18 +826,13 @@ int build_pinv(bx_graph_solver* h, Level& L, const bx_graph_level& src) {
       cudaMalloc(&isz, (size_t)n * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&cmp, (size_t)n * sizeof(int)) != cudaSuccess)
     rc = gfail(BX_ENOMEM, "bx_graph_create: dense level");
-  unsigned timed_out = 0;
   if (rc == BX_OK) {
-    PinvArgs a{n, L.dense, piv, cmp, isz, h->ctl};
-    void* args[] = {&a};
     if (cudaMemcpy(L.dense, A.data(), A.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(isz, inv_size.data(), (size_t)n * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(cmp, comp.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemset(h->ctl, 0, 2 * sizeof(unsigned)) != cudaSuccess ||
-        cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_graph_pinv), dim3((unsigned)std::min(n, h->grid)),
-                                    dim3(512), args, 0, nullptr) != cudaSuccess ||
-        cudaMemcpy(&timed_out, h->ctl + 1, sizeof(unsigned), cudaMemcpyDeviceToHost) != cudaSuccess || timed_out)
+        cudaMemcpy(cmp, comp.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
       rc = gfail(BX_ECUDA, "bx_graph_create: dense level");
+    else
+      rc = run_pinv(PinvArgs{n, L.dense, piv, cmp, isz, h->ctl}, h->grid);
   }
   cudaFree(piv);
   cudaFree(isz);
@@ -1024,10 +1031,16 @@ extern "C" int bx_lap_gj_dense(bx_graph_handle h, double tol, int max_iter, int*
 
 extern "C" int bx_graph_barrier_check(bx_graph_handle h, int* timed_out) {
   if (!h || !timed_out) return gfail(BX_EINVAL, "null argument");
+  constexpr int kStuck = 0x80;             // a count that no wait can reach
   GCK(cudaMemset(h->T1, 0, (size_t)h->n * sizeof(double)));
-  const int rc = solve_async(h, h->T1, h->T2, 1, 1e-12, 4, 0, nullptr, 0x80);   // a count no wait can reach
+  int rc = solve_async(h, h->T1, h->T2, 1, 1e-12, 4, 0, nullptr, kStuck);
   if (rc != BX_OK) return rc;
   *timed_out = solve_result(h, 1, nullptr, nullptr, nullptr) == BX_ECUDA ? 1 : 0;
+  // the dense level's inverse: one node, in the workspace (each array two doubles at least)
+  GCK(cudaMemset(h->Q, 0, sizeof(double)));
+  GCK(cudaMemset(h->P0, 0, sizeof(int)));
+  rc = run_pinv(PinvArgs{1, h->T1, h->T2, reinterpret_cast<const int*>(h->P0), h->Q, h->ctl}, 1, kStuck);
+  *timed_out = *timed_out && rc == BX_ECUDA ? 1 : 0;
   GCK(cudaGetLastError());
   return BX_OK;
 }

@@ -288,8 +288,9 @@ class LapGJ:
         return self._run(self.lib.bx_lap_gj_apply, X, tol, max_iter, stream)
 
     def barrier_check(self):
-        """Run a solve with a grid barrier that cannot complete; True if its
-        bounded wait (two seconds) ran out and was reported."""
+        """Run a solve and a dense level's inverse with grid barriers that
+        cannot complete; True if both bounded waits (two seconds each) ran out
+        and were reported."""
         t = ct.c_int()
         _lib.check(self.lib.bx_graph_barrier_check(self.h, ct.byref(t)), 'bx_graph_barrier_check')
         return bool(t.value)

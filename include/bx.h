@@ -356,9 +356,10 @@ int bx_lap_gj_apply(bx_graph_handle h, const double* X, double* Y, int nrhs, dou
  * matrix is formed */
 int bx_lap_gj_dense(bx_graph_handle h, double tol, int max_iter, int* iters, double* rel_res,
                     void* stream, bx_dense_op_handle* out);
-/* Failure detection of the solver, tested without a fault: a solve whose grid
- * barrier can never complete, so that its bounded wait (two seconds) runs out.
- * *timed_out = 1 if that was reported; the handle solves on afterwards. */
+/* Failure detection of the solver, tested without a fault: a solve, and a
+ * dense level's inverse as bx_graph_create forms it, whose grid barriers can
+ * never complete, so that their bounded waits (two seconds each) run out.
+ * *timed_out = 1 if both were reported; the handle solves on afterwards. */
 int bx_graph_barrier_check(bx_graph_handle h, int* timed_out);
 int bx_graph_destroy(bx_graph_handle h);
 
