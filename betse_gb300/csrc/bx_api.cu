@@ -853,8 +853,7 @@ cudaError_t enqueue_env_pre(bx_cluster* h, cudaStream_t s) {
   bx::EnvConst ec = make_env_const(h);
   const int gi = env_grid(h->G * h->I);
   bx::k_env_np_flux<double><<<gi, kEnvTPB, 0, s>>>(env_np(h, 0));
-  bx::k_env_update<false><<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_fx, h->d_fy, h->d_env_ptr,
-                                                h->d_mem_flux_sa, ec);
+  bx::k_env_update<<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_fx, h->d_fy, ec);
   h->launches += 2;
   if (h->par.sharpness < 1.0) {
     bx::k_env_integrate_scatter<false><<<gi, kEnvTPB, 0, s>>>(h->d_cnew, h->d_tmp2, h->d_env_ptr, h->d_mem_flux_sa, ec);
@@ -878,8 +877,7 @@ cudaError_t enqueue_env(bx_cluster* h, bool out, bool flux_done, cudaStream_t s)
     bx::k_env_scatter_add<<<gi, kEnvTPB, 0, s>>>(h->d_cenv, src, h->d_env_ptr, h->d_mem_flux_sa, ec);
     h->launches += 1;
   } else if (h->par.sharpness < 1.0) {
-    bx::k_env_update<false><<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_fx, h->d_fy, h->d_env_ptr,
-                                                  h->d_mem_flux_sa, ec);
+    bx::k_env_update<<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_fx, h->d_fy, ec);
     bx::k_env_integrate_scatter<true><<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_env_ptr, h->d_mem_flux_sa, ec);
     h->launches += 2;
   } else {

@@ -46,33 +46,18 @@ __device__ __forceinline__ void env_charge_out(int k, double rho, const uint8_t*
   if (rho_env) rho_env[k] = rho;
 }
 
-// c <- cb + div(-f) dt  [+ membrane exchange if FUSE_SCATTER]
-// (update_ecm sim.py:2247-2254, then update_Co's ECM term sim_toolbox.py:1189-1195
-//  with div_env = M_divmap_mem2ecm @ (-flux) / (cell_height delta^2), :1229-1232).
-// One thread per (ion, grid cell); while the new concentration is written in
-// place, the kernel reads only fluxes and its own cell's value.
-template <bool FUSE_SCATTER>
-__global__ void k_env_update(double* cenv, double* tmp, const double* __restrict__ fx,
-                             const double* __restrict__ fy, const int* __restrict__ env_ptr,
-                             const double* __restrict__ mem_flux_sa, EnvConst e) {
+// tmp = cb + div(-f) dt (update_ecm sim.py:2247-2254), where the membrane
+// exchange is a pass of its own.  One thread per (ion, grid cell).
+__global__ void k_env_update(const double* __restrict__ cenv, double* tmp, const double* __restrict__ fx,
+                             const double* __restrict__ fy, EnvConst e) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= e.I * e.G) return;
   const int ion = t / e.G, k = t - ion * e.G;
   const int i = k / e.nx, j = k - i * e.nx;
-  {
-    const double* fxi = fx + (size_t)ion * e.G;
-    const double* fyi = fy + (size_t)ion * e.G;
-    const double div = ddx_neg(fxi, e, i, j) + ddy_neg(fyi, e, i, j);
-    double c = cb_at(cenv, e, ion, i, j) + div * e.dt;
-    if (FUSE_SCATTER) {
-      double s = 0.0;
-      for (int q = env_ptr[k]; q < env_ptr[k + 1]; ++q) s += -mem_flux_sa[(size_t)q * kMfs + ion];
-      c = c + (s * e.inv_h_d2) * e.dt;
-      cenv[(size_t)ion * e.G + k] = c;
-    } else {
-      tmp[(size_t)ion * e.G + k] = c;
-    }
-  }
+  const double* fxi = fx + (size_t)ion * e.G;
+  const double* fyi = fy + (size_t)ion * e.G;
+  const double div = ddx_neg(fxi, e, i, j) + ddy_neg(fyi, e, i, j);
+  tmp[(size_t)ion * e.G + k] = cb_at(cenv, e, ion, i, j) + div * e.dt;
 }
 
 // The environment charge of each grid cell from its final concentrations
