@@ -513,18 +513,18 @@ def fp64_roofline(kernel_ms, n_mems, peak, kernel, workload):
     path = os.path.join(ROOT, 'profiles', 'fp64_counts.json')
     counts = json.load(open(path)).get('kernels', {}).get(workload, {}) if os.path.exists(path) else {}
     entry, counted = counts.get(kernel), kernel
-    family = kernel.split(' (')[0]
-    if entry is None and family in ('k_cell_step<double>', 'k_plain_step'):
+    if entry is None and kernel.startswith('k_cell_step<double>'):
         # another tile size of the same kernel: the same code per membrane
-        # slot (or junction and cell), so its count per membrane stands in
+        # slot, so its count per membrane stands in.  (k_plain_step evaluates
+        # a junction across a tile edge in both tiles: the size itself only)
         for name, e in counts.items():
-            if name.startswith(family):
+            if name.startswith('k_cell_step<double>'):
                 entry, counted = e, name
                 break
     if entry is None:
         r.update(achieved=None, frac=None, note='no FP64 instruction count captured for this kernel')
         return r
-    per_mem = entry['fp64_warp_inst_per_launch'] / entry['membranes']
+    per_mem = entry['fp64_warp_inst_per_launch'] / entry.get('steps_per_launch', 1) / entry['membranes']
     inst = per_mem * n_mems
     a = inst / (kernel_ms / 1e3) / 1e9
     r.update(achieved=a, frac=a / r['peak'], fp64_warp_inst_per_launch=int(inst),
@@ -565,6 +565,10 @@ def config_plain250(wl, stream, flush, cpu=True):
         launch = e.launch_config()
         ms = timed_run_ms(e, T, stream, flush)
         e.upload(**st)
+        l0 = e.launch_count()
+        e.step(T, stream=stream.cuda_stream)
+        launches = e.launch_count() - l0
+        e.upload(**st)
         kms = e.time_cell_kernel(200)
         kb = e.cell_kernel_bytes()
     out = {'workload': w['desc'], 'cells': g.n_cells, 'membranes': g.n_mems, 'time_steps_per_run': T,
@@ -573,7 +577,7 @@ def config_plain250(wl, stream, flush, cpu=True):
                                       note='a 1.4k-membrane cluster is bound by the dependent FP64 instruction '
                                            'chain of a step and the grid barrier between steps, not by HBM',
                                       step=step_bytes('fp64', g.n_cells, g.n_mems)),
-           'kernel_launches_per_run': 1,                 # the resident form: every step in one launch
+           'kernel_launches_per_run': launches,
            'autotuned_launch': {'cta_slots': launch[0], 'kernel': 'k_plain_step'},
            'autotune_table': table}
     out['roofline_fp64'] = fp64_roofline(kms, g.n_mems, fp64_peak(stream), f'k_plain_step ({launch[0] // 4} cells)',
