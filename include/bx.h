@@ -443,8 +443,8 @@ int bx_step_fp64_noalloc(const bx_geom* g, const bx_params* p, const double* Dm,
  * grouped into tiles) and the kernel.  The plain form runs the factored step
  * (transmembrane flux and pumps once per cell, gap-junction flux once per
  * junction; many steps in one cooperative launch where the tiles are
- * co-resident) and, with outputs, Phi_b, extracellular spaces or
- * polarizability, the per-membrane kernel.  For the split form:
+ * co-resident); with outputs, Phi_b, polarizability, or extracellular spaces
+ * together with the Ca-ATPase, the per-membrane kernel.  For the split form:
  *   0  tile kernel (one tile per CTA, one launch per step; every variant)
  *   1  persistent pipelined tile kernel
  *   2  factored kernel: one thread per cell; the transmembrane flux and the
@@ -456,7 +456,8 @@ int bx_step_fp64_noalloc(const bx_geom* g, const bx_params* p, const double* Dm,
  *   4  factored kernel, persistent and software-pipelined: each warp stages
  *      its next tiles' cell data, gap-junction entries and partner records
  *      in shared memory (cp.async) while it computes (results as kernel 2)
- *   5  (plain form) as 0
+ *   5  (plain form) as 0; refused with polarizability, extracellular spaces,
+ *      voltage-gated gap junctions or the Ca-ATPase
  * Bits 8-15 of kernel, when nonzero, pick the factored kernel's variant (the
  * third column of bx_autotune_table: 2, 4, 12, 13, 14 or 16).
  * Kernels 1-4 need no extracellular spaces, no voltage-gated gap junctions
