@@ -1030,6 +1030,7 @@ int upload_param_arrays(bx_cluster* h) {
     const int Mc = h->cl_mem[c + 1] - h->cl_mem[c];
     escale[c] = p.dt / (p.vol_env * (double)Mc);
   }
+  BX_CU(cudaStreamSynchronize(h->stream));   // steps in flight read these arrays
   BX_CU(h2d(h->d_pump, pump.data(), h->ncl));
   BX_CU(h2d(h->d_env_scale, escale.data(), h->ncl));
   if (h->mode == MODE_SPLIT) {
@@ -1729,7 +1730,6 @@ void bx_destroy(bx_handle h) {
 // others), after a change to the other.  was_six: before the change.
 static int follow_ion_set(bx_cluster* h, bool was_six) {
   if (is_betse_six_ions(h) == was_six) return BX_OK;
-  BX_CU(cudaStreamSynchronize(h->stream));
   if (h->mode != MODE_SPLIT) return h->pl_base ? build_plain_layout(h) : BX_OK;
   drop_resident(h);                    // laid out again by the next step that runs it
   BX_CU(build_geo_blob(h));
