@@ -651,10 +651,11 @@ void drop_resident(bx_cluster* h) {
   h->r_state = 0;
 }
 
+// The instance for a CTA's tiles: measured beside the kernel.
 template <int ZP>
 const void* resident_kernel(int ntile_max) {
   if (ntile_max <= 22) return reinterpret_cast<const void*>(bx::k_split_resident<ZP, 1, 704>);
-  if (ntile_max <= 32) return reinterpret_cast<const void*>(bx::k_split_resident<ZP, 1, 1024>);
+  if (ntile_max <= 28) return reinterpret_cast<const void*>(bx::k_split_resident<ZP, 1, 896>);
   return reinterpret_cast<const void*>(bx::k_split_resident<ZP, 2, 1024>);
 }
 

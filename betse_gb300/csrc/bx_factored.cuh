@@ -395,10 +395,16 @@ __device__ __forceinline__ void res_gj_range(const SplitConst& k, int I, const f
 }
 
 // CPT: cells per thread (their carried sums in registers), MAXT: most threads.
-// One cell a thread and 704 threads (22 tiles a CTA: clusters to 107,000 cells)
-// leave 92 registers (72 are used) and one pass; with 64 registers and a second,
-// empty pass over the cells a step took, in us, at 100,043 / 62,000 / 31,000 /
-// 9,918 cells 8.25 / 7.91 / 6.24 / 6.75, now 8.12 / 7.63 / 5.85 / 6.46.
+// Fewer threads leave the compiler more registers (704: 72 used, 896 and 1024:
+// 64), one cell a thread one pass instead of a second, empty one.  us a step,
+// runs of 2000 steps, two cells and 1024 threads | one cell and 1024 | 896 | 704:
+//   10,017 cells   7.07 |      | 6.34 | 6.31        108,718 (23 tiles a CTA)  8.02 | 8.20 | 7.95
+//   32,126         6.10 |      | 5.93 | 5.89        114,992 (24)              8.20 | 8.33 | 8.16
+//   64,703         7.80 |      | 6.71 | 6.64        123,227 (26)              9.82 | 9.95 | 9.76
+//  100,043 (21)    7.91 |      | 7.92 | 7.77        129,406 (27)              8.97 | 9.12 | 9.02
+//                                                   135,802 (28)              9.32 | 9.27 | 9.13
+// So 704 to 22 tiles, 896 to 28, then two cells a thread and 1024 (shared
+// memory ends at some 28 tiles of ordinary cells; cells of few junctions go on).
 template <int ZP, int CPT, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1)
 k_split_resident(FactGeom fg, SplitPtrs p, SplitConst k, ResArrays ra, int n_steps) {

@@ -1,6 +1,6 @@
 // bx_plain.cuh -- the plain FP64 step, factored per cell and per junction.
 //
-// GB300's FP64 pipe (one warp instruction in ~18 cycles per SM) bounds the
+// GB300's FP64 pipe (one warp instruction in ~19 cycles per SM) bounds the
 // plain form, so the kernel is built around how few FP64 instructions a step
 // needs.  Without extracellular spaces, Phi_b and polarizability every
 // membrane of a cell sees the same Vmem, the same membrane-side
