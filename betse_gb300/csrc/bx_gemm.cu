@@ -34,6 +34,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -381,11 +382,50 @@ int gemm(bx_dense_op* op, const double* X, double* Y, int nrhs, bool accumulate,
   return BX_OK;
 }
 
-// the error word, in mapped host memory, and the device's size
+// The operators' error words: one page of mapped host memory, kept until the
+// process ends.  (A word allocated and freed with its operator took 0.3 ms of
+// the 0.5 that a small one is made and released in.)  Operators beyond the page
+// have a word of their own.
+class ErrWords {
+ public:
+  cudaError_t take(unsigned int** w) {
+    std::lock_guard<std::mutex> lock(m_);
+    if (!page_) {
+      const cudaError_t e = cudaHostAlloc(&page_, kWords * sizeof(unsigned int), cudaHostAllocMapped | cudaHostAllocPortable);
+      if (e != cudaSuccess) return e;
+      for (int i = kWords - 1; i >= 0; --i) free_.push_back(page_ + i);
+    }
+    if (free_.empty()) {
+      const cudaError_t e = cudaHostAlloc(w, sizeof(unsigned int), cudaHostAllocMapped | cudaHostAllocPortable);
+      if (e != cudaSuccess) return e;
+    } else {
+      *w = free_.back();
+      free_.pop_back();
+    }
+    **w = 0u;
+    return cudaSuccess;
+  }
+  void give(unsigned int* w) {
+    std::lock_guard<std::mutex> lock(m_);
+    if (page_ && w >= page_ && w < page_ + kWords) free_.push_back(w);
+    else cudaFreeHost(w);
+  }
+
+ private:
+  static constexpr int kWords = 1024;
+  std::mutex m_;
+  unsigned int* page_ = nullptr;
+  std::vector<unsigned int*> free_;
+};
+ErrWords& err_words() {
+  static ErrWords* w = new ErrWords;       // (not destroyed: operators may outlive it)
+  return *w;
+}
+
+// the error word and the device's size
 cudaError_t alloc_err(bx_dense_op* op) {
-  cudaError_t e = cudaHostAlloc(&op->err, sizeof(unsigned int), cudaHostAllocMapped);
+  cudaError_t e = err_words().take(&op->err);
   if (e != cudaSuccess) return e;
-  *op->err = 0u;
   int dev = 0;
   e = cudaGetDevice(&dev);
   return e != cudaSuccess ? e : cudaDeviceGetAttribute(&op->sms, cudaDevAttrMultiProcessorCount, dev);
@@ -561,7 +601,7 @@ int bx_dense_op_destroy(bx_dense_op_handle op) {
   cudaFree(op->b_hi);
   cudaFree(op->b_lo);
   cudaFree(op->resid);
-  cudaFreeHost(op->err);
+  if (op->err) err_words().give(op->err);   // (freeing device memory has waited for the device)
   delete op;
   return BX_OK;
 }
