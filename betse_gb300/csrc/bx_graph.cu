@@ -156,8 +156,6 @@ __global__ void k_scaled_identity(int n, int K, int col0, const double* __restri
   FOR_RC(n, K) E[(long long)i * K + k] = (i == col0 + k) ? s[i] : 0.0;
 }
 
-__device__ __forceinline__ double nan_of() { return __longlong_as_double(0x7ff8000000000000LL); }
-
 // One level as the solver reads it.
 struct CgLevel {
   int n;
@@ -180,6 +178,7 @@ struct CgArgs {
   double tol;
   int max_iter;
   unsigned* ctl;           // barrier counter, timeout flag
+  double* worst;           // [8] worst relative residual of each group's columns
   double* out;             // {iterations, worst relative residual}
 };
 
@@ -198,6 +197,7 @@ struct CgCta {
   double* sub;             // shared: [3][4][32]
   int* flag;               // shared
   int kt, col, row, rows;  // rows: rows per pass
+  int kl, kown;            // log2 kt; columns of this group's slabs (some past K in the last one)
   int nrb, rb, group;      // row blocks, this CTA's row block and column group
   unsigned round;          // barriers passed
   double* scal;
@@ -206,13 +206,15 @@ struct CgCta {
   __device__ CgCta(const CgArgs& args, const CgLevel* lv_, double* red_, double* sub_, double* scal_, int* flag_)
       : a(args), lv(lv_), red(red_), sub(sub_), flag(flag_), round(0), ok(true) {
     kt = 1;
-    while (kt < a.K && kt < 32) kt <<= 1;
+    kl = 0;
+    while (kt < a.K && kt < 32) kt <<= 1, ++kl;
     col = threadIdx.x & (kt - 1);
     row = threadIdx.x / kt;
     rows = kCgT / kt;
     nrb = (int)gridDim.x / a.G;
     rb = (int)blockIdx.x / a.G;
     group = (int)blockIdx.x % a.G;
+    kown = ((a.K + kt - 1) / kt - group + a.G - 1) / a.G * kt;
     scal = a.K <= kSharedRhs ? scal_ : a.scal + (size_t)blockIdx.x * 8 * a.K;
   }
   // row block b of nb of n rows, whole aggregates
@@ -222,7 +224,8 @@ struct CgCta {
     hi = n < lo + per ? n : lo + per;
   }
   __device__ void range(int n, int& lo, int& hi) const { rows_of(n, nrb, rb, lo, hi); }
-  __device__ bool own(int k) const { return (k / kt) % a.G == group; }
+  // column q of this group's slabs (past K: none)
+  __device__ int own(int q) const { return (group + (q >> kl) * a.G) * kt + (q & (kt - 1)); }
   // the levels into `to`, the matrix rows of the staged ones into `sm`
   __device__ static void stage(const CgArgs& a, CgLevel* to, unsigned char* sm) {
     for (int l = 0; l <= a.lc; ++l) {
@@ -285,14 +288,13 @@ struct CgCta {
     __syncthreads();
   }
   // totals of quantities 0..nq-1 of buffer buf into tot[q][k], this group's
-  // columns or all of them: a warp per
-  // (quantity, column), its lanes in a fixed order
-  __device__ void totals(int buf, int nq, bool all = false) const {
+  // columns: a warp per (quantity, column), its lanes in a fixed order
+  __device__ void totals(int buf, int nq) const {
     const int lane = threadIdx.x & 31, K = a.K;
     double* tot = scal + (size_t)5 * K;
-    for (int e = threadIdx.x >> 5; e < nq * K; e += kCgT / 32) {
-      const int q = e / K, k = e - q * K;
-      if (!all && !own(k)) continue;
+    for (int e = threadIdx.x >> 5; e < nq * kown; e += kCgT / 32) {
+      const int q = e / kown, k = own(e - q * kown);
+      if (k >= K) continue;
       const double* p = a.part + ((size_t)buf * 3 + q) * nrb * K + k;
       double s = 0.0;
       for (int c0 = lane; c0 < nrb; c0 += 32 * 5) {              // 152 CTAs: one round of loads
@@ -304,7 +306,16 @@ struct CgCta {
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) tot[e] = s;
+      if (lane == 0) tot[(size_t)q * K + k] = s;
+    }
+    __syncthreads();
+  }
+  // f(k) over this group's columns, a thread each
+  template <class F>
+  __device__ void over_own(F f) const {
+    for (int q = threadIdx.x; q < kown; q += kCgT) {
+      const int k = own(q);
+      if (k < a.K) f(k);
     }
     __syncthreads();
   }
@@ -418,10 +429,11 @@ struct CgCta {
         }
       }
     } else {
-      // a thread per (row, column of this group), columns fastest
-      const int slabs = (K + kt - 1) / kt, kown = (slabs - group + a.G - 1) / a.G * kt;
-      for (int e = rb * kCgT + (int)threadIdx.x; e < n * kown; e += kCgT * nrb) {
-        const int c = e / kown, q = e - c * kown, k = (group + q / kt * a.G) * kt + q % kt;
+      // a thread per (row, column of this group), columns fastest; the warps of a
+      // group's CTAs in turn, so that few rows keep every SM busy (a CTA after the
+      // other: lapGJinv X of 100 nodes, 300 columns 1420 us, 1320 now)
+      for (int e = (int)((threadIdx.x >> 5) * nrb + rb) * 32 + (int)(threadIdx.x & 31); e < n * kown; e += kCgT * nrb) {
+        const int c = e / kown, k = own(e - c * kown);
         if (k >= K) continue;
         const double* m = a.dense + (size_t)c * n;
         double s0 = 0.0, s1 = 0.0;
@@ -489,6 +501,9 @@ struct CgCta {
   }
 };
 
+// the larger of two values that are not negative, NaN where either is
+__device__ __forceinline__ double max_or_nan(double x, double y) { return x != x || y <= x ? x : y; }
+
 // num / den, 0 where either vanishes (a converged column stops moving)
 __device__ __forceinline__ double guarded_ratio(double num, double den) {
   return (den != 0.0 && num != 0.0) ? num / den : 0.0;
@@ -512,7 +527,11 @@ __global__ void __launch_bounds__(kCgT, 1) k_graph_cg(CgArgs a) {
   const CgLevel& L = slv[0];
   // column scalars: r.z of the last and of this iteration (by parity), |b|^2,
   // the mean to take off and beta or alpha.  One thread a column computes
-  // them: on the slow FP64 pipe every warp doing so cost 7,000 cycles a phase.
+  // them, of this group's columns: on the slow FP64 pipe every warp doing so cost
+  // 7,000 cycles a phase.  (Every CTA with all columns, and the residuals in one
+  // warp, lapGJinv X took, in us: 100 nodes, 1024 columns 4390, 2340 now; 700
+  // nodes 24,200, 16,800 now; 1500 nodes 34,400, 26,400 now; 20,000 nodes, 256
+  // columns 95,700, 91,100 now.)
   double *rz0 = g.scal, *rz1 = rz0 + K, *bb = rz1 + K, *mean = bb + K, *fac = mean + K;
   enum { BUF_Z = 0, BUF_R = 1 };   // sums that may be read while the next phase's are written
 
@@ -524,8 +543,7 @@ __global__ void __launch_bounds__(kCgT, 1) k_graph_cg(CgArgs a) {
   }
   if (!g.barrier()) return;
   g.totals(BUF_Z, 1);
-  for (int k = threadIdx.x; k < K; k += kCgT) mean[k] = g.tot(0, k) * (1.0 / n);
-  __syncthreads();
+  g.over_own([&](int k) { mean[k] = g.tot(0, k) * (1.0 / n); });
   for (int kb = g.group * kt; kb < K; kb += a.G * kt) {
     const int k = kb + g.col;
     double v = 0.0;
@@ -542,8 +560,8 @@ __global__ void __launch_bounds__(kCgT, 1) k_graph_cg(CgArgs a) {
     g.cta_sum(BUF_R, kb, 1, &v);
   }
   if (!g.barrier()) return;
-  g.totals(BUF_R, 1, true);
-  for (int k = threadIdx.x; k < K; k += kCgT) bb[k] = g.tot(0, k);
+  g.totals(BUF_R, 1);
+  g.over_own([&](int k) { bb[k] = g.tot(0, k); });
   if (!g.precondition(BUF_Z)) return;
 
   double worst = 0.0;
@@ -556,13 +574,12 @@ __global__ void __launch_bounds__(kCgT, 1) k_graph_cg(CgArgs a) {
     const bool first = it == 1;              // no old P: z with beta = 0 in its place
     const double* Po = first ? a.Z : (it & 1) ? a.P1 : a.P0;
     double* Pn = (it & 1) ? a.P0 : a.P1;
-    for (int k = threadIdx.x; k < K; k += kCgT) {
+    g.over_own([&](int k) {
       const double m = g.tot(0, k) * (1.0 / n), nw = g.tot(1, k) - m * g.tot(2, k);
       mean[k] = m;
       rzn[k] = nw;
       fac[k] = first ? 0.0 : guarded_ratio(nw, rzo[k]);
-    }
-    __syncthreads();
+    });
     for (int kb = g.group * kt; kb < K; kb += a.G * kt) {
       const int k = kb + g.col;
       double v = 0.0;
@@ -584,8 +601,7 @@ __global__ void __launch_bounds__(kCgT, 1) k_graph_cg(CgArgs a) {
     // ---- X, R
     g.totals(BUF_R, 1);
     const bool check = it % kCheckEvery == 0 || it == a.max_iter;
-    for (int k = threadIdx.x; k < K; k += kCgT) fac[k] = guarded_ratio(rzn[k], g.tot(0, k));
-    __syncthreads();
+    g.over_own([&](int k) { fac[k] = guarded_ratio(rzn[k], g.tot(0, k)); });
     for (int kb = g.group * kt; kb < K; kb += a.G * kt) {
       const int k = kb + g.col;
       double v = 0.0;
@@ -603,23 +619,27 @@ __global__ void __launch_bounds__(kCgT, 1) k_graph_cg(CgArgs a) {
     }
     if (!g.barrier()) return;
     if (check) {
-      // the worst column, the same in every CTA
-      g.totals(BUF_Z, 1, true);
-      if (threadIdx.x < 32) {                // one warp: FP64 compares are slow
-        double w = 0.0;
-        bool nan = false;
-        for (int k = lane; k < K; k += 32) {
-          const double b = bb[k];
-          const double x = b > 0.0 ? sqrt(g.tot(0, k) / b) : 0.0;
-          nan |= x != x;
-          w = fmax(w, x);
-        }
-        nan = __any_sync(0xffffffffu, nan);
-        for (int o = 16; o > 0; o >>= 1) w = fmax(w, __shfl_xor_sync(0xffffffffu, w, o));
-        if (lane == 0) red[0] = nan ? nan_of() : w;
+      // the worst column, the same in every CTA (NaN if any is): the group's from
+      // its totals, then the groups' across a barrier
+      g.totals(BUF_Z, 1);
+      double w = 0.0;
+      g.over_own([&](int k) { w = max_or_nan(w, bb[k] > 0.0 ? g.tot(0, k) / bb[k] : 0.0); });
+      if ((int)(threadIdx.x & ~31u) < g.kown)              // (FP64 compares are slow: warps with columns only)
+        for (int o = 16; o > 0; o >>= 1) w = max_or_nan(w, __shfl_xor_sync(0xffffffffu, w, o));
+      if (lane == 0) red[threadIdx.x >> 5] = w;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        for (int q = 1; q < (min(g.kown, kCgT) + 31) / 32; ++q) w = max_or_nan(w, red[q]);   // (the other warps had no column)
+        w = sqrt(w);
+        red[0] = w;
+        if (a.G > 1 && g.rb == 0) a.worst[g.group] = w;
       }
       __syncthreads();
       worst = red[0];
+      if (a.G > 1) {
+        if (!g.barrier()) return;
+        for (int q = 0; q < a.G; ++q) worst = max_or_nan(worst, __ldcg(a.worst + q));
+      }
       __syncthreads();
       if (!(worst > a.tol) || it == a.max_iter) break;    // converged, NaN or out of iterations
     }
@@ -736,6 +756,7 @@ int solve_async(bx_graph_solver* h, const double* B, double* X, int K, double to
   a.B = B; a.X = X; a.R = h->R; a.Z = h->Z; a.P0 = h->P0; a.P1 = h->P1; a.Q = h->Q;
   a.part = h->part; a.scal = h->scal; a.tol = tol; a.max_iter = max_iter; a.ctl = h->ctl + 2 * slot;
   a.out = h->out + 2 * slot;
+  a.worst = h->out + 4;
   GCK(cudaMemsetAsync(a.ctl, 0, 2 * sizeof(unsigned), s));
   if (counter) GCK(cudaMemsetAsync(a.ctl, counter, sizeof(unsigned), s));
   void* args[] = {&a};
@@ -938,7 +959,7 @@ extern "C" int bx_graph_create(int n_levels, const bx_graph_level* levels, const
     for (double** v : {&h->R, &h->Z, &h->P0, &h->P1, &h->Q, &h->T1, &h->T2}) *v = h->alloc<double>(big);
     h->part = h->alloc<double>((size_t)2 * 3 * h->grid * max_rhs);
     h->scal = h->alloc<double>((size_t)8 * h->grid * max_rhs);
-    h->out = h->alloc<double>(4);
+    h->out = h->alloc<double>(4 + 8);      // and the column groups' residuals
     h->ctl = h->alloc<unsigned>(4);
     ok = h->w_ptr && h->w_col && h->w_val && h->area && h->R && h->Z && h->P0 && h->P1 && h->Q && h->T1 && h->T2 &&
          h->part && h->scal && h->out && h->ctl;
