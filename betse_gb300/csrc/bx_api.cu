@@ -126,7 +126,7 @@ struct bx_cluster {
   // ---- split form: tile-major slots (Q membrane slots, S cell slots)
   int Q = 0, S = 0;
   uint8_t* t_lcell = nullptr;
-  int *t_nn = nullptr, *t_map_env = nullptr, *t_nn_env = nullptr, *t_c0 = nullptr, *t_m0 = nullptr,
+  int *t_nn = nullptr, *t_map_env = nullptr, *t_nn_env = nullptr, *t_env_row = nullptr /* ECM */, *t_c0 = nullptr, *t_m0 = nullptr,
       *t_slot_of_cell = nullptr;
   float *t_sa = nullptr, *t_gw = nullptr, *t_dtv = nullptr, *t_dvc = nullptr;
   short2* t_rng = nullptr;
@@ -172,7 +172,7 @@ struct bx_cluster {
   cudaGraphExec_t graph = nullptr;
   bool graph_valid = false;
   int64_t layout_gen = 0;          // bumped with every change that a captured graph would not see
-  std::vector<int> h_cell_ptr, h_m2c, h_map_env;
+  std::vector<int> h_cell_ptr, h_m2c, h_map_env, h_env_slot;
   std::vector<double> h_phib;
   // ---- environment fields on demand (bx_env_fields)
   float2* f_lap = nullptr;         // lapENVinv as double-float pairs [G][f_ld], columns >= G zero
@@ -228,7 +228,7 @@ void free_all(bx_cluster* h) {
       h->d_ny, h->d_swm, h->d_swo, h->d_cell_vol, h->d_cell_sa, h->d_diviterm, h->d_mem_sa_f,
       h->d_gj_w_f, h->d_gjw0_f, h->d_dtv, h->d_dvc, h->d_Dm, h->d_Dm_f, h->d_vm[0], h->d_vm[1],
       h->d_ccm[0], h->d_ccm[1], h->d_cc, h->s_cc2, h->s_rec[0], h->s_rec[1], h->s_count,
-      h->t_lcell, h->t_nn, h->t_map_env, h->t_nn_env, h->t_c0, h->t_m0, h->t_slot_of_cell, h->t_sa,
+      h->t_lcell, h->t_nn, h->t_map_env, h->t_nn_env, h->t_env_row, h->t_c0, h->t_m0, h->t_slot_of_cell, h->t_sa,
       h->t_gw, h->t_dtv, h->t_dvc, h->t_rng,
       h->s_cenv_f, h->s_pump, h->s_part, h->s_phib, h->d_cenv, h->d_phib, h->d_env_part,
       h->d_mem_flux_sa, h->d_pump, h->d_env_scale, h->d_Denv, h->d_Ex, h->d_Ey, h->d_fx, h->d_fy,
@@ -439,7 +439,7 @@ bx::SplitPtrs split_ptrs(bx_cluster* h, int parity) {
   p.o_drho = h->o_drho;
   p.cenv_grid = h->ecm ? h->d_cenv : nullptr;
   p.mfs = h->d_mem_flux_sa;
-  p.env_slot = h->d_env_slot;
+  p.env_row = h->t_env_row;
   p.gjo = h->t_gjo;
   p.o_gjopen = h->o_gjopen;
   p.ca_env = ca_env_ptr(h);
@@ -857,7 +857,7 @@ cudaError_t enqueue_env_pre(bx_cluster* h, cudaStream_t s) {
   bx::k_env_update<<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_fx, h->d_fy, ec);
   h->launches += 2;
   if (h->par.sharpness < 1.0) {
-    bx::k_env_integrate_scatter<false><<<gi, kEnvTPB, 0, s>>>(h->d_cnew, h->d_tmp2, h->d_env_ptr, h->d_mem_flux_sa, ec);
+    bx::k_env_integrate<<<gi, kEnvTPB, 0, s>>>(h->d_cnew, h->d_tmp2, ec);
     h->launches += 1;
   }
   return cudaGetLastError();
@@ -868,6 +868,7 @@ cudaError_t enqueue_env(bx_cluster* h, bool out, bool flux_done, cudaStream_t s)
   bx::EnvConst ec = make_env_const(h);
   const int gg = env_grid(h->G);
   const int gi = env_grid(h->G * h->I);   // one thread per (ion, grid cell)
+  const unsigned gc = (unsigned)((h->G + bx::kEnvUpCells - 1) / bx::kEnvUpCells);
   const bool split = h->mode == MODE_SPLIT && !(h->par.sharpness < 1.0);   // FP32 stencils around FP64 state
   if (!flux_done && !h->ca) {
     bx::k_env_np_flux<double><<<gi, kEnvTPB, 0, s>>>(env_np(h, 0));   // (the split form's FP32 flux: with its cells)
@@ -875,17 +876,16 @@ cudaError_t enqueue_env(bx_cluster* h, bool out, bool flux_done, cudaStream_t s)
   }
   if (h->ca) {
     const double* src = (h->par.sharpness < 1.0) ? h->d_cnew : h->d_tmp2;
-    bx::k_env_scatter_add<<<gi, kEnvTPB, 0, s>>>(h->d_cenv, src, h->d_env_ptr, h->d_mem_flux_sa, ec);
+    bx::k_env_scatter<false><<<gc, bx::kEnvUpT, 0, s>>>(h->d_cenv, src, h->d_env_ptr, h->d_mem_flux_sa, ec);
     h->launches += 1;
   } else if (h->par.sharpness < 1.0) {
     bx::k_env_update<<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_fx, h->d_fy, ec);
-    bx::k_env_integrate_scatter<true><<<gi, kEnvTPB, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_env_ptr, h->d_mem_flux_sa, ec);
+    bx::k_env_scatter<true><<<gc, bx::kEnvUpT, 0, s>>>(h->d_cenv, h->d_tmp2, h->d_env_ptr, h->d_mem_flux_sa, ec);
     h->launches += 2;
   } else {
     // the common configuration: update + charge fused, then the fields in one
     // tiled launch (with the cell kernel's, which computes the flux too, three
     // dependent launches a step)
-    const unsigned gc = (unsigned)((h->G + bx::kEnvUpCells - 1) / bx::kEnvUpCells);
     const unsigned ntx = (unsigned)((h->nx + bx::kEnvTX - 1) / bx::kEnvTX),
                    nty = (unsigned)((h->ny + bx::kEnvTY - 1) / bx::kEnvTY);
     const double* phib = h->phib_nonzero ? h->d_phib : nullptr;
@@ -1192,7 +1192,7 @@ int build_split_layout(bx_cluster* h, const std::vector<int>& blk) {
   const int Q = tpb * nblk, S = bx::kCellsPerCta * nblk;
   const std::vector<int>& ptr = h->h_cell_ptr;
   std::vector<uint8_t> lcell(Q, 255);
-  std::vector<int> nn_slot(Q), map_env(Q, 0), nn_env(Q, 0), t_c0(nblk), t_m0(nblk);
+  std::vector<int> nn_slot(Q), map_env(Q, 0), nn_env(Q, 0), env_row(h->ecm ? Q : 0), t_c0(nblk), t_m0(nblk);
   std::vector<float> sa(Q, 0.f), gw(Q, 0.f);
   std::vector<short2> rng(S, make_short2(0, 0));
   h->h_slot_of_cell.assign(C, 0);
@@ -1213,6 +1213,7 @@ int build_split_layout(bx_cluster* h, const std::vector<int>& blk) {
         sa[qq] = (float)h->h_msa[m];
         gw[qq] = h->h_bflag[m] ? 0.f : (float)h->h_gjw[m];
         map_env[qq] = h->h_map_env[m];
+        if (h->ecm) env_row[qq] = h->h_env_slot[m];
       }
     }
   }
@@ -1221,12 +1222,12 @@ int build_split_layout(bx_cluster* h, const std::vector<int>& blk) {
     nn_slot[qq] = h->h_slot_of_cell[h->h_m2c[h->h_nn[m]]];
     nn_env[qq] = h->h_map_env[h->h_nn[m]];
   }
-  void* old[] = {h->t_lcell, h->t_nn, h->t_map_env, h->t_nn_env, h->t_c0, h->t_m0, h->t_slot_of_cell,
+  void* old[] = {h->t_lcell, h->t_nn, h->t_map_env, h->t_nn_env, h->t_env_row, h->t_c0, h->t_m0, h->t_slot_of_cell,
                  h->t_sa, h->t_gw, h->t_dtv, h->t_dvc, h->t_rng, h->d_Dm_f, h->s_cc2, h->s_rec[0], h->s_rec[1],
                  h->t_gjo, h->t_slot_of_mem};
   for (void* q : old)
     if (q) cudaFree(q);
-  h->t_lcell = nullptr; h->t_nn = h->t_map_env = h->t_nn_env = h->t_c0 = h->t_m0 = h->t_slot_of_cell = nullptr;
+  h->t_lcell = nullptr; h->t_nn = h->t_map_env = h->t_nn_env = h->t_env_row = h->t_c0 = h->t_m0 = h->t_slot_of_cell = nullptr;
   h->t_sa = h->t_gw = h->t_dtv = h->t_dvc = nullptr; h->t_rng = nullptr; h->d_Dm_f = nullptr;
   h->s_cc2 = nullptr; h->s_rec[0] = h->s_rec[1] = nullptr;
   h->t_gjo = nullptr;
@@ -1240,6 +1241,7 @@ int build_split_layout(bx_cluster* h, const std::vector<int>& blk) {
   BX_CU(dalloc(&h->t_lcell, Q)); BX_CU(h2d(h->t_lcell, lcell.data(), Q));
   BX_CU(dalloc(&h->t_nn, Q)); BX_CU(h2d(h->t_nn, nn_slot.data(), Q));
   BX_CU(dalloc(&h->t_map_env, Q)); BX_CU(h2d(h->t_map_env, map_env.data(), Q));
+  if (h->ecm) { BX_CU(dalloc(&h->t_env_row, Q)); BX_CU(h2d(h->t_env_row, env_row.data(), Q)); }
   BX_CU(dalloc(&h->t_nn_env, Q)); BX_CU(h2d(h->t_nn_env, nn_env.data(), Q));
   BX_CU(dalloc(&h->t_c0, nblk)); BX_CU(h2d(h->t_c0, t_c0.data(), nblk));
   BX_CU(dalloc(&h->t_m0, nblk)); BX_CU(h2d(h->t_m0, t_m0.data(), nblk));
@@ -1607,6 +1609,7 @@ int create_impl(const bx_geom* gs, const bx_params* ps, int ncl, int precision, 
     for (int k = 0; k < G; ++k) env_ptr[k + 1] += env_ptr[k];
     std::vector<int> fill(env_ptr.begin(), env_ptr.end() - 1);
     for (int m = 0; m < M; ++m) env_slot[m] = fill[map_env[m]]++;
+    h->h_env_slot = env_slot;
     for (int k = 0; k < G; ++k) touched[k] = env_ptr[k + 1] > env_ptr[k];
     double s = 0.0;
     for (int m = 0; m < M; ++m) s += gs[0].mem_sa_per_env[map_env[m]];

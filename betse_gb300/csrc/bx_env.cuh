@@ -71,52 +71,63 @@ __global__ void k_env_charge(const double* __restrict__ cenv, const uint8_t* __r
   env_charge_out(k, rho, touched, vsrc, rho_env, e);
 }
 
-// fd.integrator (finitediff.py:1479-1512) when sharpness < 1, then the membrane
-// exchange (SCATTER; without it the smoothed grid is written to cenv, which is
-// then a separate buffer).  One thread per (ion, grid cell).
-template <bool SCATTER = true>
-__global__ void k_env_integrate_scatter(double* cenv, const double* __restrict__ tmp,
-                                        const int* __restrict__ env_ptr,
-                                        const double* __restrict__ mem_flux_sa, EnvConst e) {
+// fd.integrator (finitediff.py:1479-1512) of grid value k of one ion
+__device__ __forceinline__ double env_integrate(const double* P, const EnvConst& e, int k) {
+  const int i = k / e.nx, j = k - i * e.nx;
+  if (on_edge(i, j, e.ny, e.nx)) return P[k];
+  const double sides = (1 - e.sharpness) / 4;
+  double F = e.sharpness * P[k];
+  F += sides * P[k + e.nx];
+  F += sides * P[k - e.nx];
+  F += sides * P[k + 1];
+  F += sides * P[k - 1];
+  return F;
+}
+
+// The membrane exchange of one ion over rows [q0, q1), four at a time (their
+// loads are independent), added in list order; a cell's lanes read a row together
+__device__ __forceinline__ double env_exchange(const double* __restrict__ mem_flux_sa, int q0, int q1, int ion) {
+  double s = 0.0;
+  for (; q0 < q1; q0 += 4) {
+    double fv[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) fv[u] = q0 + u < q1 ? mem_flux_sa[(size_t)(q0 + u) * kMfs + ion] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (q0 + u < q1) s += -fv[u];
+  }
+  return s;
+}
+
+// The smoothed grid, where the membrane exchange is a later pass.  One thread
+// per (ion, grid cell).
+__global__ void k_env_integrate(double* out, const double* __restrict__ tmp, EnvConst e) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= e.I * e.G) return;
   const int ion = t / e.G, k = t - ion * e.G;
-  const int i = k / e.nx, j = k - i * e.nx;
-  const double sides = (1 - e.sharpness) / 4;
-  {
-    const double* P = tmp + (size_t)ion * e.G;
-    double F;
-    if (on_edge(i, j, e.ny, e.nx)) {
-      F = P[k];
-    } else {
-      F = e.sharpness * P[k];
-      F += sides * P[k + e.nx];
-      F += sides * P[k - e.nx];
-      F += sides * P[k + 1];
-      F += sides * P[k - 1];
-    }
-    if (!SCATTER) {
-      cenv[(size_t)ion * e.G + k] = F;
-      return;
-    }
-    double s = 0.0;
-    for (int q = env_ptr[k]; q < env_ptr[k + 1]; ++q) s += -mem_flux_sa[(size_t)q * kMfs + ion];
-    cenv[(size_t)ion * e.G + k] = F + (s * e.inv_h_d2) * e.dt;
-  }
+  out[t] = env_integrate(tmp + (size_t)ion * e.G, e, k);
 }
 
 // The membrane exchange onto an environment already advanced by the
-// Nernst-Planck update (and smoothing): update_Co's ECM term
-// (sim_toolbox.py:1185-1200), the same arithmetic as the fused kernels.
-__global__ void k_env_scatter_add(double* cenv, const double* __restrict__ src,
-                                  const int* __restrict__ env_ptr,
-                                  const double* __restrict__ mem_flux_sa, EnvConst e) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= e.I * e.G) return;
-  const int ion = t / e.G, k = t - ion * e.G;
-  double s = 0.0;
-  for (int q = env_ptr[k]; q < env_ptr[k + 1]; ++q) s += -mem_flux_sa[(size_t)q * kMfs + ion];
-  cenv[t] = src[t] + (s * e.inv_h_d2) * e.dt;
+// Nernst-Planck update: update_Co's ECM term (sim_toolbox.py:1185-1200), the
+// same arithmetic as the fused kernels.  INTEGRATE: src is smoothed on the way
+// (sharpness < 1).  kEnvUpCells grid cells per CTA, a lane per (cell, ion) with
+// the ions contiguous, which read an exchange row together (by itself, 20,000
+// cells on 200 x 200: 10.0 us; a thread per ion and cell in grid order, row after
+// row, 11.8).
+constexpr int kEnvUpT = 192, kEnvUpCells = 32;
+template <bool INTEGRATE>
+__global__ void __launch_bounds__(kEnvUpT) k_env_scatter(double* cenv, const double* __restrict__ src,
+                                                         const int* __restrict__ env_ptr,
+                                                         const double* __restrict__ mem_flux_sa, EnvConst e) {
+  const int k0 = blockIdx.x * kEnvUpCells, nk = min(kEnvUpCells, e.G - k0);
+  for (int q = threadIdx.x; q < nk * e.I; q += kEnvUpT) {
+    const int lk = q / e.I, ion = q - lk * e.I, k = k0 + lk;
+    const double s = env_exchange(mem_flux_sa, env_ptr[k], env_ptr[k + 1], ion);
+    const double* P = src + (size_t)ion * e.G;
+    const double F = INTEGRATE ? env_integrate(P, e, k) : P[k];
+    cenv[(size_t)ion * e.G + k] = F + (s * e.inv_h_d2) * e.dt;
+  }
 }
 
 // get_current ECM branch (ion_current.py:79-110): the axis-0 pass of a
@@ -193,7 +204,6 @@ __global__ void k_env_neg_grad(const double* __restrict__ F, double scale, doubl
 // warp instructions per four cells took 24 us (split) and 22 us (FP64) on
 // 200 x 200 cells; as written 11.5 and 13 us (a launch by itself; split with the
 // fluxes and constants converted from FP64 by every thread 15.0).
-constexpr int kEnvUpT = 192, kEnvUpCells = 32;
 template <typename R>
 __global__ void __launch_bounds__(kEnvUpT) k_env_update_charge(double* cenv, const R* __restrict__ fx,
                                                                const R* __restrict__ fy,
@@ -211,18 +221,7 @@ __global__ void __launch_bounds__(kEnvUpT) k_env_update_charge(double* cenv, con
     const R* fyi = fy + (size_t)ion * e.G;
     const R div = ddx_neg<R>(fxi, e, i, j) + ddy_neg<R>(fyi, e, i, j);
     double c = cb_at(cenv, e, ion, i, j) + (double)(div * env_dt<R>(e));
-    // the membrane exchange, four rows at a time (their loads are
-    // independent), added in list order; a cell's lanes read a row together
-    double s = 0.0;
-    const int q1 = env_ptr[k + 1];
-    for (int q0 = env_ptr[k]; q0 < q1; q0 += 4) {
-      double fv[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) fv[u] = q0 + u < q1 ? mem_flux_sa[(size_t)(q0 + u) * kMfs + ion] : 0.0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (q0 + u < q1) s += -fv[u];
-    }
+    const double s = env_exchange(mem_flux_sa, env_ptr[k], env_ptr[k + 1], ion);
     c = c + (s * e.inv_h_d2) * e.dt;
     cenv[(size_t)ion * e.G + k] = c;
     zc[q] = e.zF[ion] * c;
