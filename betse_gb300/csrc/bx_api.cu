@@ -157,7 +157,7 @@ struct bx_cluster {
       *pl_n_local = nullptr, *pl_mem_ent = nullptr, *pl_mem_gate = nullptr;
   double *pl_mem_w = nullptr, *pl_dsa = nullptr, *pl_sa = nullptr, *pl_ivol = nullptr, *pl_part = nullptr,
          *pl_gpart = nullptr;
-  unsigned *pl_ticket = nullptr, *pl_ctl = nullptr;   // [groups + ncl]; barrier counter and timeout flag
+  unsigned *pl_ticket = nullptr, *pl_ctl = nullptr;   // [groups + ncl]; barrier counter and timeout flag (behind d_status)
   int64_t pl_nent = 0;
   // ---- outputs
   double *o_fmem = nullptr, *o_fgj = nullptr, *o_rate = nullptr, *o_rho = nullptr, *o_Jn = nullptr,
@@ -1410,7 +1410,7 @@ int build_plain_layout(bx_cluster* h) {
                o_clg = take((ncl + 1) * sizeof(int)), o_ep = take((nt + 1) * sizeof(int)),
                o_nl = take(nt * sizeof(int)), o_me = take((size_t)M * sizeof(int)),
                o_mg = take(mem_gate.size() * sizeof(int)), o_tk = take((ng + ncl) * sizeof(unsigned)),
-               o_ctl = take(2 * sizeof(unsigned)), host_bytes = off, o_part = take((size_t)2 * nt * I * sizeof(double)),
+               host_bytes = off, o_part = take((size_t)2 * nt * I * sizeof(double)),
                o_gp = take((size_t)(2 * ng + 8 * ncl) * I * sizeof(double)), o_mw = take((size_t)M * sizeof(double)),
                o_sa = take((size_t)C * sizeof(double)), o_iv = take((size_t)C * sizeof(double)),
                o_dsa = take((size_t)I * (h->ecm ? M : C) * sizeof(double));
@@ -1438,7 +1438,6 @@ int build_plain_layout(bx_cluster* h) {
   h->pl_tile_cl = i32(o_tcl); h->pl_cl_tile = i32(o_clt); h->pl_cl_group = i32(o_clg); h->pl_ent_ptr = i32(o_ep);
   h->pl_n_local = i32(o_nl); h->pl_mem_ent = i32(o_me); h->pl_mem_gate = i32(o_mg);
   h->pl_ticket = reinterpret_cast<unsigned*>(d + o_tk);
-  h->pl_ctl = reinterpret_cast<unsigned*>(d + o_ctl);
   h->pl_part = dbl(o_part); h->pl_gpart = dbl(o_gp); h->pl_mem_w = dbl(o_mw); h->pl_sa = dbl(o_sa);
   h->pl_ivol = dbl(o_iv); h->pl_dsa = dbl(o_dsa);
   bx::k_plain_static<<<(C + 255) / 256, 256, 0, h->stream>>>(C, h->d_cell_ptr, h->d_gj_w, h->d_mem_sa, h->d_cell_vol,
@@ -1644,8 +1643,9 @@ int create_impl(const bx_geom* gs, const bx_params* ps, int ncl, int precision, 
   if (h->polar) { ALLOC(h->d_Rrads, M); H2D(h->d_Rrads, rr.data(), M); }
   ALLOC(h->d_pump, ncl); ALLOC(h->d_env_scale, ncl);
   ALLOC(h->d_phib, G);
-  ALLOC(h->d_status, 4);
-  if (cudaMemset(h->d_status, 0, 4 * sizeof(unsigned long long)) != cudaSuccess ||
+  ALLOC(h->d_status, 5);
+  h->pl_ctl = reinterpret_cast<unsigned*>(h->d_status + 4);
+  if (cudaMemset(h->d_status, 0, 5 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMemset(h->d_phib, 0, (size_t)G * sizeof(double)) != cudaSuccess)
     return bail(BX_ECUDA, "cudaMemset");
   if (h->mode == MODE_SPLIT) {
@@ -1799,19 +1799,17 @@ int bx_set_membrane_diffusivity(bx_handle h, const double* Dm) {
     BX_CU(cudaMemcpy(h->d_Dm_f, f.data(), n * sizeof(float), cudaMemcpyHostToDevice));
   } else {
     BX_CU(cudaMemcpy(h->d_Dm, Dm, n * sizeof(double), cudaMemcpyHostToDevice));
-    if (h->pl_dsa) {
-      BX_CU(plain_dsa(h));
-      BX_CU(cudaStreamSynchronize(h->stream));
-    }
+    if (h->pl_dsa) BX_CU(plain_dsa(h));        // on the handle's stream, which every step follows
   }
   h->have_dm = true;
   return BX_OK;
 }
 
-// FP32 copy of an FP64 array, rounded to nearest
-__global__ void k_round_to_float(const double* __restrict__ a, float* __restrict__ b, int n) {
+// FP32 copy of an FP64 array (with a second row of blocks, of two), rounded to nearest
+__global__ void k_round_to_float(const double* __restrict__ a, float* __restrict__ b, int n,
+                                 const double* __restrict__ a2, float* __restrict__ b2) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = __double2float_rn(a[i]);
+  if (i < n) (blockIdx.y ? b2 : b)[i] = __double2float_rn((blockIdx.y ? a2 : a)[i]);
 }
 
 int bx_set_env_diffusivity(bx_handle h, const double* D_env) {
@@ -1821,7 +1819,7 @@ int bx_set_env_diffusivity(bx_handle h, const double* D_env) {
   BX_CU(cudaMemcpyAsync(h->d_Denv, D_env, (size_t)h->I * h->G * sizeof(double), cudaMemcpyHostToDevice, h->stream));
   if (h->d_Denv_f) {
     const int n = h->I * h->G;
-    k_round_to_float<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(h->d_Denv, h->d_Denv_f, n);
+    k_round_to_float<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(h->d_Denv, h->d_Denv_f, n, nullptr, nullptr);
     BX_CU(cudaGetLastError());
   }
   BX_CU(cudaStreamSynchronize(h->stream));
@@ -1916,8 +1914,8 @@ int bx_state_upload(bx_handle h, const bx_state* s) {
   bx::k_state_check<<<(M + tb - 1) / tb, tb, 0, st>>>(io, vm_dst, h->st_cam, split ? 1 : 2, h->d_flag,
                                                       split ? nullptr : h->d_ccm[0]);
   BX_CU(cudaGetLastError());
-  for (unsigned* c : {h->r_ctl, h->pl_ctl})
-    if (c) BX_CU(cudaMemsetAsync(c, 0, 2 * sizeof(unsigned), st));   // a fresh state: no timeout
+  if (unsigned* c = split ? h->r_ctl : h->pl_res ? h->pl_ctl : nullptr)
+    BX_CU(cudaMemsetAsync(c, 0, 2 * sizeof(unsigned), st));   // a fresh state: no timeout
   int flag[2] = {0, 0};
   BX_CU(cudaMemcpyAsync(flag, h->d_flag, sizeof(flag), cudaMemcpyDeviceToHost, st));
   BX_CU(cudaStreamSynchronize(st));
@@ -1939,10 +1937,10 @@ int bx_state_upload(bx_handle h, const bx_state* s) {
       BX_CU(cudaGetLastError());
     }
     if (!h->ecm) {
-      k_round_to_float<<<(unsigned)((nenv + 255) / 256), 256, 0, st>>>(h->d_cenv, h->s_cenv_f, (int)nenv);
+      k_round_to_float<<<(unsigned)((nenv + 255) / 256), 256, 0, st>>>(h->d_cenv, h->s_cenv_f, (int)nenv, nullptr, nullptr);
     } else {
-      k_round_to_float<<<(unsigned)((h->G + 255) / 256), 256, 0, st>>>(h->d_Ex, h->d_Ex_f, h->G);
-      k_round_to_float<<<(unsigned)((h->G + 255) / 256), 256, 0, st>>>(h->d_Ey, h->d_Ey_f, h->G);
+      k_round_to_float<<<dim3((unsigned)((h->G + 255) / 256), 2), 256, 0, st>>>(h->d_Ex, h->d_Ex_f, h->G, h->d_Ey,
+                                                                                h->d_Ey_f);
     }
     BX_CU(cudaGetLastError());
     BX_CU(cudaStreamSynchronize(st));
@@ -2106,12 +2104,13 @@ int bx_step(bx_handle h, int n_steps, int want_outputs, void* stream) {
 
 int bx_status(bx_handle h, bx_step_status* st) {
   if (!h || !st) return fail(BX_EINVAL, "null argument");
-  unsigned long long v[4];
+  unsigned long long v[5];                   // the counters, then the plain form's barrier words
   unsigned ctl[2] = {0u, 0u};
   unsigned* rc = h->mode == MODE_SPLIT ? h->r_ctl : h->pl_res ? h->pl_ctl : nullptr;
   BX_CU(cudaMemcpyAsync(v, h->d_status, sizeof(v), cudaMemcpyDeviceToHost, h->stream));
-  if (rc) BX_CU(cudaMemcpyAsync(ctl, rc, sizeof(ctl), cudaMemcpyDeviceToHost, h->stream));
+  if (rc && rc != h->pl_ctl) BX_CU(cudaMemcpyAsync(ctl, rc, sizeof(ctl), cudaMemcpyDeviceToHost, h->stream));
   BX_CU(cudaStreamSynchronize(h->stream));
+  if (rc == h->pl_ctl) std::memcpy(ctl, &v[4], sizeof(ctl));
   st->steps_done = h->steps_done;
   st->nan_vm = (int32_t)std::min<unsigned long long>(v[0], 0x7fffffff);
   st->nan_conc = (int32_t)std::min<unsigned long long>(v[1], 0x7fffffff);
