@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kTcThreads) k_fwd_tc(FwdArgs a) {
 // the transposed neighbour mean of the layer above's G.  Bound by the FMA pipe
 // (the gradients are FP32); with a warp per node, operands by shuffle and the
 // weight gradients in their own passes a training step of 30,858 nodes took
-// 653 us, 245 now (a middle layer 109 us before, 36 to 44 now).
+// 680 us, its call included, 270 now (a middle layer 109 us before, 38 to 44 now).
 constexpr int kBwdT = 256, kBwdRows = 64, kBwdPerSM = 2;
 
 struct BwdArgs {

@@ -18,8 +18,8 @@
 //     before and after the coarse correction, which is over-weighted by 1.8
 //     (unsmoothed aggregation under-corrects smooth errors);
 //   * the first level of at most 512 nodes is solved exactly with its
-//     pseudo-inverse, built on the GPU at creation (with 2048 nodes 72 CG
-//     iterations instead of 84, but 30 ms more at creation); in blocks of more
+//     pseudo-inverse, built on the GPU at creation (with 2048 nodes 76 CG
+//     iterations instead of 88, but 30 ms more at creation); in blocks of more
 //     than eight columns, which the FP64 pipe bounds, the first level whose
 //     dense product stays under 4 % of the work (its nodes squared at most
 //     twice the finest level's); a graph of at most 512 nodes is that one
@@ -27,9 +27,9 @@
 //   * every right-hand side and every preconditioned residual is projected
 //     orthogonal to the constants (the null space of L), so the iterate
 //     stays in the range of L+.
-// At 100k cells this takes 70 iterations to a relative residual of 1e-12
-// (two sweeps on each side and a 64-node coarsest level: 73; plain
-// Jacobi-preconditioned CG: ~1500).
+// At 100k cells this takes 84 iterations to a relative residual of 1e-12, 88 to
+// 0.4 of it, where a solve to 1e-12 stops (two sweeps on each side and a 64-node
+// coarsest level: 76 to 1e-12; plain Jacobi-preconditioned CG: ~1500).
 //
 // A solve is one cooperative launch (k_graph_cg), one CTA per SM, whose phases
 // (product, update, a restriction and a prolongation per level, the dense
@@ -37,9 +37,9 @@
 // launches an iteration at 100k cells and one column was 36 kernels and 0.3 ms;
 // it is 50 us now, about 10 us of it FP64 work and 14 us barriers, the rest the
 // L2 round trips of the phases.  lapGJinv X (two solves to 1e-12), ms, separate
-// launches -> one launch: 100k cells, 1 / 16 / 64 / 256 columns 45.8 -> 8.5,
-// 87 -> 52, 232 -> 139, 849 -> 487; 20k cells 28.1 -> 4.7, 30.4 -> 15.8, 51.6 ->
-// 29.3, 150 -> 90; 5k cells, one column 20.3 -> 3.0.  Wide blocks are bound by
+// launches -> one launch: 100k cells, 1 / 16 / 64 / 256 columns 46.4 -> 9.0,
+// 87 -> 48, 233 -> 137, 852 -> 505; 20k cells 29.0 -> 4.8, 32.3 -> 15.9, 54.1 ->
+// 29.5, 151 -> 91; 5k cells, one column 21.1 -> 3.0.  Wide blocks are bound by
 // the FP64 pipe: one sweep instead of two on each side, s = omega D^-1 b kept
 // beside b and the prolongation folded into the sweep above it leave 45 FP64
 // instructions a node and column of about 100.
@@ -192,7 +192,7 @@ struct CgArgs {
 // round trips (row pointer, column, neighbour's value) instead of one.
 //
 // ONE: one group, so that its columns are all of them (one column, 100,043 cells:
-// 9.24 ms an apply with the group's columns counted, 8.95 without).
+// 9.24 ms an apply with the group's columns counted, 8.99 without).
 template <bool ONE>
 struct CgCta {
   const CgArgs& a;
